@@ -16,10 +16,6 @@ namespace {
 
 thread_local char g_last_error[256] = "";
 
-// Warps (of 8 per block) of the hybrid FP64 kernel that run on the FP64 pipe;
-// the others run the integer-pipe evaluation.
-constexpr int kDefaultHwRows = 4;
-
 using heat::check_err;
 using heat::cuda_fail;
 using heat::two_step_form;
@@ -148,7 +144,7 @@ cudaError_t enqueue_one(heat_ctx *c, int cur, cudaStream_t st) {
   if (c->flags & HEAT_BITEXACT)
     return heat::launch_exact_faces(un, uo, c->rhs, c->ks, g, c->factor, st);
   if (c->kq)
-    return heat::launch_fast_mix(un, uo, c->rhs, c->kq, c->c0, c->cf, g, c->hw_rows, c->err, st);
+    return heat::launch_fx(un, uo, c->kq, c->rhs, g, c->err, st);
   return heat::launch_fast(un, uo, c->rhs, c->c0, c->cf, g, st);
 }
 
@@ -282,46 +278,27 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
       c->launches += 1;
     }
   } else {
-    bool use_int = !(c->flags & HEAT_HWFP64);
-    c->hw_rows = kDefaultHwRows;
-    if (const char *ev = std::getenv("HEAT_HW_ROWS")) {  // tuning knob, 0..8
-      int v = std::atoi(ev);
-      if (v >= 0 && v <= 8) c->hw_rows = v;
-    }
-    if (c->hw_rows == 8) use_int = false;
-    // Both weight sets (the hybrid's two kinds of rows) come from one fused
-    // pass; HEAT_SETUP_SPLIT=1 runs the two separate kernels instead (same
-    // values; for comparison).
-    const char *sp = std::getenv("HEAT_SETUP_SPLIT");
-    const bool fused = use_int && c->hw_rows > 0 && !(sp && sp[0] == '1') &&
-                       g.ny <= 65535;  // one grid row of blocks per grid row j
-    if (fused) {
-      TRY(dalloc(&c->c0, g.elems, c->stream));
-      for (int a = 0; a < 3; ++a) TRY(dalloc(&c->cf[a], g.elems, c->stream));
-    }
-    if (use_int) {
-      // Integer-pipe form: per-point fixed-point factor*kappa.  Falls back to
-      // the FP64-pipe kernel when the fixed-point range check fails.
+    // Default form: per-point fixed-point weights.  Problems they cannot
+    // represent, and HEAT_HWFP64, use the FP64-pipe kernel and its FP64 weights.
+    bool fixed = !(c->flags & HEAT_HWFP64) && heat::fx_usable(d->rhs != nullptr);
+    if (fixed) {
       TRY(dalloc(&c->kq, g.elems, c->stream));
       int bad = 0;
       int *d_bad = reinterpret_cast<int *>(c->partials);
       cudaError_t e = cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream);
-      if (e == cudaSuccess)
-        e = fused ? heat::launch_weights_setup(c->kq, c->c0, c->cf, d_bad, kap, g, c->factor,
-                                               c->stream)
-                  : heat::launch_kq_setup(c->kq, d_bad, kap, g, c->factor, c->stream);
+      if (e == cudaSuccess) e = heat::launch_kq_setup(c->kq, d_bad, kap, g, c->factor, c->stream);
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) { rc = cuda_fail(e, "fixed-point setup"); goto done; }
-      c->launches += 1;
+      c->launches += 2;
       if (bad) {
         cudaFreeAsync(c->kq, c->stream);
         c->kq = nullptr;
-        use_int = false;
+        fixed = false;
       }
     }
-    if (!fused && (!use_int || c->hw_rows > 0)) {
+    if (!fixed) {
       TRY(dalloc(&c->c0, g.elems, c->stream));
       for (int a = 0; a < 3; ++a) TRY(dalloc(&c->cf[a], g.elems, c->stream));
       cudaError_t e = heat::launch_fast_coeffs(c->c0, c->cf, kap, g, c->factor, c->stream);
@@ -689,11 +666,9 @@ int heat_diag_fp32c_timeout(heat_ctx *c) {
 int heat_diag_fp64_timeout(heat_ctx *c) {
   if (!c) return HEAT_EINVAL;
   // Only contexts that step with the TMA-staged default FP64 launch.
-  if (c->precision != HEAT_FP64 || !c->kq || c->hw_rows != 4 ||
-      !heat::fast_tma_usable(c->g, c->rhs != nullptr))
-    return HEAT_ESTATE;
-  cudaError_t e = heat::launch_fast_tma(c->u[c->cur ^ 1], c->u[c->cur], c->kq, c->c0, c->cf,
-                                        c->rhs, c->g, c->err, c->stream, 0u);
+  if (c->precision != HEAT_FP64 || !c->kq) return HEAT_ESTATE;
+  cudaError_t e = heat::launch_fx(c->u[c->cur ^ 1], c->u[c->cur], c->kq, c->rhs, c->g, c->err,
+                                  c->stream, 0u);
   if (e != cudaSuccess) return cuda_fail(e, "default FP64 kernel launch");
   c->launches += 1;
   return HEAT_OK;

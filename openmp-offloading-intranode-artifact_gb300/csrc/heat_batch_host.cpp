@@ -15,9 +15,9 @@
 //
 // Grids large enough to fill the GPU alone (HEAT_BATCH_SOLO_POINTS interior
 // points, default 2,000,000) are stepped with their single-grid kernels
-// instead -- the FP64 hybrid launch, and two FP32C steps per launch -- on a
-// stream of their own beside the table kernels; the tile table carries the
-// small grids, which one launch per grid would leave the GPU mostly idle for.
+// instead (two FP32C steps per launch) on a stream of their own beside the table
+// kernels; the tile table carries the small grids, which one launch per grid
+// would leave the GPU mostly idle for.
 // On configuration 3 (64 grids of 48..384 points per axis) the table alone
 // measured 129 GLUP/s, with solo grids 137.
 //
@@ -67,7 +67,7 @@ struct heat_batch {
   size_t g_cap[2] = {0, 0};
   heat::BatchTile *t_buf[2] = {nullptr, nullptr};
   size_t t_cap[2] = {0, 0};
-  CUtensorMap *m_buf[2] = {nullptr, nullptr};  // two-step tiles' tensor maps, 7 per grid
+  CUtensorMap *m_buf[2] = {nullptr, nullptr};  // tensor maps of the TMA-staged grids
   size_t m_cap[2] = {0, 0};
   std::vector<int> pairs;       // active entries in the table with two steps per launch
   long long pair_flips = 0;     // buffer swaps of those grids since the table was built
@@ -112,8 +112,7 @@ int batch_form(const heat_ctx *c) {
   if (c->precision == HEAT_FP32C) return kFormF32c;
   if (c->flags & HEAT_NAIVE) return -1;
   if (c->flags & HEAT_BITEXACT) return kFormExact;
-  if (!c->kq) return kFormHw;
-  return (c->hw_rows == 4 && !c->rhs && batch_ws_usable(4)) ? kFormMixWs : kFormMix;
+  return c->kq ? kFormFx : kFormHw;
 }
 
 void batch_set_override(heat_batch *b, const TuneChoice &ch) {
@@ -199,7 +198,6 @@ heat::BatchGrid describe(const heat_ctx *c, int form) {
   g.S = c->g.plane;
   g.factor = c->factor;
   g.cur = c->cur;
-  g.hw_rows = c->hw_rows;
   g.err = c->err;
   if (form == heat::kFormF32c || form == heat::kFormF32c2) {
     g.f[0] = c->v[0];
@@ -214,11 +212,11 @@ heat::BatchGrid describe(const heat_ctx *c, int form) {
     g.rhs = c->rhs;
     if (form == heat::kFormExact) {
       for (int a = 0; a < 3; ++a) g.w[a] = c->ks[a];
-    } else {
+    } else if (form == heat::kFormHw) {
       g.w[0] = c->c0;
       for (int a = 0; a < 3; ++a) g.w[a + 1] = c->cf[a];
+    } else {
       g.kq = c->kq;
-      if (form == heat::kFormHw) g.hw_rows = 8;
     }
   }
   return g;
@@ -226,7 +224,7 @@ heat::BatchGrid describe(const heat_ctx *c, int form) {
 
 // Throughput guesses (GLUP/s on GB300) used only to split the SMs between
 // forms that run side by side.
-const double kFormRate[heat::kNumForms] = {100.0, 80.0, 29.0, 200.0, 110.0, 300.0};
+const double kFormRate[heat::kNumForms] = {200.0, 80.0, 29.0, 200.0, 300.0};
 
 // A side stream (and its join event) for kind f, created on first use.
 bool ensure_side(heat_batch *b, int f) {
@@ -247,34 +245,42 @@ int rebuild(heat_batch *b) {
   b->pair_flips = 0;
   std::vector<heat::BatchGrid> grids;
   std::vector<heat::BatchTile> per_form[heat::kNumKinds];
-  std::vector<CUtensorMap> maps;      // the two-step grids' maps, 7 each
+  std::vector<CUtensorMap> maps;            // the TMA-staged grids' maps
   std::vector<std::pair<int, int>> map_at;  // (grid index, first map)
   double work[heat::kNumKinds] = {};
+  auto points = [](const heat_ctx *c) {
+    return (long long)(c->g.nx - 2) * (c->g.ny - 2) * (c->g.nz - 2);
+  };
+  // Planes of default-FP64 tiles in the table, without and with a source term.
+  long fx_planes[2] = {0, 0};
+  for (const heat_batch::Entry &en : b->entries)
+    if (en.remaining > 0 && !(b->solo_points > 0 && points(en.ctx) >= b->solo_points) &&
+        heat::batch_form(en.ctx) == heat::kFormFx)
+      fx_planes[en.ctx->rhs != nullptr] += (long)heat::fx_tiles_x(en.ctx->g.nx) *
+                                           heat::fx_tiles_y(en.ctx->g.ny) * (en.ctx->g.nz - 2);
   for (size_t e = 0; e < b->entries.size(); ++e) {
     heat_batch::Entry &en = b->entries[e];
     if (en.remaining <= 0) continue;
     heat_ctx *c = en.ctx;
     en.base_steps = c->steps_done;
     en.pairs = false;
-    const long long pts = (long long)(c->g.nx - 2) * (c->g.ny - 2) * (c->g.nz - 2);
-    en.solo = b->solo_points > 0 && pts >= b->solo_points;
+    en.solo = b->solo_points > 0 && points(c) >= b->solo_points;
     if (en.solo) {
       b->solo.push_back((int)e);
       continue;
     }
     int form = heat::batch_form(c);
-    // The autotuner's choices for the grid's form and depth class (the
-    // warpgroup-split form shares the hybrid form's entries).
-    const int tform = form == heat::kFormMixWs ? heat::kFormMix : form;
-    heat::TuneChoice ch = heat::tuned_choice(tform, c->g.nz);
+    // The autotuner's choices for the grid's form and depth class.
+    heat::TuneChoice ch = heat::tuned_choice(form, c->g.nz);
     if (b->override_.kchunk > 0) ch.kchunk = b->override_.kchunk;
     if (b->override_.rows > 0) ch.rows = b->override_.rows;
     if (b->override_.minb > 0) ch.minb = b->override_.minb;
     if (b->override_.depth > 0) ch.depth = b->override_.depth;
     const int minb = std::max(heat::kMinbLo, std::min(ch.minb, heat::kMinbLo + heat::kNumMinb - 1));
     if (form == heat::kFormF32c && ch.depth == 2 && heat::two_step_form(c)) form = heat::kFormF32c2;
-    if (form == heat::kFormMixWs && !heat::batch_ws_usable(minb)) form = heat::kFormMix;
-    const int kind = heat::kind_of(form, grid_has_rhs(c), form == heat::kFormF32c2 ? heat::kMinbLo : minb);
+    // The TMA-staged table kernels come in one variant.
+    const bool one = form == heat::kFormF32c2 || form == heat::kFormFx;
+    const int kind = heat::kind_of(form, grid_has_rhs(c), one ? heat::kMinbLo : minb);
     const int gi = (int)grids.size();
     grids.push_back(describe(c, form));
     b->active.push_back((int)e);
@@ -293,7 +299,18 @@ int rebuild(heat_batch *b) {
       rows = 1;
       tile_h = 16;
     }
-    const int ntx = (c->g.nx - 2 + 31) / 32, nty = (c->g.ny - 2 + tile_h - 1) / tile_h;
+    int ntx = (c->g.nx - 2 + 31) / 32, nty = (c->g.ny - 2 + tile_h - 1) / tile_h;
+    if (form == heat::kFormFx) {
+      map_at.push_back({gi, (int)maps.size()});
+      maps.resize(maps.size() + 4);
+      if (!heat::encode_fx_maps(&maps[maps.size() - 4], c->u, c->kq, c->rhs, c->g))
+        return HEAT_ECUDA;
+      // A small table fills the GPU with shorter tiles than the tuned ones.
+      kc = std::min(kc, std::max(1, heat::fx_fill_chunk(fx_planes[c->rhs != nullptr], c->rhs)));
+      rows = 1;
+      ntx = heat::fx_tiles_x(c->g.nx);
+      nty = heat::fx_tiles_y(c->g.ny);
+    }
     for (int k0 = 1; k0 < c->g.nz - 1; k0 += kc) {
       const int k1 = std::min(k0 + kc, c->g.nz - 1);
       for (int ty = 0; ty < nty; ++ty)

@@ -9,12 +9,11 @@
 namespace heat {
 
 enum BatchForm : int {
-  kFormMix = 0,    // default FP64: hw_rows warps on the FP64 pipe, the rest integer
+  kFormFx = 0,     // default FP64 (fixed point, TMA-staged, 32 x 16 tiles)
   kFormHw = 1,     // default FP64 on the FP64 pipe only
   kFormExact = 2,  // bit-exact FP64 (face kappa sums)
   kFormF32c = 3,   // FP32-compensated, one step per launch
-  kFormMixWs = 4,  // default FP64, hw_rows = 4, no source term: warpgroup-split kernel
-  kFormF32c2 = 5,  // FP32-compensated, two steps per launch (TMA-staged, 32 x 16 tiles)
+  kFormF32c2 = 4,  // FP32-compensated, two steps per launch (TMA-staged, 32 x 16 tiles)
 };
 
 // One grid of a batch as the kernel sees it.  f[b] / cr[b] are the two field
@@ -24,23 +23,22 @@ enum BatchForm : int {
 struct BatchGrid {
   int form;
   int nx, ny, nz, P;
-  int hw_rows;
   int cur;
-  int pad_;
   size_t S;
   double factor;
   void *f[2];
   uint16_t *cr[2];
   const void *rhs;
-  const void *w[4];  // Mix/Hw: c0, cx, cy, cz   Exact: kx, ky, kz   F32c: wx, wy, wz
-  const unsigned long long *kq;
+  const void *w[4];  // Hw: c0, cx, cy, cz   Exact: kx, ky, kz   F32c: wx, wy, wz
+  const unsigned long long *kq;  // Fx
   int *err;            // the context's error flag (bounded waits that ran out)
-  const void *tmaps;   // F32c2: seven CUtensorMaps in device memory (v0 v1 c0 c1 wx wy wz)
+  const void *tmaps;   // CUtensorMaps in device memory: Fx four (u0 u1 K rhs), F32c2 seven
+                       // (v0 v1 c0 c1 wx wy wz)
 };
 
 // A tile of grid `grid` walking planes [k0, k1): 32 columns (tx) by 8 * rows
-// rows (ty), each thread walking `rows` columns 8 rows apart; F32c2 tiles are
-// 32 x 16 (two-step kernel's tile) and rows is 1.
+// rows (ty), each thread walking `rows` columns 8 rows apart; Fx and F32c2 tiles
+// are 32 x 16 (their kernels' tiles) and rows is 1.
 struct BatchTile {
   int grid;
   int tx, ty;
@@ -48,7 +46,7 @@ struct BatchTile {
   int rows;
 };
 
-constexpr int kNumForms = 6;
+constexpr int kNumForms = 5;
 // Blocks-per-SM variants of the table kernels (their register caps): 2, 3, 4.
 constexpr int kNumMinb = 3;
 constexpr int kMinbLo = 2;
@@ -63,10 +61,17 @@ inline int form_of_kind(int kind) { return kind / (2 * kNumMinb); }
 cudaError_t launch_batch(int kind, const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                          int flip, int blocks, cudaStream_t st);
 int batch_blocks_per_sm(int kind);
-// Whether the warpgroup-split table kernel's variant for `minb` blocks per SM
-// compiled to the register count its setmaxnreg bounds assume (else the
-// general hybrid kernel runs those tiles).
-bool batch_ws_usable(int minb = 4);
+// heat_fp64_fx.cu: the default FP64 form's table kernel, its tiles per axis,
+// their depth and its per-grid maps.
+cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int ntiles, bool rhs,
+                            int flip, cudaStream_t st);
+int fx_tiles_x(int nx);
+int fx_tiles_y(int ny);
+// Planes per block that fill the GPU with blocks for a launch of tile_planes
+// planes of tiles in all; long launches want no longer chunks than 16 or so.
+int fx_fill_chunk(long tile_planes, bool rhs);
+bool encode_fx_maps(CUtensorMap *m4, double *const u[2], const unsigned long long *K,
+                    const double *rhs, const heat_geom &g);
 // heat_fp32c_tma.cu: the two-step FP32C table kernel and its per-grid maps.
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                                    int flip, cudaStream_t st);
@@ -84,7 +89,7 @@ struct TuneChoice {
 };
 TuneChoice tuned_choice(int form, int nz);
 // Default blocks-per-SM variant of a form's table kernel.
-inline int default_minb(int form) { return form == kFormMix ? 3 : 4; }
+inline int default_minb(int form) { return form == kFormFx ? 3 : 4; }
 
 // heat_batch_run with the final stream synchronisation optional (sync=false:
 // the launches are queued and the bookkeeping advanced on return).

@@ -1,0 +1,693 @@
+// Default FP64 form: every point on the integer pipes, in fixed point at a
+// scale shared by a 2 x 2 patch of columns.
+//
+// GB300 retires 2 FP64 operations per clock and SM, and 64 to 128 integer
+// ones.  The update
+//
+//   u_new = uC + rhs + sum_f w_f (u_f - uC),   w_f = factor (kappa_a + kappa_b)
+//
+// (the reference's expression, OpenMP_Single_Source/heat3D_variable_coeff.c:
+// 174-181, regrouped) costs 7 FP64 operations, which caps a kernel on the FP64
+// pipe at 85 GLUP/s.  Here it is evaluated exactly but for the last bits of its
+// products in 64-bit integers and rounded once:
+//
+//   * A thread owns a 2 x 2 patch of columns (rows j0 + 2m, j0 + 2m + 1, even
+//     column i and i + 1) and walks planes.  At plane k its stencil region is
+//     the patch at planes k - 1, k, k + 1 and the patch's eight in-plane
+//     neighbours.  The largest exponent in the region (one more if any value
+//     is negative, rounded up to an even number) gives the scale E: a value
+//     becomes the integer A = value * 2^(1083 - E), |A| < 2^61.
+//   * If no nonzero value of the patch itself (three planes) lies more than
+//     kSlack = 6 binary orders below E, those A are exact (8 orders would be), and
+//     one unit of A is at most 1/4 ulp of the smallest of them.  A neighbour
+//     further below is cut to whole units, an error of one unit times its weight.
+//   * Weights come from the per-point K = factor * kappa, kept as two limbs
+//     K = k1 2^-32 + k0 2^-63 with |k0| <= 2^30: a face weight is the two limb
+//     sums, no carry, and its low limb is a signed 32-bit number.
+//   * Each face adds D w (D = A_f - A_C, limbs d1 signed, d0 unsigned) as three
+//     32 x 32 -> 64 multiply-adds into exact accumulators: H += d1 w1,
+//     X += d1 w0 (units of 2^-31), Y += d0 w1 (2^-32); only d0 w0, below one
+//     unit, is dropped.  H + round(X) + round(Y) is then rounded to nearest
+//     even by one int64 -> FP64 conversion (one operation of the FP64 pipe), and
+//     the scale goes into its exponent field.
+//
+// The error of a step is that rounding plus about one unit of A; a sum of seven
+// FP64 multiply-adds has seven roundings, and rounded weights besides.  A
+// constant region stays exactly constant (every D is 0).
+//
+// Patches outside those bounds (a wider range of magnitudes, exponents near
+// either end, infinities, NaNs) take walk::int_point per point, which aligns
+// each point's seven values to their own largest exponent.  Which of the two a
+// patch takes, and E, depend only on the field's values in its region, never on
+// tiles or z-chunks, so a grid's results are the same bits in any launch.
+// (kSlack: of a Gaussian of width 0.05 on 512^3, whose tails fall by up to one
+// binary order per point, no patch is outside it; 16 x 8-point patches would
+// leave 70 % of the grid outside.)
+//
+// The integers carried along z move to a new scale by shifting, which is exact
+// because both scales hold the patch exactly.
+//
+// Staging: a block is 32 x 16 columns (128 threads, 16 x 8 patches).  Planes of
+// u and K (and the source term) land by TMA in a 4-deep ring, boxes 36 x 18
+// from column i0 - 2 (16-byte aligned), each slot completing on its own
+// mbarrier; one block barrier per plane frees the oldest slot, whose next plane
+// thread 0 then requests.
+//
+// Bound: the integer pipes.  At 512^3: 167 GLUP/s (0.79 ms a step; 133.5 for
+// rows split between 7 FP64 operations and a per-point alignment in integers,
+// the launch before this one), with the reference's source term 139 (115.7).
+// About 137 warp instructions per point (300 for an integer row of that
+// launch); ALU, FMA-heavy (18 of its instructions the wide multiply-adds, twice
+// the cost of the others) and issue are each about 60 % busy, DRAM 55 %.
+// Measured and not kept: the neighbours above and below converted by the FP64
+// pipe as the patch's own are (157; that pipe is then at 75 % and the others wait
+// for it), no value converted by it (164), five blocks per SM at 96 registers
+// (165), 32 x 32 tiles (156), 64 x 8 (166), the plane loop unrolled by 2 (162).
+//
+// Every mbarrier wait is bounded: a wait that runs out stops the block at the
+// next barrier (the flag is OR-reduced), thread 0 waits (bounded) for its loads
+// in flight, *err is set and the host reports HEAT_ETIMEOUT.
+
+#include <cuda.h>
+
+#include <cstring>
+
+#include "heat_batch_internal.h"
+#include "heat_internal.h"
+#include "heat_tma.cuh"
+#include "heat_walk.cuh"
+
+namespace heat {
+namespace {
+
+typedef unsigned long long u64;
+typedef long long i64;
+
+constexpr int TX = 32, TY = 16;          // columns of a tile
+constexpr int NTX = TX / 2, NTY = TY / 2;
+constexpr int NT = NTX * NTY;            // threads, one per 2 x 2 patch
+constexpr int BX = TX + 4, BY = TY + 2;  // box: columns i0 - 2 .. i0 + 33, rows j0 - 1 .. j0 + 16
+// Ring depth: planes k, k + 1 and two in flight; one with a source term, whose
+// slots are larger (four blocks of 4 would not fit an SM).
+template <bool RHS>
+constexpr int kRing = RHS ? 3 : 4;
+constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills
+
+constexpr unsigned kExp = 1u << 20;      // one binary order in the high word of a double
+constexpr unsigned kExpMask = 0x7ff00000u;
+constexpr unsigned kSlack = 8 * kExp;
+constexpr int kLeast = 1 << (53 - 32);  // high word of 2^53
+constexpr unsigned kLowE = 128 * kExp, kMidE = 1083 * kExp, kHighE = 2030 * kExp;
+
+// Element count of `rows` box rows padded to 128 bytes: each array of a slot
+// starts on a 128-byte boundary, as TMA shared-memory destinations must.
+constexpr int pad128(int elems) { return (elems * 8 + 127) / 128 * 128 / 8; }
+constexpr int kPad = pad128(BX * BY), kRPad = pad128(TX * TY);
+
+template <bool RHS>
+struct __align__(128) Slot {
+  u64 u[kPad];
+  u64 k[kPad];
+};
+template <>
+struct __align__(128) Slot<true> {
+  u64 u[kPad];
+  u64 k[kPad];
+  u64 r[kRPad];  // source term at the tile's own columns
+};
+template <bool RHS>
+constexpr unsigned kSlotBytes = (2u * BX * BY + (RHS ? TX * TY : 0)) * 8u;
+static_assert(sizeof(Slot<false>) % 128 == 0 && sizeof(Slot<true>) % 128 == 0 &&
+                  (kPad * 8) % 128 == 0,
+              "ring slots and their arrays start on 128-byte boundaries");
+
+template <bool RHS>
+struct Smem {
+  Slot<RHS> ring[kRing<RHS>];
+  u64 bar[kRing<RHS>];
+};
+
+// Where a tile finds its tensor maps: kernel parameters for a single grid,
+// device memory for a batch (u of buffers 0 and 1, K, source term).
+struct Maps {
+  CUtensorMap u, k, r;
+};
+struct ParamMaps {
+  const Maps &m;
+  __device__ __forceinline__ const CUtensorMap *u() const { return &m.u; }
+  __device__ __forceinline__ const CUtensorMap *k() const { return &m.k; }
+  __device__ __forceinline__ const CUtensorMap *r() const { return &m.r; }
+};
+struct TableMaps {
+  const CUtensorMap *tm;
+  int src;
+  __device__ __forceinline__ const CUtensorMap *u() const { return &tm[src]; }
+  __device__ __forceinline__ const CUtensorMap *k() const { return &tm[2]; }
+  __device__ __forceinline__ const CUtensorMap *r() const { return &tm[3]; }
+};
+
+// Exponent range and signs of a set of values, from their high words.  Zeros
+// do not count in mn (t - 1 wraps to the top), nor do subnormals, which beside
+// a normal number are below 2^-60 units and read as 0; fx_tile tells a region
+// of zeros from one of subnormals.
+struct Range {
+  unsigned mx = 0, mn = ~0u, sg = 0;
+  __device__ __forceinline__ void see(u64 v) {
+    const unsigned hi = (unsigned)(v >> 32), t = hi & kExpMask;
+    mx = max(mx, t);
+    mn = min(mn, t - 1);
+    sg |= hi;
+  }
+  // A value that only has to be below the scale.
+  __device__ __forceinline__ void bound(u64 v) {
+    const unsigned hi = (unsigned)(v >> 32);
+    mx = max(mx, hi & kExpMask);
+    sg |= hi;
+  }
+  __device__ __forceinline__ void see(const Range &o) {
+    mx = max(mx, o.mx);
+    mn = min(mn, o.mn);
+    sg |= o.sg;
+  }
+  // Scale (exponent field) of the region.
+  __device__ __forceinline__ unsigned scale() const {
+    const unsigned up = (int)sg < 0 ? 2 * kExp : kExp;
+    return max((mx + up) & ~(2 * kExp - 1), kLowE);
+  }
+  __device__ __forceinline__ bool fits(unsigned E) const {
+    return E - min(mn, E) <= kSlack + 1 && E <= kHighE && mx != 0;
+  }
+};
+
+__device__ __forceinline__ u64 shr(u64 a, unsigned n) {  // 0 for n >= 64
+  u64 r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
+  return r;
+}
+__device__ __forceinline__ u64 sar(u64 a, unsigned n) {
+  u64 r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
+  return r;
+}
+__device__ __forceinline__ u64 shl(u64 a, unsigned n) {
+  u64 r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
+  return r;
+}
+
+// |v| in units of 2^(E - 1083): the significand left-aligned, its leading bit
+// or-ed in, shifted right by 3 + E - e (over 63, so to 0, where the exponent
+// field is 0).
+__device__ __forceinline__ u64 magnitude(u64 v, unsigned E) {
+  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v, t = hi & kExpMask;
+  const unsigned h = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+  return shr(((u64)h << 32) | (lo << 11), (E + 3 * kExp - t) >> 20);
+}
+// The same of a value that is not negative, for E <= kMidE, by the FP64 pipe:
+// the scale goes into the exponent field (0 stays below 1/2 unit) and the
+// conversion does the rest.
+__device__ __forceinline__ u64 convert(u64 v, unsigned E) {
+  return (u64)__double2ll_rn(
+      __hiloint2double((int)((unsigned)(v >> 32) + (kMidE - E)), (int)(unsigned)v));
+}
+__device__ __forceinline__ u64 with_sign(u64 a, u64 v) {
+  const u64 s = (u64)((i64)v >> 63);
+  return (a ^ s) - s;
+}
+
+// r units of 2^(E - 1083).
+__device__ __forceinline__ double scaled(double r, unsigned E) {
+  const unsigned hi = (unsigned)__double2hiint(r);  // 0 only for 0
+  return __hiloint2double((int)(hi ? hi + (E - kMidE) : 0u), __double2loint(r));
+}
+
+template <bool B>
+struct Bool {
+  static constexpr bool value = B;
+};
+
+struct Acc {
+  u64 H, X, Y;
+  __device__ __forceinline__ explicit Acc(u64 centre) : H(centre), X(1ull << 31), Y(1ull << 31) {}
+  // += D * w
+  __device__ __forceinline__ void face(u64 D, unsigned w0, unsigned w1) {
+    const unsigned d0 = (unsigned)D, d1 = (unsigned)(D >> 32);
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(H) : "r"(d1), "r"(w1));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(X) : "r"(d1), "r"(w0));
+    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(Y) : "r"(d0), "r"(w1));
+  }
+  __device__ __forceinline__ void face(u64 D, u64 ka, u64 kb) {
+    face(D, (unsigned)ka + (unsigned)kb, (unsigned)(ka >> 32) + (unsigned)(kb >> 32));
+  }
+  // The sum in units, to the nearest FP64 value.
+  __device__ __forceinline__ double rounded() {
+    asm("mad.wide.s32 %0, %1, 2, %0;" : "+l"(H) : "r"((unsigned)(X >> 32)));
+    H += Y >> 32;
+    return __ll2double_rn((i64)H);
+  }
+  // += v to the nearest unit
+  __device__ __forceinline__ void add(u64 v, unsigned E) {
+    const u64 h = magnitude(v, E - kExp);  // in half units
+    H += with_sign((h >> 1) + (h & 1), v);
+  }
+};
+
+// A point of a patch outside the shared scale's bounds: box offset p, the value
+// vd below it and the limbs of the weight to it.  The same arithmetic at the
+// point's own scale, the largest exponent of its seven values (and the source
+// term), every value cut to that scale's units; exponents near either end,
+// infinities and NaNs take walk::int_point.  pd: the value below in global
+// memory (vd may have read a subnormal as 0).
+template <bool RHS>
+__device__ __noinline__ double point(const Slot<RHS> &sk, const Slot<RHS> &sn, int p, int prhs,
+                                     u64 vd, unsigned w0, unsigned w1, const u64 *pd) {
+  const u64 c = sk.u[p], f[6] = {sn.u[p], vd, sk.u[p - 1], sk.u[p + 1], sk.u[p - BX], sk.u[p + BX]};
+  Range r;
+  r.bound(c);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) r.bound(f[q]);
+  u64 vr = 0;
+  if constexpr (RHS) {
+    vr = sk.r[prhs];
+    r.bound(vr);
+  }
+  const u64 kc = sk.k[p];
+  const u64 k[6] = {sn.k[p], 0, sk.k[p - 1], sk.k[p + 1], sk.k[p - BX], sk.k[p + BX]};
+  const unsigned E = r.mx + ((int)r.sg < 0 ? kExp : 0u);
+  if (E - kLowE <= kHighE - kLowE) {
+    auto load = [&](u64 v) { return with_sign(magnitude(v, E), v); };
+    const u64 A = load(c);
+    Acc a(A);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      if (q == 1)
+        a.face(load(f[q]) - A, w0, w1);
+      else
+        a.face(load(f[q]) - A, kc, k[q]);
+    }
+    if constexpr (RHS) a.add(vr, E);
+    return scaled(a.rounded(), E);
+  }
+  const u64 ud = *pd;
+  if (((c | f[0] | ud | f[2] | f[3] | f[4] | f[5] | vr) << 1) == 0) return 0.0;
+  // K in units of 2^-64, as int_point takes it; the one below from the face's limbs
+  auto weight = [](unsigned k0, unsigned k1) {
+    return ((u64)k1 << 32) + 2ull * (u64)(i64)(int)k0;
+  };
+  auto w = [&](u64 x) { return weight((unsigned)x, (unsigned)(x >> 32)); };
+  return walk::int_point<RHS>(
+      walk::decode(c), walk::decode(f[0]), walk::decode(ud), walk::decode(f[3]), walk::decode(f[2]),
+      walk::decode(f[5]), walk::decode(f[4]), w(kc), w(k[0]),
+      weight(w0 - (unsigned)kc, w1 - (unsigned)(kc >> 32)), w(k[3]), w(k[2]), w(k[5]), w(k[4]), vr,
+      [=] { return walk::Raw7{c, f[3], f[2], f[5], f[4], f[0], ud}; });
+}
+
+// Keeps the compiler from holding values read before this point in registers.
+__device__ __forceinline__ void reload() { asm volatile("" ::: "memory"); }
+
+__device__ __forceinline__ ulonglong2 ld2(const u64 *p) {
+  return *reinterpret_cast<const ulonglong2 *>(p);
+}
+
+// One step over the (32 x 16)-column tile (tx, ty), planes [kb, ke), of the
+// field u into un.  Returns true if a wait ran out.
+template <bool RHS, class M>
+__device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__restrict__ un,
+                                        const u64 *__restrict__ u, const u64 *__restrict__ K,
+                                        int tx, int ty, int nx, int ny, int P, size_t S, int kb,
+                                        int ke, unsigned wait_limit) {
+  const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
+  const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly;  // patch: i, i + 1; j, j + 1
+  const int o = (2 * ly + 1) * BX + 2 * lx + 2;              // its first point in a box
+  const bool x0 = i >= 1 && i < nx - 1, x1 = i + 1 < nx - 1;
+  const bool y0 = j < ny - 1, y1 = j + 1 < ny - 1;
+  const bool active = y0 && (x0 || x1);  // the patch holds a point to write
+
+  if (t == 0) {
+    for (int s = 0; s < kRing<RHS>; ++s) tma::mbar_init(&sm.bar[s]);
+    tma::mbar_init_fence();
+  }
+  __syncthreads();
+  auto issue = [&](int p, int s) {
+    if (t != 0 || p > ke) return;
+    Slot<RHS> &sl = sm.ring[s];
+    u64 *b = &sm.bar[s];
+    tma::fence_proxy_async();
+    tma::mbar_expect(b, kSlotBytes<RHS>);
+    tma::load3(sl.u, maps.u(), tx * TX - 2, ty * TY, p, b);
+    tma::load3(sl.k, maps.k(), tx * TX - 2, ty * TY, p, b);
+    if constexpr (RHS) tma::load3(sl.r, maps.r(), tx * TX, ty * TY + 1, p, b);
+  };
+  for (int s = 0; s < kRing<RHS>; ++s) issue(kb - 1 + s, s);
+
+  // Carried along z, points in the order (i, j), (i + 1, j), (i, j + 1),
+  // (i + 1, j + 1): the patch at plane k (A1) and its difference to plane k - 1
+  // (Dd) at scale E (0: not held), the weight limbs of the face below, K and
+  // the ranges.
+  u64 Dd[4], A1[4];
+  unsigned W0[4], W1[4];
+  Range r0, r1;
+  unsigned E = 0;
+  bool failed = !tma::mbar_wait(&sm.bar[0], 0, wait_limit) ||
+                !tma::mbar_wait(&sm.bar[1], 0, wait_limit);
+  if (!failed) {
+    u64 a[4], b[4], ka[4], Kc[4];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      ulonglong2 v = ld2(&sm.ring[0].u[o + q * BX]);
+      a[2 * q] = v.x, a[2 * q + 1] = v.y;
+      v = ld2(&sm.ring[1].u[o + q * BX]);
+      b[2 * q] = v.x, b[2 * q + 1] = v.y;
+      v = ld2(&sm.ring[0].k[o + q * BX]);
+      ka[2 * q] = v.x, ka[2 * q + 1] = v.y;
+      v = ld2(&sm.ring[1].k[o + q * BX]);
+      Kc[2 * q] = v.x, Kc[2 * q + 1] = v.y;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      r0.see(a[q]);
+      r1.see(b[q]);
+      W0[q] = (unsigned)ka[q] + (unsigned)Kc[q];
+      W1[q] = (unsigned)(ka[q] >> 32) + (unsigned)(Kc[q] >> 32);
+    }
+    Range r = r0;
+    r.see(r1);
+    E = r.scale();  // at most the first plane's scale, so what that needs exact is exact
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      A1[q] = with_sign(magnitude(b[q], E), b[q]);
+      Dd[q] = with_sign(magnitude(a[q], E), a[q]) - A1[q];
+    }
+    if (!r.fits(E)) {
+      E = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) A1[q] = a[q];
+    }
+  }
+
+  // Slots of planes k - 1 and k at the top of an iteration, and the parity of
+  // the next plane's phase.
+  int s0 = 0, s1 = 1;
+  unsigned parity = 0;
+  double *w = un + (size_t)kb * S + (size_t)j * P + i;  // the patch at plane k
+  int k = kb;
+  for (; k < ke; ++k, w += S) {
+    const int s2 = s1 == kRing<RHS> - 1 ? 0 : s1 + 1;
+    if (s2 == 0) parity ^= 1;
+    if (!failed) failed = !tma::mbar_wait(&sm.bar[s2], parity, wait_limit);
+    failed = __syncthreads_or(failed);
+    if (failed) break;
+    issue(k - 1 + kRing<RHS>, s0);  // every thread is done with plane k - 1
+    const Slot<RHS> &sk = sm.ring[s1], &sn = sm.ring[s2];
+
+    s0 = s1;
+    s1 = s2;
+    if (!active) continue;
+    Range r2, r = r0;
+    {
+      u64 up[4], h[8];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        ulonglong2 v = ld2(&sn.u[o + q * BX]);
+        up[2 * q] = v.x, up[2 * q + 1] = v.y;
+        h[q] = sk.u[o + q * BX - 1];
+        h[2 + q] = sk.u[o + q * BX + 2];
+        v = ld2(&sk.u[q ? o + 2 * BX : o - BX]);
+        h[4 + 2 * q] = v.x, h[5 + 2 * q] = v.y;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) r2.see(up[q]);
+      r.see(r1);
+      r.see(r2);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) r.bound(h[q]);
+    }
+    u64 rr[4];
+    if constexpr (RHS) {
+      // The source counts towards the largest exponent only: it is added to
+      // the nearest unit.
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        rr[q] = sk.r[(2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1)];
+        r.bound(rr[q]);
+      }
+    }
+    const unsigned En = r.scale();
+    if (r.fits(En)) {
+      if (E != En) {
+        if (E == 0) {  // the plane before went point by point
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const u64 a = A1[q], b = sk.u[o + (q >> 1) * BX + (q & 1)];
+            A1[q] = with_sign(magnitude(b, En), b);
+            Dd[q] = with_sign(magnitude(a, En), a) - A1[q];
+          }
+        } else {
+          const int d = (int)(En - E) >> 20;
+          const unsigned dn = (unsigned)max(d, 0), ups = (unsigned)max(-d, 0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            Dd[q] = sar(shl(Dd[q], ups), dn);
+            A1[q] = sar(shl(A1[q], ups), dn);
+          }
+        }
+        E = En;
+      }
+      // The values are read from shared memory again here, row by row, rather
+      // than kept in registers from the range pass.
+      u64 A2[4];
+      int least = 0x7fffffff;  // high word of the smallest result (its size), in units
+      auto patch = [&](auto plain) {
+        auto load = [&](u64 v) {
+          const u64 m = magnitude(v, E);
+          return plain.value ? m : with_sign(m, v);
+      };
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          reload();
+          double out[2];
+          const int oy = o + y * BX, oo = y ? o + 2 * BX : o - BX;
+          const ulonglong2 vU = ld2(&sn.u[oy]), vO = ld2(&sk.u[oo]);
+          const ulonglong2 kC = ld2(&sk.k[oy]), kI = ld2(&sk.k[y ? o : o + BX]), kO = ld2(&sk.k[oo]),
+                           kU = ld2(&sn.k[oy]);
+          A2[2 * y] = plain.value ? convert(vU.x, E) : load(vU.x);
+          A2[2 * y + 1] = plain.value ? convert(vU.y, E) : load(vU.y);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int q = 2 * y + x, side = x ? oy + 2 : oy - 1;
+            const u64 Kc = x ? kC.y : kC.x, Ku = x ? kU.y : kU.x;
+            const unsigned U0 = (unsigned)Kc + (unsigned)Ku;
+            const unsigned U1 = (unsigned)(Kc >> 32) + (unsigned)(Ku >> 32);
+            Acc a(A1[q]);
+            a.face(A2[q] - A1[q], U0, U1);
+            a.face(Dd[q], W0[q], W1[q]);
+            a.face(A1[q ^ 1] - A1[q], Kc, x ? kC.x : kC.y);
+            a.face(load(sk.u[side]) - A1[q], Kc, sk.k[side]);
+            a.face(A1[q ^ 2] - A1[q], Kc, x ? kI.y : kI.x);
+            a.face(load(x ? vO.y : vO.x) - A1[q], Kc, x ? kO.y : kO.x);
+            if constexpr (RHS) a.add(rr[q], E);
+            const double v = a.rounded();
+          if ((x ? x1 : x0) && (y ? y1 : y0)) {
+            const int h = (int)(a.H >> 32);
+            least = min(least, plain.value ? h : h ^ (h >> 31));
+          }
+          out[x] = scaled(v, E);
+            Dd[q] = A1[q] - A2[q];
+            W0[q] = U0, W1[q] = U1;
+          }
+          if (y ? y1 : y0) {
+            double *wy = w + (y ? P : 0);
+            if (x0 && x1) {
+              *reinterpret_cast<double2 *>(wy) = make_double2(out[0], out[1]);
+            } else {
+              if (x0) wy[0] = out[0];
+              if (x1) wy[1] = out[1];
+            }
+          }
+        }
+      };
+      if ((int)r.sg >= 0 && E <= kMidE)
+        patch(Bool<true>{});
+      else
+        patch(Bool<false>{});
+#pragma unroll
+      for (int q = 0; q < 4; ++q) A1[q] = A2[q];
+      if (least < kLeast) {
+        // A result too small for the scale's units (zeros in the patch, small
+        // neighbours): point by point, planes below from global memory.
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          if (!((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0))) continue;
+          const int p = o + (q >> 1) * BX + (q & 1);
+          double *wq = w + ((q & 2 ? P : 0) + (q & 1));
+          const u64 *pd = u + (wq - un) - S;
+          const u64 Kc = sk.k[p], Kd = K[pd - u];
+          *wq = point<RHS>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), *pd,
+                           (unsigned)Kc + (unsigned)Kd,
+                           (unsigned)(Kc >> 32) + (unsigned)(Kd >> 32), pd);
+        }
+      }
+    } else {
+      // Point by point.  E = 0: A1 then holds the patch's values (bits) at the
+      // plane below.
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int p = o + (q >> 1) * BX + (q & 1);
+        const u64 below =
+            E ? (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E)) : A1[q];
+        if ((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0)) {
+          double *wq = w + ((q & 2 ? P : 0) + (q & 1));
+          *wq = point<RHS>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), below, W0[q],
+                           W1[q], u + (wq - un) - S);
+        }
+        A1[q] = sk.u[p];
+        const u64 Kc = sk.k[p], Ku = sn.k[p];
+        W0[q] = (unsigned)Kc + (unsigned)Ku;
+        W1[q] = (unsigned)(Kc >> 32) + (unsigned)(Ku >> 32);
+      }
+      E = 0;
+    }
+    r0 = r1;
+    r1 = r2;
+  }
+  // Planes k - 1 and on were requested up to plane k + kRing<RHS> - 2.
+  if (failed && t == 0)
+    for (int p = k - 1; p <= min(k + kRing<RHS> - 2, ke); ++p)
+      tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing<RHS>], (p - kb + 1) / kRing<RHS> & 1u);
+  return failed;
+}
+
+template <bool RHS>
+__device__ __forceinline__ Smem<RHS> &smem() {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  return *reinterpret_cast<Smem<RHS> *>(smem_raw);
+}
+
+template <bool RHS>
+__global__ void __launch_bounds__(NT, kMinB)
+    k_fx(const __grid_constant__ Maps maps, double *__restrict__ un, const u64 *__restrict__ u,
+         const u64 *__restrict__ K, int nx, int ny, int nz, int P, size_t S, int kchunk, int *__restrict__ err,
+         unsigned wait_limit) {
+  const int kb = 1 + blockIdx.z * kchunk;
+  const int ke = min(kb + kchunk, nz - 1);
+  if (kb >= ke) return;  // whole block
+  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, blockIdx.x, blockIdx.y, nx, ny, P, S, kb,
+                   ke, wait_limit) &&
+      threadIdx.x == 0)
+    atomicExch(err, 1);
+}
+
+// The batch table's tiles: one block per tile.  Grid g's maps are in device
+// memory, four per grid; each launch reads buffer cur ^ flip.
+template <bool RHS>
+__global__ void __launch_bounds__(NT, kMinB)
+    k_batch_fx(const BatchGrid *__restrict__ grids, const BatchTile *__restrict__ tiles, int flip) {
+  const BatchTile tl = tiles[blockIdx.x];
+  const BatchGrid &g = grids[tl.grid];
+  const int src = g.cur ^ flip, dst = src ^ 1;
+  const CUtensorMap *tm = static_cast<const CUtensorMap *>(g.tmaps);
+  // The maps were written by a host copy before the launch; order the tensor
+  // proxy's reads of them after it.
+  if (threadIdx.x < 4)
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm + threadIdx.x)
+                 : "memory");
+  __syncthreads();
+  if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq, tl.tx,
+                   tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1, kWaitLimit) &&
+      threadIdx.x == 0)
+    atomicExch(g.err, 1);
+}
+
+template <bool RHS>
+constexpr size_t smem_bytes() { return sizeof(Smem<RHS>) + 128; }
+
+bool allow_smem(const void *kernel, size_t bytes) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
+      cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
+template <bool RHS>
+bool usable() {
+  static const bool ok = tma::encoder() && allow_smem((const void *)k_fx<RHS>, smem_bytes<RHS>()) &&
+                         allow_smem((const void *)k_batch_fx<RHS>, smem_bytes<RHS>());
+  return ok;
+}
+
+bool encode(CUtensorMap *m, const void *base, const heat_geom &g, unsigned x, unsigned y) {
+  return tma::encode_field(m, base, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, g, x, y);
+}
+
+template <bool RHS>
+long resident() {
+  static const long n = resident_blocks((const void *)k_fx<RHS>, NT, smem_bytes<RHS>());
+  return n;
+}
+
+template <bool RHS>
+cudaError_t launch(const Maps &m, double *u_new, const double *u_old, const u64 *K,
+                   const heat_geom &g, int *err, cudaStream_t st, unsigned wait_limit) {
+  const int interior = g.nz - 2;
+  int kc = fx_fill_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny) * interior, RHS);
+  kc = kc >= 16 ? wave_chunk(g, TX, TY, resident<RHS>()) : kc < interior ? kc : interior;
+  dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
+  k_fx<RHS><<<gr, NT, smem_bytes<RHS>(), st>>>(m, u_new, (const u64 *)u_old, K, g.nx, g.ny, g.nz,
+                                               g.pitch, g.plane, kc, err, wait_limit);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+// Tiles start at column 0 (an even, 16-byte aligned column; it is a boundary
+// column and not written) and row 1.
+int fx_tiles_x(int nx) { return (nx - 1 + TX - 1) / TX; }
+int fx_tiles_y(int ny) { return (ny - 2 + TY - 1) / TY; }
+
+// A lone block needs about 1 us a plane and 4 us to start and finish a launch,
+// a full SM (4 blocks) 2 us a plane of each: small grids want short chunks until
+// the GPU holds 1.7 blocks for every resident one (64^3: 7.1 us a step at 1
+// plane, 12.3 at 8; 128^3: 18.5 at 4, 20.5 at 8 and at 2).  From 16 planes on a
+// launch takes whole waves (512^3: 789 to 800 us between 17 and 64 planes, 820
+// and more beyond).
+int fx_fill_chunk(long tile_planes, bool rhs) {
+  const long n = rhs ? resident<true>() : resident<false>();
+  return n > 0 ? (int)((3 * tile_planes + 5 * n - 1) / (5 * n)) : 16;
+}
+
+bool fx_usable(bool rhs) { return rhs ? usable<true>() : usable<false>(); }
+
+cudaError_t launch_fx(double *u_new, const double *u_old, const unsigned long long *K,
+                      const double *rhs, const heat_geom &g, int *err, cudaStream_t st,
+                      unsigned wait_limit) {
+  Maps m;
+  std::memset(&m.r, 0, sizeof m.r);
+  if (!encode(&m.u, u_old, g, BX, BY) || !encode(&m.k, K, g, BX, BY) ||
+      (rhs && !encode(&m.r, rhs, g, TX, TY)))
+    return cudaErrorInvalidValue;
+  if (wait_limit > kWaitLimit) wait_limit = kWaitLimit;
+  if (!fx_usable(rhs != nullptr)) return cudaErrorInvalidConfiguration;
+  return rhs ? launch<true>(m, u_new, u_old, K, g, err, st, wait_limit)
+             : launch<false>(m, u_new, u_old, K, g, err, st, wait_limit);
+}
+
+bool encode_fx_maps(CUtensorMap *m4, double *const u[2], const unsigned long long *K,
+                    const double *rhs, const heat_geom &g) {
+  if (!rhs) std::memset(&m4[3], 0, sizeof m4[3]);
+  return encode(&m4[0], u[0], g, BX, BY) && encode(&m4[1], u[1], g, BX, BY) &&
+         encode(&m4[2], K, g, BX, BY) && (!rhs || encode(&m4[3], rhs, g, TX, TY));
+}
+
+cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int ntiles, bool rhs,
+                            int flip, cudaStream_t st) {
+  if (ntiles <= 0) return cudaSuccess;
+  if (!fx_usable(rhs)) return cudaErrorInvalidConfiguration;
+  if (rhs)
+    k_batch_fx<true><<<ntiles, NT, smem_bytes<true>(), st>>>(grids, tiles, flip);
+  else
+    k_batch_fx<false><<<ntiles, NT, smem_bytes<false>(), st>>>(grids, tiles, flip);
+  return cudaGetLastError();
+}
+
+}  // namespace heat

@@ -36,8 +36,7 @@ struct heat_ctx {
   double *ks[3];            // face kappa sums kx, ky, kz (bit-exact kernel)
   double *c0;               // centre weight 1 - sum of face weights (fast, FP64 pipe)
   double *cf[3];            // face weights factor*(kappa_a+kappa_b) (fast, FP64 pipe)
-  unsigned long long *kq;   // round(factor*kappa*2^64) (fast, integer pipes)
-  int hw_rows;              // warps per block on the FP64 pipe in the hybrid kernel
+  unsigned long long *kq;   // factor*kappa as fixed-point limbs (default form; NULL: FP64 pipe)
 
   // FP32C state.
   float *v[2];              // FP32 fields
@@ -147,29 +146,18 @@ cudaError_t launch_fast(double *u_new, const double *u_old, const double *rhs,
                         const double *c0, double *const cf[3], const heat_geom &g,
                         cudaStream_t st);
 
-// heat_fp64_int.cu
-// K and c0, cx, cy, cz in one pass (the two kernels below, fused; same values).
-cudaError_t launch_weights_setup(unsigned long long *K, double *c0, double *const cf[3], int *bad,
-                                 const double *kappa, const heat_geom &g, double factor,
-                                 cudaStream_t st);
+// heat_fp64_weights.cu: the default form's fixed-point weights; bad[0] (zeroed
+// by the caller) is set when the form cannot represent the problem.
 cudaError_t launch_kq_setup(unsigned long long *K, int *bad, const double *kappa,
                             const heat_geom &g, double factor, cudaStream_t st);
-// hw_rows of the 8 warps in each block take the FP64 pipe, the rest the
-// integer pipes; K may be NULL only when hw_rows == 8, c0/cf only when 0.
-// err: the context's flag, set when a bounded wait of the TMA-staged kernel
-// runs out (HEAT_ETIMEOUT).
-cudaError_t launch_fast_mix(double *u_new, const double *u_old, const double *rhs,
-                            const unsigned long long *K, const double *c0,
-                            double *const cf[3], const heat_geom &g, int hw_rows,
-                            int *err, cudaStream_t st);
 
-// heat_fp64_tma.cu: the hw_rows = 4 split with every input staged by TMA
-// (bit-identical to the k_fast_ws launch), with or without a source term.
-bool fast_tma_usable(const heat_geom &g, bool rhs = false);
-cudaError_t launch_fast_tma(double *u_new, const double *u_old, const unsigned long long *K,
-                            const double *c0, double *const cf[3], const double *rhs,
-                            const heat_geom &g, int *err, cudaStream_t st,
-                            unsigned wait_limit = kWaitLimit);
+// heat_fp64_fx.cu: one step of the default form (fixed point, TMA-staged), with
+// or without a source term.  err: the context's flag, set when a bounded wait
+// runs out (HEAT_ETIMEOUT).
+bool fx_usable(bool rhs);
+cudaError_t launch_fx(double *u_new, const double *u_old, const unsigned long long *K,
+                      const double *rhs, const heat_geom &g, int *err, cudaStream_t st,
+                      unsigned wait_limit = kWaitLimit);
 // n steps of context c from buffer `cur` on stream st with its own
 // single-grid kernels (two steps per launch where its form has them); the
 // context's bookkeeping is untouched.  ctx_flips gives the parity of buffer

@@ -136,7 +136,7 @@ int form_of(int precision, unsigned flags) {
   if (precision == HEAT_FP32C) return heat::kFormF32c;
   if (flags & HEAT_BITEXACT) return heat::kFormExact;
   if (flags & HEAT_HWFP64) return heat::kFormHw;
-  return heat::kFormMix;
+  return heat::kFormFx;
 }
 
 // GLUP/s of a batch of identical grids with the choices ch.

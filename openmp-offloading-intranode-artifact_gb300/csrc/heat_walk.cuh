@@ -202,71 +202,9 @@ __device__ __forceinline__ double int_point(const Dec &dc, const Dec &du, const 
                     Kn, Ks, Ku, Kd);
 }
 
-// Column state of the integer-pipe walk: one (i, j) column, advanced one
-// plane per step(); the next plane's loads are issued one step ahead.
-template <bool RHS>
-struct IntCol {
-  size_t c;
-  u64 bd, bc, Kd, Kc;
-  Dec dd, dc;
-  u64 nu, ne, nw, nn, ns, mu, me, mw, mn, ms;
-
-  __device__ __forceinline__ void fetch(const u64 *__restrict__ ub, const u64 *__restrict__ K,
-                                        int P, size_t S, size_t q) {
-    nu = ub[q + S]; ne = ub[q + 1]; nw = ub[q - 1]; nn = ub[q + P]; ns = ub[q - P];
-    mu = K[q + S]; me = K[q + 1]; mw = K[q - 1]; mn = K[q + P]; ms = K[q - P];
-  }
-
-  __device__ __forceinline__ void start(const u64 *__restrict__ ub, const u64 *__restrict__ K,
-                                        int P, size_t S, size_t c_) {
-    c = c_;
-    bd = ub[c - S];
-    bc = ub[c];
-    dd = decode(bd);
-    dc = decode(bc);
-    Kd = K[c - S];
-    Kc = K[c];
-    fetch(ub, K, P, S, c);
-  }
-
-  // Writes the new value of plane c and moves to the next plane; `more`
-  // says whether a next plane follows (its loads are issued now).
-  __device__ __forceinline__ void step(double *__restrict__ un, const u64 *__restrict__ ub,
-                                       const double *__restrict__ rhs,
-                                       const u64 *__restrict__ K, int P, size_t S, bool more) {
-    const u64 bu = nu, be = ne, bw = nw, bn = nn, bs = ns;
-    const u64 Ku = mu, Ke = me, Kw = mw, Kn = mn, Ks = ms;
-    if (more) fetch(ub, K, P, S, c + S);
-    const Dec du = decode(bu), de = decode(be), dw = decode(bw), dn = decode(bn), ds = decode(bs);
-    const u64 br = RHS ? (u64)__double_as_longlong(rhs[c]) : 0ull;
-    const u64 bcc = bc, bdd = bd;
-    un[c] = int_point<RHS>(dc, du, dd, de, dw, dn, ds, Kc, Ku, Kd, Ke, Kw, Kn, Ks, br,
-                                [=] { return Raw7{bcc, be, bw, bn, bs, bu, bdd}; });
-    bd = bc;
-    bc = bu;
-    dd = dc;
-    dc = du;
-    Kd = Kc;
-    Kc = Ku;
-    c += S;
-  }
-};
-
-// The integer-pipe walk over one (i, j) column, planes [kb, ke).
-template <bool RHS>
-__device__ __forceinline__ void walk_int(double *__restrict__ un, const u64 *__restrict__ ub,
-                                         const double *__restrict__ rhs,
-                                         const u64 *__restrict__ K, int P, size_t S,
-                                         size_t c, int kb, int ke) {
-  IntCol<RHS> col;
-  col.start(ub, K, P, S, c);
-  for (int k = kb; k < ke; ++k) col.step(un, ub, rhs, K, P, S, k + 1 < ke);
-}
-
 // Column state of the FP64-pipe walk (precomputed double weights, 7 FMA per
-// point).  The plane's loads are issued one step ahead: next to the integer
-// warps of the hybrid launch these warps are few, and would otherwise wait
-// on memory instead of keeping the FP64 pipe busy.
+// point).  The plane's loads are issued one step ahead, so they overlap the
+// arithmetic.
 template <bool RHS>
 struct HwCol {
   size_t c;
@@ -333,9 +271,8 @@ struct HwCol {
   }
 };
 
-// The FP64-pipe walk over one (i, j) column, planes [kb, ke); the plane loop
-// unrolled UNROLL times.
-template <bool RHS, int UNROLL = 1>
+// The FP64-pipe walk over one (i, j) column, planes [kb, ke).
+template <bool RHS>
 __device__ __forceinline__ void walk_hw(double *__restrict__ un, const double *__restrict__ u,
                                         const double *__restrict__ rhs,
                                         const double *__restrict__ c0,
@@ -345,11 +282,6 @@ __device__ __forceinline__ void walk_hw(double *__restrict__ un, const double *_
                                         size_t c, int kb, int ke) {
   HwCol<RHS> col;
   col.start(u, rhs, c0, cx, cy, cz, P, S, c);
-  // Unrolled by 2, the prefetch registers alternate instead of being copied
-  // into the working ones each plane: k_fast_ws without a source term asks
-  // for it (512^3: 114 GLUP/s against 111.5; by 3 or 4 no gain).  The batch
-  // kernels do not: there it adds spills (k_batch_ws 288 B against 184).
-#pragma unroll (UNROLL)
   for (int k = kb; k < ke; ++k) col.step(un, u, rhs, c0, cx, cy, cz, P, S, k + 1 < ke);
 }
 

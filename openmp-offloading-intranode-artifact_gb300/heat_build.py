@@ -77,7 +77,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             for f in [ex.submit(_run, j) for j in jobs]:
                 f.result()
-    objs = sorted(OBJ.glob("*.o"))
+    # Only the objects of sources that are there: _build may hold others' leftovers.
+    objs = sorted(OBJ / (src.name + ".o") for pat in ("*.cu", "*.cpp") for src in CSRC.glob(pat))
     if force or jobs or _stale(LIB, objs):
         _run([nvcc, *ARCH, "-shared", "-o", str(LIB), *map(str, objs), "-lpthread", "-ldl"])
     drv_src = PKG / "driver" / "heatdrv.c"
