@@ -18,9 +18,10 @@
 //     is negative, rounded up to an even number) gives the scale E: a value
 //     becomes the integer A = value * 2^(1083 - E), |A| < 2^61.
 //   * If no nonzero value of the patch itself (three planes) lies more than
-//     kSlack = 6 binary orders below E, those A are exact (8 orders would be), and
-//     one unit of A is at most 1/4 ulp of the smallest of them.  A neighbour
-//     further below is cut to whole units, an error of one unit times its weight.
+//     kSlack = 8 binary orders below E, those A are exact.  A neighbour further
+//     below is cut to whole units, an error of one unit times its weight; a
+//     result below 2^53 units, where a unit is more than 1/2 ulp, is formed anew
+//     point by point.
 //   * Weights come from the per-point K = factor * kappa, kept as two limbs
 //     K = k1 2^-32 + k0 2^-63 with |k0| <= 2^30: a face weight is the two limb
 //     sums, no carry, and its low limb is a signed 32-bit number.
@@ -36,33 +37,34 @@
 // constant region stays exactly constant (every D is 0).
 //
 // Patches outside those bounds (a wider range of magnitudes, exponents near
-// either end, infinities, NaNs) take walk::int_point per point, which aligns
-// each point's seven values to their own largest exponent.  Which of the two a
-// patch takes, and E, depend only on the field's values in its region, never on
-// tiles or z-chunks, so a grid's results are the same bits in any launch.
-// (kSlack: of a Gaussian of width 0.05 on 512^3, whose tails fall by up to one
-// binary order per point, no patch is outside it; 16 x 8-point patches would
-// leave 70 % of the grid outside.)
+// either end, infinities, NaNs) go point by point, each at the largest exponent
+// of its own seven values.  Which of the two a patch takes, and E, depend only on
+// the field's values in its region, never on tiles or z-chunks, so a grid's
+// results are the same bits in any launch.
+// (Patches are small so that steep fields fit: of a Gaussian of width 0.05 on
+// 512^3, whose tails fall by up to one binary order per point, no patch is
+// outside the bounds; of 16 x 8-point patches 40 % would be.)
 //
 // The integers carried along z move to a new scale by shifting, which is exact
 // because both scales hold the patch exactly.
 //
 // Staging: a block is 32 x 16 columns (128 threads, 16 x 8 patches).  Planes of
-// u and K (and the source term) land by TMA in a 4-deep ring, boxes 36 x 18
+// u and K (and the source term) land by TMA in a ring 4 deep (3), boxes 36 x 18
 // from column i0 - 2 (16-byte aligned), each slot completing on its own
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 167 GLUP/s (0.79 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 165 GLUP/s (0.80 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 139 (115.7).
-// About 137 warp instructions per point (300 for an integer row of that
+// the launch before this one), with the reference's source term 146 (115.7).
+// About 139 warp instructions per point (300 for an integer row of that
 // launch); ALU, FMA-heavy (18 of its instructions the wide multiply-adds, twice
 // the cost of the others) and issue are each about 60 % busy, DRAM 55 %.
 // Measured and not kept: the neighbours above and below converted by the FP64
-// pipe as the patch's own are (157; that pipe is then at 75 % and the others wait
-// for it), no value converted by it (164), five blocks per SM at 96 registers
-// (165), 32 x 32 tiles (156), 64 x 8 (166), the plane loop unrolled by 2 (162).
+// pipe as the patch's own are (157 when this was 167; that pipe is then at 75 %
+// and the others wait for it), no value converted by it (164), five blocks per SM
+// at 96 registers (165), 32 x 32 tiles (156), 64 x 8 (166), the plane loop
+// unrolled by 2 (162).
 //
 // Every mbarrier wait is bounded: a wait that runs out stops the block at the
 // next barrier (the flag is OR-reduced), thread 0 waits (bounded) for its loads
@@ -256,9 +258,12 @@ struct Acc {
 // vd below it and the limbs of the weight to it.  The same arithmetic at the
 // point's own scale, the largest exponent of its seven values (and the source
 // term), every value cut to that scale's units; exponents near either end,
-// infinities and NaNs take walk::int_point.  pd: the value below in global
+// infinities and NaNs take walk::int_point.  PLAIN: no value is negative.  A
+// whole grid of such points runs at 99 GLUP/s (512^3; 87 with signs always).  A
+// function of its own: inlined, or four points to a call, they run at 119 and
+// 112, but the fast form, scheduled around them, at 144 and 142 for 164.  pd: the value below in global
 // memory (vd may have read a subnormal as 0).
-template <bool RHS>
+template <bool RHS, bool PLAIN>
 __device__ __noinline__ double point(const Slot<RHS> &sk, const Slot<RHS> &sn, int p, int prhs,
                                      u64 vd, unsigned w0, unsigned w1, const u64 *pd) {
   const u64 c = sk.u[p], f[6] = {sn.u[p], vd, sk.u[p - 1], sk.u[p + 1], sk.u[p - BX], sk.u[p + BX]};
@@ -273,9 +278,12 @@ __device__ __noinline__ double point(const Slot<RHS> &sk, const Slot<RHS> &sn, i
   }
   const u64 kc = sk.k[p];
   const u64 k[6] = {sn.k[p], 0, sk.k[p - 1], sk.k[p + 1], sk.k[p - BX], sk.k[p + BX]};
-  const unsigned E = r.mx + ((int)r.sg < 0 ? kExp : 0u);
+  const unsigned E = r.mx + (!PLAIN && (int)r.sg < 0 ? kExp : 0u);
   if (E - kLowE <= kHighE - kLowE) {
-    auto load = [&](u64 v) { return with_sign(magnitude(v, E), v); };
+    auto load = [&](u64 v) {
+      const u64 m = magnitude(v, E);
+      return PLAIN ? m : with_sign(m, v);
+    };
     const u64 A = load(c);
     Acc a(A);
 #pragma unroll
@@ -522,7 +530,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           double *wq = w + ((q & 2 ? P : 0) + (q & 1));
           const u64 *pd = u + (wq - un) - S;
           const u64 Kc = sk.k[p], Kd = K[pd - u];
-          *wq = point<RHS>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), *pd,
+          *wq = point<RHS, false>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), *pd,
                            (unsigned)Kc + (unsigned)Kd,
                            (unsigned)(Kc >> 32) + (unsigned)(Kd >> 32), pd);
         }
@@ -537,8 +545,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             E ? (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E)) : A1[q];
         if ((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0)) {
           double *wq = w + ((q & 2 ? P : 0) + (q & 1));
-          *wq = point<RHS>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), below, W0[q],
-                           W1[q], u + (wq - un) - S);
+          const int pr = (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1);
+          const u64 *pd = u + (wq - un) - S;
+          *wq = (int)r.sg >= 0 ? point<RHS, true>(sk, sn, p, pr, below, W0[q], W1[q], pd)
+                               : point<RHS, false>(sk, sn, p, pr, below, W0[q], W1[q], pd);
         }
         A1[q] = sk.u[p];
         const u64 Kc = sk.k[p], Ku = sn.k[p];
