@@ -136,6 +136,7 @@ void free_ctx(heat_ctx *c) {
 // with the kernel its form selects; the context's bookkeeping is untouched.
 cudaError_t enqueue_one(heat_ctx *c, int cur, cudaStream_t st) {
   const heat_geom &g = c->g;
+  if (c->kq) return heat::launch_fx(c, cur, st);
   double *uo = c->u[cur], *un = c->u[cur ^ 1];
   if (c->precision == HEAT_FP32C)
     return heat::launch_fp32c(c->v[cur ^ 1], c->carry[cur ^ 1], c->v[cur], c->carry[cur], c->fcf,
@@ -143,8 +144,6 @@ cudaError_t enqueue_one(heat_ctx *c, int cur, cudaStream_t st) {
   if (c->flags & HEAT_NAIVE) return heat::launch_naive(un, uo, c->rhs, c->kappa, g, c->factor, st);
   if (c->flags & HEAT_BITEXACT)
     return heat::launch_exact_faces(un, uo, c->rhs, c->ks, g, c->factor, st);
-  if (c->kq)
-    return heat::launch_fx(un, uo, c->kq, c->rhs, g, c->err, st);
   return heat::launch_fast(un, uo, c->rhs, c->c0, c->cf, g, st);
 }
 
@@ -283,6 +282,7 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
     bool fixed = !(c->flags & HEAT_HWFP64) && heat::fx_usable(d->rhs != nullptr);
     if (fixed) {
       TRY(dalloc(&c->kq, g.elems, c->stream));
+      fixed = heat::encode_fx_maps(c->maps, c->u, c->kq, c->rhs, g);
       int bad = 0;
       int *d_bad = reinterpret_cast<int *>(c->partials);
       cudaError_t e = cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream);
@@ -292,7 +292,7 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) { rc = cuda_fail(e, "fixed-point setup"); goto done; }
       c->launches += 2;
-      if (bad) {
+      if (bad || !fixed) {
         cudaFreeAsync(c->kq, c->stream);
         c->kq = nullptr;
         fixed = false;
@@ -334,6 +334,7 @@ int init_fp32c(heat_ctx *c, const heat_desc *d) {
     TRY(dalloc(&c->carry[b], g.elems, c->stream));
   }
   for (int a = 0; a < 3; ++a) TRY(dalloc(&c->fcf[a], g.elems, c->stream));
+  c->have_maps = heat::encode_fp32c_maps(c->maps, c->v, c->carry, c->fcf, g);
   TRY(dalloc(&c->partials, 2 * heat::kNormBlocks + 2, c->stream));
   c->n_partials = heat::kNormBlocks;
   TRY(dalloc(&c->err, 1, c->stream));
@@ -392,8 +393,7 @@ int cuda_fail(cudaError_t e, const char *what) {
 }
 
 bool two_step_form(const heat_ctx *c) {
-  return c->precision == HEAT_FP32C && !c->frhs && !(c->flags & HEAT_NO_TEMPORAL) &&
-         fp32c_tb2_ok(c->g);
+  return c->precision == HEAT_FP32C && !c->frhs && !(c->flags & HEAT_NO_TEMPORAL) && c->have_maps;
 }
 
 int check_err(heat_ctx *c) {
@@ -415,8 +415,7 @@ cudaError_t enqueue_ctx_steps(heat_ctx *c, int cur, long long n, cudaStream_t st
   if (two_step_form(c))
     for (; s + 2 <= n && e == cudaSuccess; s += 2) {
       // two steps per launch: the result lands in the other buffer
-      e = launch_fp32c_tb2(c->v[cur ^ 1], c->carry[cur ^ 1], c->v[cur], c->carry[cur], c->fcf, c->g,
-                           c->err, st);
+      e = launch_fp32c_tb2(c, cur, st);
       cur ^= 1;
       if (launches) ++*launches;
     }
@@ -507,8 +506,7 @@ int heat_step(heat_ctx *c, int nsteps) {
   if (two_step_form(c)) {
     // Two steps per launch; the result lands in the other buffer.
     for (; s + 2 <= nsteps; s += 2) {
-      cudaError_t e = heat::launch_fp32c_tb2(c->v[c->cur ^ 1], c->carry[c->cur ^ 1], c->v[c->cur],
-                                             c->carry[c->cur], c->fcf, c->g, c->err, c->stream);
+      cudaError_t e = heat::launch_fp32c_tb2(c, c->cur, c->stream);
       if (e != cudaSuccess) return cuda_fail(e, "two-step kernel launch");
       c->launches += 1;
       c->cur ^= 1;
@@ -656,8 +654,7 @@ int heat_diag_fp32c_timeout(heat_ctx *c) {
   // wait gives up, it sets the context's error flag, drains its own loads in
   // flight (with the full bounded wait) and returns without writing a point.
   // The context's buffers and step count are left as they were.
-  cudaError_t e = heat::launch_fp32c_tb2(c->v[c->cur ^ 1], c->carry[c->cur ^ 1], c->v[c->cur],
-                                         c->carry[c->cur], c->fcf, c->g, c->err, c->stream, 0u);
+  cudaError_t e = heat::launch_fp32c_tb2(c, c->cur, c->stream, 0u);
   if (e != cudaSuccess) return cuda_fail(e, "two-step kernel launch");
   c->launches += 1;
   return HEAT_OK;
@@ -667,8 +664,7 @@ int heat_diag_fp64_timeout(heat_ctx *c) {
   if (!c) return HEAT_EINVAL;
   // Only contexts that step with the TMA-staged default FP64 launch.
   if (c->precision != HEAT_FP64 || !c->kq) return HEAT_ESTATE;
-  cudaError_t e = heat::launch_fx(c->u[c->cur ^ 1], c->u[c->cur], c->kq, c->rhs, c->g, c->err,
-                                  c->stream, 0u);
+  cudaError_t e = heat::launch_fx(c, c->cur, c->stream, 0u);
   if (e != cudaSuccess) return cuda_fail(e, "default FP64 kernel launch");
   c->launches += 1;
   return HEAT_OK;

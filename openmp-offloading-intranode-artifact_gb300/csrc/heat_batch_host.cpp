@@ -292,8 +292,7 @@ int rebuild(heat_batch *b) {
       b->pairs.push_back((int)e);
       map_at.push_back({gi, (int)maps.size()});
       maps.resize(maps.size() + 7);
-      if (!heat::encode_fp32c_maps(&maps[maps.size() - 7], c->v, c->carry, c->fcf, c->g))
-        return HEAT_ECUDA;
+      std::copy(c->maps, c->maps + 7, maps.end() - 7);
       // two steps per 32 x 16 tile; the temporal blocking wants long z-walks
       kc = std::max(kc, std::min(16, interior));
       rows = 1;
@@ -303,8 +302,7 @@ int rebuild(heat_batch *b) {
     if (form == heat::kFormFx) {
       map_at.push_back({gi, (int)maps.size()});
       maps.resize(maps.size() + 4);
-      if (!heat::encode_fx_maps(&maps[maps.size() - 4], c->u, c->kq, c->rhs, c->g))
-        return HEAT_ECUDA;
+      std::copy(c->maps, c->maps + 4, maps.end() - 4);
       // A small table fills the GPU with shorter tiles than the tuned ones.
       kc = std::min(kc, std::max(1, heat::fx_fill_chunk(fx_planes[c->rhs != nullptr], c->rhs)));
       rows = 1;

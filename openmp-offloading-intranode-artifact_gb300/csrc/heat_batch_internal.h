@@ -61,8 +61,8 @@ inline int form_of_kind(int kind) { return kind / (2 * kNumMinb); }
 cudaError_t launch_batch(int kind, const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                          int flip, int blocks, cudaStream_t st);
 int batch_blocks_per_sm(int kind);
-// heat_fp64_fx.cu: the default FP64 form's table kernel, its tiles per axis,
-// their depth and its per-grid maps.
+// heat_fp64_fx.cu: the default FP64 form's table kernel, its tiles per axis and
+// their depth.
 cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int ntiles, bool rhs,
                             int flip, cudaStream_t st);
 int fx_tiles_x(int nx);
@@ -70,13 +70,9 @@ int fx_tiles_y(int ny);
 // Planes per block that fill the GPU with blocks for a launch of tile_planes
 // planes of tiles in all; long launches want no longer chunks than 16 or so.
 int fx_fill_chunk(long tile_planes, bool rhs);
-bool encode_fx_maps(CUtensorMap *m4, double *const u[2], const unsigned long long *K,
-                    const double *rhs, const heat_geom &g);
-// heat_fp32c_tma.cu: the two-step FP32C table kernel and its per-grid maps.
+// heat_fp32c_tma.cu: the two-step FP32C table kernel.
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                                    int flip, cudaStream_t st);
-bool encode_fp32c_maps(CUtensorMap *m7, float *const v[2], uint16_t *const c[2],
-                       float *const w[3], const heat_geom &g);
 
 // Form of a context in the batch kernel, or -1 if the batch cannot run it.
 int batch_form(const heat_ctx *c);

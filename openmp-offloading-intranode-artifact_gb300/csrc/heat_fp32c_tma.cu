@@ -125,6 +125,7 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     for (int s = 0; s < R; ++s) mbar_init(&sm.bar[s]);
     tma::mbar_init_fence();
   }
+  chain();
   __syncthreads();
 
   // Warp 0 keeps the bookkeeping (which slots have a load in flight, and each
@@ -367,32 +368,22 @@ cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tile
       cudaFuncSetAttribute(k_batch_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)fp32c_tb2_smem()) == cudaSuccess;
   if (!attr) return cudaErrorInvalidConfiguration;
-  k_batch_fp32c_tb2<<<ntiles, NT, fp32c_tb2_smem(), st>>>(grids, tiles, flip);
-  return cudaGetLastError();
+  return launch_chained(k_batch_fp32c_tb2, ntiles, NT, fp32c_tb2_smem(), st, grids, tiles, flip);
 }
 
-bool encode_fp32c_maps(CUtensorMap *m7, float *const v[2], uint16_t *const c[2],
+// False where the row and plane strides are not multiples of 16 bytes, which TMA
+// wants (pitch a multiple of 8 points), or the encoder is missing.
+bool encode_fp32c_maps(CUtensorMap *m, float *const v[2], uint16_t *const cr[2],
                        float *const w[3], const heat_geom &g) {
-  return encode(&m7[0], v[0], false, g) && encode(&m7[1], v[1], false, g) &&
-         encode(&m7[2], c[0], true, g) && encode(&m7[3], c[1], true, g) &&
-         encode(&m7[4], w[0], false, g) && encode(&m7[5], w[1], false, g) &&
-         encode(&m7[6], w[2], false, g);
+  return g.pitch % 8 == 0 && encode(&m[0], v[0], false, g) && encode(&m[1], v[1], false, g) &&
+         encode(&m[2], cr[0], true, g) && encode(&m[3], cr[1], true, g) &&
+         encode(&m[4], w[0], false, g) && encode(&m[5], w[1], false, g) &&
+         encode(&m[6], w[2], false, g);
 }
 
-// Whether the two-step kernel can run this geometry: row and plane strides in
-// bytes must be multiples of 16 for TMA (pitch a multiple of 8 points).
-bool fp32c_tb2_ok(const heat_geom &g) {
-  return (g.pitch % 8) == 0 && g.nx >= 3 && tma::encoder() != nullptr;
-}
-
-cudaError_t launch_fp32c_tb2(float *v_new, uint16_t *c_new, const float *v, const uint16_t *cr,
-                             float *const w[3], const heat_geom &g, int *err, cudaStream_t st,
-                             unsigned wait_limit) {
+cudaError_t launch_fp32c_tb2(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
   if (wait_limit > tma::kWaitLimit) wait_limit = tma::kWaitLimit;
-  Maps m;
-  if (!encode(&m.v, v, false, g) || !encode(&m.c, cr, true, g) || !encode(&m.wx, w[0], false, g) ||
-      !encode(&m.wy, w[1], false, g) || !encode(&m.wz, w[2], false, g))
-    return cudaErrorInvalidValue;
+  const heat_geom &g = c->g;
   static bool attr = cudaFuncSetAttribute(k_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)fp32c_tb2_smem()) == cudaSuccess;
   if (!attr) return cudaErrorInvalidConfiguration;
@@ -405,9 +396,10 @@ cudaError_t launch_fp32c_tb2(float *v_new, uint16_t *c_new, const float *v, cons
   static const long resident = resident_blocks((const void *)k_fp32c_tb2, NT, fp32c_tb2_smem());
   const int kchunk = wave_chunk(g, OX, OY, resident, 24, 96, 16);
   dim3 grid(bx, by, (interior + kchunk - 1) / kchunk);
-  k_fp32c_tb2<<<grid, NT, fp32c_tb2_smem(), st>>>(m, v_new, c_new, g.nx, g.ny, g.nz, g.pitch,
-                                                  g.plane, kchunk, err, wait_limit);
-  return cudaGetLastError();
+  return launch_chained(k_fp32c_tb2, grid, NT, fp32c_tb2_smem(), st,
+                        Maps{c->maps[cur], c->maps[2 + cur], c->maps[4], c->maps[5], c->maps[6]},
+                        c->v[cur ^ 1], c->carry[cur ^ 1], g.nx, g.ny, g.nz, g.pitch, g.plane,
+                        kchunk, c->err, wait_limit);
 }
 
 }  // namespace heat

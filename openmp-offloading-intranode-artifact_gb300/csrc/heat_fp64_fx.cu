@@ -296,7 +296,7 @@ __device__ __noinline__ double point(const Slot<RHS> &sk, const Slot<RHS> &sn, i
     if constexpr (RHS) a.add(vr, E);
     return scaled(a.rounded(), E);
   }
-  const u64 ud = *pd;
+  const u64 ud = __ldcg(pd);
   if (((c | f[0] | ud | f[2] | f[3] | f[4] | f[5] | vr) << 1) == 0) return 0.0;
   // K in units of 2^-64, as int_point takes it; the one below from the face's limbs
   auto weight = [](unsigned k0, unsigned k1) {
@@ -335,6 +335,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     for (int s = 0; s < kRing<RHS>; ++s) tma::mbar_init(&sm.bar[s]);
     tma::mbar_init_fence();
   }
+  chain();
   __syncthreads();
   auto issue = [&](int p, int s) {
     if (t != 0 || p > ke) return;
@@ -530,7 +531,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           double *wq = w + ((q & 2 ? P : 0) + (q & 1));
           const u64 *pd = u + (wq - un) - S;
           const u64 Kc = sk.k[p], Kd = K[pd - u];
-          *wq = point<RHS, false>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), *pd,
+          *wq = point<RHS, false>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), __ldcg(pd),
                            (unsigned)Kc + (unsigned)Kd,
                            (unsigned)(Kc >> 32) + (unsigned)(Kd >> 32), pd);
         }
@@ -637,15 +638,16 @@ long resident() {
 }
 
 template <bool RHS>
-cudaError_t launch(const Maps &m, double *u_new, const double *u_old, const u64 *K,
-                   const heat_geom &g, int *err, cudaStream_t st, unsigned wait_limit) {
+cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
+  const heat_geom &g = c->g;
   const int interior = g.nz - 2;
   int kc = fx_fill_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny) * interior, RHS);
   kc = kc >= 16 ? wave_chunk(g, TX, TY, resident<RHS>()) : kc < interior ? kc : interior;
   dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
-  k_fx<RHS><<<gr, NT, smem_bytes<RHS>(), st>>>(m, u_new, (const u64 *)u_old, K, g.nx, g.ny, g.nz,
-                                               g.pitch, g.plane, kc, err, wait_limit);
-  return cudaGetLastError();
+  return launch_chained(k_fx<RHS>, gr, NT, smem_bytes<RHS>(), st,
+                        Maps{c->maps[cur], c->maps[2], c->maps[3]}, c->u[cur ^ 1],
+                        (const u64 *)c->u[cur], c->kq, g.nx, g.ny, g.nz, g.pitch, g.plane, kc,
+                        c->err, wait_limit);
 }
 
 }  // namespace
@@ -668,36 +670,26 @@ int fx_fill_chunk(long tile_planes, bool rhs) {
 
 bool fx_usable(bool rhs) { return rhs ? usable<true>() : usable<false>(); }
 
-cudaError_t launch_fx(double *u_new, const double *u_old, const unsigned long long *K,
-                      const double *rhs, const heat_geom &g, int *err, cudaStream_t st,
-                      unsigned wait_limit) {
-  Maps m;
-  std::memset(&m.r, 0, sizeof m.r);
-  if (!encode(&m.u, u_old, g, BX, BY) || !encode(&m.k, K, g, BX, BY) ||
-      (rhs && !encode(&m.r, rhs, g, TX, TY)))
-    return cudaErrorInvalidValue;
-  if (wait_limit > kWaitLimit) wait_limit = kWaitLimit;
-  if (!fx_usable(rhs != nullptr)) return cudaErrorInvalidConfiguration;
-  return rhs ? launch<true>(m, u_new, u_old, K, g, err, st, wait_limit)
-             : launch<false>(m, u_new, u_old, K, g, err, st, wait_limit);
+bool encode_fx_maps(CUtensorMap *m, double *const u[2], const unsigned long long *K,
+                    const double *rhs, const heat_geom &g) {
+  if (!rhs) std::memset(&m[3], 0, sizeof m[3]);
+  return encode(&m[0], u[0], g, BX, BY) && encode(&m[1], u[1], g, BX, BY) &&
+         encode(&m[2], K, g, BX, BY) && (!rhs || encode(&m[3], rhs, g, TX, TY));
 }
 
-bool encode_fx_maps(CUtensorMap *m4, double *const u[2], const unsigned long long *K,
-                    const double *rhs, const heat_geom &g) {
-  if (!rhs) std::memset(&m4[3], 0, sizeof m4[3]);
-  return encode(&m4[0], u[0], g, BX, BY) && encode(&m4[1], u[1], g, BX, BY) &&
-         encode(&m4[2], K, g, BX, BY) && (!rhs || encode(&m4[3], rhs, g, TX, TY));
+cudaError_t launch_fx(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
+  if (!fx_usable(c->rhs != nullptr)) return cudaErrorInvalidConfiguration;
+  if (wait_limit > kWaitLimit) wait_limit = kWaitLimit;
+  return c->rhs ? launch<true>(c, cur, st, wait_limit) : launch<false>(c, cur, st, wait_limit);
 }
 
 cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int ntiles, bool rhs,
                             int flip, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
   if (!fx_usable(rhs)) return cudaErrorInvalidConfiguration;
-  if (rhs)
-    k_batch_fx<true><<<ntiles, NT, smem_bytes<true>(), st>>>(grids, tiles, flip);
-  else
-    k_batch_fx<false><<<ntiles, NT, smem_bytes<false>(), st>>>(grids, tiles, flip);
-  return cudaGetLastError();
+  return rhs ? launch_chained(k_batch_fx<true>, ntiles, NT, smem_bytes<true>(), st, grids, tiles, flip)
+             : launch_chained(k_batch_fx<false>, ntiles, NT, smem_bytes<false>(), st, grids, tiles,
+                              flip);
 }
 
 }  // namespace heat

@@ -1,6 +1,7 @@
 // Internal declarations shared by the translation units of libheat.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
@@ -44,6 +45,11 @@ struct heat_ctx {
   float *fcf[3];            // FP32 face weights
   float *frhs;              // FP32 source (NULL when none)
 
+  // Tensor maps of the TMA-staged steps, made once: default FP64 form u0 u1 K rhs,
+  // FP32C two-step form v0 v1 carry0 carry1 wx wy wz.
+  CUtensorMap maps[7];
+  bool have_maps;
+
   // Device flag a kernel sets when a bounded wait ran out (HEAT_ETIMEOUT).
   int *err;
 
@@ -69,6 +75,37 @@ __device__ __forceinline__ double fw(double factor, double ka, double kb) {
 __device__ __forceinline__ double centre(double e, double w, double n, double s, double u,
                                          double d) {
   return __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(e, w), n), s), u), d));
+}
+#endif
+
+#ifdef __CUDACC__
+// A TMA-staged step kernel begins with chain(): it lets the next launch of its
+// stream start (blocks set up, waiting in their own chain()) and waits until the
+// launch before it is complete and its results visible.  Nothing may touch a
+// field before it, and its fields are read by TMA or __ldcg only: a kernel that
+// starts beside the one that writes them may not read them through the
+// read-only path, as the column walks' const __restrict__ loads do.
+__device__ __forceinline__ void chain() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
+// Launches a kernel that begins with chain(), so that it may start before the
+// kernel ahead of it on the stream ends.  Launches after it that are not made
+// through here still wait for all of it.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t st, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 #endif
 
@@ -151,12 +188,13 @@ cudaError_t launch_fast(double *u_new, const double *u_old, const double *rhs,
 cudaError_t launch_kq_setup(unsigned long long *K, int *bad, const double *kappa,
                             const heat_geom &g, double factor, cudaStream_t st);
 
-// heat_fp64_fx.cu: one step of the default form (fixed point, TMA-staged), with
-// or without a source term.  err: the context's flag, set when a bounded wait
-// runs out (HEAT_ETIMEOUT).
+// heat_fp64_fx.cu: one step of the default form (fixed point, TMA-staged) of
+// context c from buffer `cur`.  encode_fx_maps fills m with the maps of a
+// field pair, its weights and source term (NULL: none).
 bool fx_usable(bool rhs);
-cudaError_t launch_fx(double *u_new, const double *u_old, const unsigned long long *K,
-                      const double *rhs, const heat_geom &g, int *err, cudaStream_t st,
+bool encode_fx_maps(CUtensorMap *m, double *const u[2], const unsigned long long *K,
+                    const double *rhs, const heat_geom &g);
+cudaError_t launch_fx(const heat_ctx *c, int cur, cudaStream_t st,
                       unsigned wait_limit = kWaitLimit);
 // n steps of context c from buffer `cur` on stream st with its own
 // single-grid kernels (two steps per launch where its form has them); the
@@ -179,12 +217,12 @@ cudaError_t launch_f32_weights(float *const w[3], const double *kappa, const hea
                                double factor, cudaStream_t st);
 cudaError_t launch_to_f32(float *o, const double *a, size_t total, cudaStream_t st);
 
-// heat_fp32c_tma.cu: two steps per launch (temporal blocking, TMA staging).
-// wait_limit bounds every mbarrier wait of the launch (kWaitLimit in product
-// use; smaller only to exercise the failure path).
-bool fp32c_tb2_ok(const heat_geom &g);
-cudaError_t launch_fp32c_tb2(float *v_new, uint16_t *c_new, const float *v, const uint16_t *cr,
-                             float *const w[3], const heat_geom &g, int *err, cudaStream_t st,
+// heat_fp32c_tma.cu: two steps per launch (temporal blocking, TMA staging) of
+// context c from buffer `cur`.  wait_limit bounds every mbarrier wait of the
+// launch (kWaitLimit in product use; smaller only to exercise the failure path).
+bool encode_fp32c_maps(CUtensorMap *m, float *const v[2], uint16_t *const cr[2],
+                       float *const w[3], const heat_geom &g);
+cudaError_t launch_fp32c_tb2(const heat_ctx *c, int cur, cudaStream_t st,
                              unsigned wait_limit = kWaitLimit);
 // Whether a context steps with launch_fp32c_tb2.
 bool two_step_form(const heat_ctx *c);
