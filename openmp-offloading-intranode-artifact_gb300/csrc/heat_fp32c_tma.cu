@@ -368,7 +368,8 @@ cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tile
       cudaFuncSetAttribute(k_batch_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)fp32c_tb2_smem()) == cudaSuccess;
   if (!attr) return cudaErrorInvalidConfiguration;
-  return launch_chained(k_batch_fp32c_tb2, ntiles, NT, fp32c_tb2_smem(), st, grids, tiles, flip);
+  k_batch_fp32c_tb2<<<ntiles, NT, fp32c_tb2_smem(), st>>>(grids, tiles, flip);
+  return cudaGetLastError();
 }
 
 // False where the row and plane strides are not multiples of 16 bytes, which TMA

@@ -530,7 +530,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           const int p = o + (q >> 1) * BX + (q & 1);
           double *wq = w + ((q & 2 ? P : 0) + (q & 1));
           const u64 *pd = u + (wq - un) - S;
-          const u64 Kc = sk.k[p], Kd = K[pd - u];
+          const u64 Kc = sk.k[p], Kd = __ldcg(K + (pd - u));
           *wq = point<RHS, false>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), __ldcg(pd),
                            (unsigned)Kc + (unsigned)Kd,
                            (unsigned)(Kc >> 32) + (unsigned)(Kd >> 32), pd);
@@ -687,9 +687,11 @@ cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int 
                             int flip, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
   if (!fx_usable(rhs)) return cudaErrorInvalidConfiguration;
-  return rhs ? launch_chained(k_batch_fx<true>, ntiles, NT, smem_bytes<true>(), st, grids, tiles, flip)
-             : launch_chained(k_batch_fx<false>, ntiles, NT, smem_bytes<false>(), st, grids, tiles,
-                              flip);
+  if (rhs)
+    k_batch_fx<true><<<ntiles, NT, smem_bytes<true>(), st>>>(grids, tiles, flip);
+  else
+    k_batch_fx<false><<<ntiles, NT, smem_bytes<false>(), st>>>(grids, tiles, flip);
+  return cudaGetLastError();
 }
 
 }  // namespace heat

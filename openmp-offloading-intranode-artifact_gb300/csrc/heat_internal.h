@@ -82,9 +82,11 @@ __device__ __forceinline__ double centre(double e, double w, double n, double s,
 // A TMA-staged step kernel begins with chain(): it lets the next launch of its
 // stream start (blocks set up, waiting in their own chain()) and waits until the
 // launch before it is complete and its results visible.  Nothing may touch a
-// field before it, and its fields are read by TMA or __ldcg only: a kernel that
-// starts beside the one that writes them may not read them through the
-// read-only path, as the column walks' const __restrict__ loads do.
+// field before it.  The L1 caches keep their read-only lines from one chained
+// launch to the next, so such a kernel reads global memory by TMA or __ldcg only:
+// the column-walk kernels (const __restrict__ fields) and the batch kernels
+// (tables, which the host rewrites) have plain launches, before which chain()
+// does nothing.
 __device__ __forceinline__ void chain() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }

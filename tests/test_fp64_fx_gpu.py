@@ -87,3 +87,20 @@ def test_a_constant_field_stays_constant(H, value):
     with H.Solver(kappa, u0, h, dt) as s:
         s.step(25)
         assert bits_equal(s.field(), u0)
+
+
+def test_many_short_requests_of_one_form(H):
+    """The batch's tables are rebuilt while its launches follow each other without
+    a pause: every request still gets its own grid's result."""
+    shapes = [(18 + 7 * (q % 5), 20 + 3 * (q % 7), 12 + 5 * (q % 6)) for q in range(90)]
+    outs = [np.empty(s[::-1]) for s in shapes]
+    with H.Server(8 << 30, tick_steps=4, prep_threads=4) as srv:
+        for q, (s, o) in enumerate(zip(shapes, outs)):
+            srv.submit(*s, steps=5 + q % 37, seed=q, field_out=o)
+        srv.wait_idle()
+        assert all(r["status"] == 0 for r in srv.poll())
+    for q in range(0, 90, 7):
+        kappa, u0, h, dt = H.inputs_config(0, q, *shapes[q])
+        with H.Solver(kappa, u0, h, dt) as a:
+            a.step(5 + q % 37)
+            assert bits_equal(a.field(), outs[q]), q
