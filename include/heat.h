@@ -189,7 +189,7 @@ typedef struct heat_tune_entry {
   int rows;            /* rows per thread: tiles of 32 x (8 * rows) columns  */
   int blocks_per_sm;   /* table kernel variant: 2, 3 or 4 resident blocks    */
   int depth;           /* time steps per launch: 1, or 2 (HEAT_FP32C grids
-                          without a source term, 32 x 16 TMA-staged tiles)   */
+                          without a source term, TMA-staged tiles)   */
 } heat_tune_entry;
 int heat_tune_choice(int precision, unsigned flags, int nz, heat_tune_entry *out);
 

@@ -283,6 +283,7 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
     if (fixed) {
       TRY(dalloc(&c->kq, g.elems, c->stream));
       fixed = heat::encode_fx_maps(c->maps, c->u, c->kq, c->rhs, g);
+      c->kchunk = heat::fx_chunk(g, c->rhs != nullptr);
       int bad = 0;
       int *d_bad = reinterpret_cast<int *>(c->partials);
       cudaError_t e = cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream);
@@ -335,6 +336,7 @@ int init_fp32c(heat_ctx *c, const heat_desc *d) {
   }
   for (int a = 0; a < 3; ++a) TRY(dalloc(&c->fcf[a], g.elems, c->stream));
   c->have_maps = heat::encode_fp32c_maps(c->maps, c->v, c->carry, c->fcf, g);
+  c->kchunk = heat::fp32c_tb2_chunk(g);
   TRY(dalloc(&c->partials, 2 * heat::kNormBlocks + 2, c->stream));
   c->n_partials = heat::kNormBlocks;
   TRY(dalloc(&c->err, 1, c->stream));

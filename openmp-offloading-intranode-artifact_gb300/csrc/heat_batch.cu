@@ -123,7 +123,7 @@ int batch_blocks_per_sm(int kind) {
   const int form = form_of_kind(kind);
   const bool rhs = (kind / kNumMinb) & 1;
   const int v = kind % kNumMinb;
-  if (form == kFormF32c2) return 2;  // the two-step kernel: 640 threads, 2 blocks per SM
+  if (form == kFormF32c2) return 2;  // the two-step kernel: 384 threads, 2 blocks per SM
   if (form == kFormFx) return 1;  // one block per tile (launch_batch ignores the block count)
   switch (form) {
     case kFormHw: return rhs ? occupancy_form<kFormHw, true>(v) : occupancy_form<kFormHw, false>(v);

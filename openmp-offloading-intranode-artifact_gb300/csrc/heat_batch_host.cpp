@@ -293,10 +293,10 @@ int rebuild(heat_batch *b) {
       map_at.push_back({gi, (int)maps.size()});
       maps.resize(maps.size() + 7);
       std::copy(c->maps, c->maps + 7, maps.end() - 7);
-      // two steps per 32 x 16 tile; the temporal blocking wants long z-walks
+      // the temporal blocking wants long z-walks
       kc = std::max(kc, std::min(16, interior));
       rows = 1;
-      tile_h = 16;
+      tile_h = heat::fp32c_tile_rows();
     }
     int ntx = (c->g.nx - 2 + 31) / 32, nty = (c->g.ny - 2 + tile_h - 1) / tile_h;
     if (form == heat::kFormFx) {

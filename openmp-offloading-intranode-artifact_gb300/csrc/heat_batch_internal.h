@@ -13,7 +13,7 @@ enum BatchForm : int {
   kFormHw = 1,     // default FP64 on the FP64 pipe only
   kFormExact = 2,  // bit-exact FP64 (face kappa sums)
   kFormF32c = 3,   // FP32-compensated, one step per launch
-  kFormF32c2 = 4,  // FP32-compensated, two steps per launch (TMA-staged, 32 x 16 tiles)
+  kFormF32c2 = 4,  // FP32-compensated, two steps per launch (TMA-staged, 32 x 20 tiles)
 };
 
 // One grid of a batch as the kernel sees it.  f[b] / cr[b] are the two field
@@ -38,7 +38,7 @@ struct BatchGrid {
 
 // A tile of grid `grid` walking planes [k0, k1): 32 columns (tx) by 8 * rows
 // rows (ty), each thread walking `rows` columns 8 rows apart; Fx and F32c2 tiles
-// are 32 x 16 (their kernels' tiles) and rows is 1.
+// are their kernels' own and rows is 1.
 struct BatchTile {
   int grid;
   int tx, ty;
@@ -71,6 +71,7 @@ int fx_tiles_y(int ny);
 // planes of tiles in all; long launches want no longer chunks than 16 or so.
 int fx_fill_chunk(long tile_planes, bool rhs);
 // heat_fp32c_tma.cu: the two-step FP32C table kernel.
+int fp32c_tile_rows();
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                                    int flip, cudaStream_t st);
 

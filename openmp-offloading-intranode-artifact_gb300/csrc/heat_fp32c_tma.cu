@@ -1,21 +1,24 @@
 // FP32-compensated form, two time steps per launch (temporal blocking), with
 // plane tiles staged into shared memory by TMA.
 //
-// A block owns a (32 x 16) tile of output columns and walks a chunk of planes;
-// it has one thread per point of the tile plus a 1-point halo (34 x 18).
+// A block owns a (32 x 20) tile of output columns and walks a chunk of planes;
+// it has one thread per pair of neighbouring columns of the tile plus a 1-point
+// halo (17 pairs by 22 rows: 374 threads in 12 warps, three on each of the SM's
+// four schedulers), and computes both with GB300's packed FP32 operations.
 // For every plane p the block's thread 0 issues TMA 3-D box loads
 // (cp.async.bulk.tensor) of the five input arrays -- v, carry, wx, wy, wz --
 // covering the tile plus a 2-point halo into one slot of a 4-deep shared
 // memory ring, completing on that slot's mbarrier; loads run two planes ahead
 // of use.  Each iteration k then
 //   1. computes step t+1 on plane k+1 over the tile plus a 1-point halo
-//      (34 x 18 points) from ring planes k, k+1, k+2 into a 3-plane ring of
+//      (34 x 22 points) from ring planes k, k+1, k+2 into a 3-plane ring of
 //      intermediate values, and
 //   2. computes step t+2 on plane k-1 over the tile from intermediate planes
 //      k-2, k-1, k and writes it to global memory.
 // Running step t+2 one plane behind step t+1 leaves one block barrier per
 // plane (it publishes the landed input plane and the previous iteration's
-// intermediate plane together); at 48 registers two blocks fit on an SM.
+// intermediate plane together), and makes the two steps of an iteration
+// independent of each other.
 // Global traffic per two updates: the five input arrays read once (plus the
 // halo, mostly served by L2) and v, carry written once -- about half of two
 // single steps.  The per-point arithmetic is exactly the single-step column
@@ -23,6 +26,14 @@
 // rounded to BF16 as the single step stores it), so two steps here are
 // bit-identical to two single steps.  Points on the grid boundary keep their
 // values at both levels.
+//
+// Bound: latency between the barriers (24 warps an SM, issue 45 % busy, DRAM
+// 70 %).  512^3: 376 GLUP/s, where one thread per point in 20 warps ran 331.
+// Measured and not kept at 512^3: 16 rows (10 warps of pairs, which load the
+// schedulers 3 : 3 : 2 : 2) 327, three blocks of them per SM at 64 registers 355;
+// 13 rows in 8 warps, three blocks per SM, 357; 28 rows in 16 warps 319; two
+// planes per barrier with a 5-deep ring 346 (20 rows); the steps under their own
+// conditions instead of in one straight line 313 for 326 (16 rows).
 //
 // Every mbarrier wait is bounded: if a load does not complete within the
 // limit the block records the failure in *err, waits (bounded) for its other
@@ -38,10 +49,11 @@
 namespace heat {
 namespace {
 
-constexpr int OX = 32, OY = 16;          // output tile
+constexpr int OX = 32, OY = 20;          // output tile
 constexpr int BXF = 40, BXC = 48, BY = OY + 4;  // TMA boxes (float arrays, BF16 carry)
-constexpr int L1X = OX + 2, L1Y = OY + 2;   // step-(t+1) region
-constexpr int NT = ((L1X * L1Y + 31) / 32) * 32;  // one thread per step-(t+1) point
+constexpr int LP = (OX + 2) / 2, L1Y = OY + 2;  // step-(t+1) region: pairs by rows
+constexpr int NT = (LP * L1Y + 31) / 32 * 32;   // one thread per pair
+constexpr int V1X = 2 * LP + 2;                 // row of the intermediate planes
 constexpr int R = 4;                     // ring depth (planes)
 static_assert((R & (R - 1)) == 0, "slot index p & (R - 1) needs R a power of two");
 
@@ -67,7 +79,7 @@ static_assert(sizeof(Slot) % 128 == 0, "ring slots must start on 128-byte bounda
 
 struct Smem {
   Slot ring[R];
-  float v1[3][NT];
+  __align__(8) float v1[3][V1X * (L1Y + 2)];  // a spare row at either end
   unsigned long long bar[R];
 };
 
@@ -106,7 +118,66 @@ struct TableMaps {
   __device__ __forceinline__ const CUtensorMap *wz() const { return &tm[6]; }
 };
 
-// Two steps over one (32 x 16)-column tile with origin (x0, y0), planes
+// Two FP32 values side by side in a 64-bit register, and GB300's packed FP32
+// operations on them: each half rounds as the scalar operation does.
+typedef unsigned long long f2;
+
+__device__ __forceinline__ f2 pair(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float lo(f2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi(f2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// a - b: -1 * b is exact, so one rounding, as in the scalar subtraction
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, 0xbf800000bf800000ull, a); }
+__device__ __forceinline__ f2 ld2(const float *p) { return *reinterpret_cast<const f2 *>(p); }
+// BF16 pair to and from FP32
+__device__ __forceinline__ f2 wide(unsigned c) {
+  return pair(__uint_as_float(c << 16), __uint_as_float(c & 0xffff0000u));
+}
+__device__ __forceinline__ unsigned bf16(f2 a) {
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi(a)), "f"(lo(a)));
+  return r;
+}
+
+// Face weights of a pair at one plane: wx[c], wx[c+1]; wx[c-1]; wy[c]; wy[c-P];
+// wz[c].
+struct W {
+  f2 x;
+  float xw;
+  f2 y, ym, z;
+};
+
+// Kahan step of a pair: centre c, in-plane neighbours (we, ee: the scalars west
+// and east of the pair), planes above and below, carry cc.  The operations and
+// their order are walk_fp32c's.
+__device__ __forceinline__ f2 kahan(const W &w, f2 wzm, f2 c, float ww, float ee, f2 n, f2 s, f2 up,
+                                    f2 dn, f2 cc, f2 &carry) {
+  f2 d = fma2(w.x, sub2(pair(hi(c), ee), c), 0ull);
+  d = fma2(pair(w.xw, lo(w.x)), sub2(pair(ww, lo(c)), c), d);
+  d = fma2(w.y, sub2(n, c), d);
+  d = fma2(w.ym, sub2(s, c), d);
+  d = fma2(w.z, sub2(up, c), d);
+  d = fma2(wzm, sub2(dn, c), d);
+  const f2 y = sub2(d, cc);
+  const f2 t = add2(c, y);
+  carry = sub2(sub2(t, c), y);
+  return t;
+}
+
+// Two steps over one (32 x 20)-column tile with origin (x0, y0), planes
 // [kb, ke), of a field whose five input arrays the maps describe.  Writes vn
 // / cn.  When a bounded wait runs out it sets *err and returns once its own
 // loads in flight have landed.
@@ -128,15 +199,13 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
   chain();
   __syncthreads();
 
-  // Warp 0 keeps the bookkeeping (which slots have a load in flight, and each
-  // slot's next completion parity) and alone spins on the mbarrier; thread 0
-  // issues the TMA.  The block barrier after the wait hands the landed tile to
-  // the other warps, which skip all of it (a warp-uniform branch).
+  // Every warp waits on the mbarriers itself (warp 0 alone, handing the planes
+  // on through the block barrier: 319 GLUP/s for 335 at 384^3); thread 0 issues
+  // the TMA.
   unsigned pending = 0, phase = 0;
   bool failed = false;
-  const bool waiter = tid < 32;
   auto issue = [&](int p) {
-    if (!waiter || p < pmin || p > pmax) return;
+    if (p < pmin || p > pmax) return;
     const int s = p & (R - 1);
     pending |= 1u << s;
     if (tid != 0) return;
@@ -151,7 +220,7 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     tma_load3(sl.c, maps.c(), X0c, Y0, p, b);
   };
   auto wait_plane = [&](int p) {
-    if (!waiter || p < pmin || p > pmax || failed) return;
+    if (p < pmin || p > pmax || failed) return;
     const int s = p & (R - 1);
     if (!mbar_wait(&sm.bar[s], (phase >> s) & 1u, wait_limit)) {
       failed = true;
@@ -163,51 +232,48 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
 
   for (int p = kb - 2; p <= kb + 1; ++p) issue(p);
 
-  // This thread's step-(t+1) point (lx, ly) in the (34 x 18) region and its
-  // smem offsets; threads with 1 <= lx <= 32, 1 <= ly <= 16 also own an
-  // output point.  Like the single-step walk, each thread carries its own
-  // column along z in registers: the centre values of the input planes, the
-  // step-(t+1) values it computed, and the face weights it already loaded;
-  // only neighbours come from shared memory.
-  const bool l1_ok = tid < L1X * L1Y;
-  const int lx = tid % L1X, ly = tid / L1X;
-  const int gx = x0 - 1 + lx, gy = y0 - 1 + ly;
-  const int o = (ly + 1) * BXF + (lx + 4);     // float box offset
-  const int oc = (ly + 1) * BXC + (lx + 8);    // carry box offset
-  const bool edge = gx <= 0 || gy <= 0 || gx >= nx - 1 || gy >= ny - 1;
-  const bool out_ok = l1_ok && lx >= 1 && lx <= OX && ly >= 1 && ly <= OY && gx < nx - 1 &&
-                      gy < ny - 1;
+  // This thread's step-(t+1) points: columns gx, gx + 1 (gx even) of row gy,
+  // pair lp and row ly of the (17 x 22) region, and their shared-memory offsets.
+  // Those with 1 <= column <= 32 and 1 <= ly <= 20 of the region are output
+  // points.  Like the single-step walk, each thread carries its own columns
+  // along z in registers: the centre values of the input planes, the step-(t+1)
+  // values it computed, and the face weights it already loaded; only neighbours
+  // come from shared memory.
+  const int lp = tid % LP;
+  const bool l1_ok = tid < LP * L1Y;
+  const int ly = l1_ok ? tid / LP : 0;  // threads past the region walk its first row and store nothing
+  const int gx = x0 - 1 + 2 * lp, gy = y0 - 1 + ly;
+  const int o = (ly + 1) * BXF + 2 * lp + 4;      // float box offset
+  const int oc = (ly + 1) * BXC + 2 * lp + 8;     // carry box offset
+  const int o1 = (ly + 1) * V1X + 2 * lp;         // intermediate plane offset
+  const bool edge_y = gy <= 0 || gy >= ny - 1;
+  const bool edge0 = edge_y || gx <= 0 || gx >= nx - 1, edge1 = edge_y || gx + 1 >= nx - 1;
+  // Whether the tile's step-(t+1) region reaches the grid's boundary in x or y.
+  const bool edge_tile = x0 == 1 || y0 == 1 || x0 + OX >= nx - 1 || y0 + OY >= ny - 1;
+  const bool out_y = l1_ok && ly >= 1 && ly <= OY && gy < ny - 1;
+  const bool out0 = out_y && lp > 0 && gx < nx - 1, out1 = out_y && lp < LP - 1 && gx + 1 < nx - 1;
 
-  struct W {
-    float x, xm, y, ym, z;  // wx[c], wx[c-1], wy[c], wy[c-P], wz[c] at one plane
-  };
-  // Step t+1 on plane p at this thread's point from centre values vm, v0, vp
-  // (planes p-1, p, p+1) and wz at plane p-1; returns the new value and carry
-  // and the plane's weights.
-  auto level1 = [&](int p, float vm, float v0, float vp, float wzm, W &wp, float &t1,
-                    float &c1) {
+  // Step t+1 on plane p at this thread's points from centre values vm, v0, vp
+  // (planes p-1, p, p+1) and wz at plane p-1; returns the new values and
+  // carries and the plane's weights.
+  auto level1 = [&](int p, f2 vm, f2 v0, f2 vp, f2 wzm, W &wp, f2 &t1, f2 &c1) {
     const Slot &cur = sm.ring[p & (R - 1)];
-    wp.x = cur.wx[o];
-    wp.xm = cur.wx[o - 1];
-    wp.y = cur.wy[o];
-    wp.ym = cur.wy[o - BXF];
-    wp.z = cur.wz[o];
-    const float cc0 = walk::bf2f(cur.c[oc]);
-    if (edge || p == 0 || p == nz - 1) {
-      t1 = v0;
-      c1 = cc0;
-      return;
+    wp.x = ld2(&cur.wx[o]);
+    wp.xw = cur.wx[o - 1];
+    wp.y = ld2(&cur.wy[o]);
+    wp.ym = ld2(&cur.wy[o - BXF]);
+    wp.z = ld2(&cur.wz[o]);
+    const f2 cc0 = wide(*reinterpret_cast<const unsigned *>(&cur.c[oc]));
+    f2 c;
+    const f2 t = kahan(wp, wzm, v0, cur.v[o - 1], cur.v[o + 2], ld2(&cur.v[o + BXF]),
+                       ld2(&cur.v[o - BXF]), vp, vm, cc0, c);
+    t1 = t;
+    c1 = wide(bf16(c));
+    const bool z = p == 0 || p == nz - 1;
+    if (edge_tile || z) {  // the same for the whole block
+      t1 = pair(edge0 || z ? lo(v0) : lo(t1), edge1 || z ? hi(v0) : hi(t1));
+      c1 = pair(edge0 || z ? lo(cc0) : lo(c1), edge1 || z ? hi(cc0) : hi(c1));
     }
-    float d = 0.0f;
-    d = fmaf(wp.x, cur.v[o + 1] - v0, d);
-    d = fmaf(wp.xm, cur.v[o - 1] - v0, d);
-    d = fmaf(wp.y, cur.v[o + BXF] - v0, d);
-    d = fmaf(wp.ym, cur.v[o - BXF] - v0, d);
-    d = fmaf(wp.z, vp - v0, d);
-    d = fmaf(wzm, vm - v0, d);
-    const float yk = __fsub_rn(d, cc0);
-    t1 = __fadd_rn(v0, yk);
-    c1 = walk::bf2f(walk::f2bf(__fsub_rn(__fsub_rn(t1, v0), yk)));
   };
 
   // Prologue: intermediate planes kb-1 and kb.  A failed wait stops the whole
@@ -218,28 +284,28 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
   wait_plane(kb + 1);
   failed = __syncthreads_or(failed);
   // Level-1 window: v(p-1), v(p), wz(p-1) for the next plane p to compute.
-  float vm = 0.f, v0 = 0.f, wzm = 0.f;
+  f2 vm = 0, v0 = 0, wzm = 0;
   // Level-2 window at the top of iteration k: own step-(t+1) values at planes
   // k-2, k-1, k, the carries at k-1, k, the weights at k-1, k and wz at k-2.
-  float l1a = 0.f, l1b = 0.f, l1cc = 0.f;
-  float c1b = 0.f, c1cc = 0.f;
+  f2 l1a = 0, l1b = 0, l1cc = 0;
+  f2 c1b = 0, c1cc = 0;
   W wb{}, wcc{};
-  float wza = 0.f;
+  f2 wza = 0;
   if (!failed && l1_ok) {
     if (kb - 2 >= 0) {
-      vm = sm.ring[(kb - 2) & (R - 1)].v[o];
-      wzm = sm.ring[(kb - 2) & (R - 1)].wz[o];
+      vm = ld2(&sm.ring[(kb - 2) & (R - 1)].v[o]);
+      wzm = ld2(&sm.ring[(kb - 2) & (R - 1)].wz[o]);
     }
-    v0 = sm.ring[(kb - 1) & (R - 1)].v[o];
-    float vp = sm.ring[kb & (R - 1)].v[o];
+    v0 = ld2(&sm.ring[(kb - 1) & (R - 1)].v[o]);
+    f2 vp = ld2(&sm.ring[kb & (R - 1)].v[o]);
     level1(kb - 1, vm, v0, vp, wzm, wb, l1b, c1b);
-    sm.v1[(kb - 1) % 3][tid] = l1b;
+    *reinterpret_cast<f2 *>(&sm.v1[(kb - 1) % 3][o1]) = l1b;
     vm = v0;
     v0 = vp;
     wzm = wb.z;
-    vp = sm.ring[(kb + 1) & (R - 1)].v[o];
+    vp = ld2(&sm.ring[(kb + 1) & (R - 1)].v[o]);
     level1(kb, vm, v0, vp, wzm, wcc, l1cc, c1cc);
-    sm.v1[kb % 3][tid] = l1cc;
+    *reinterpret_cast<f2 *>(&sm.v1[kb % 3][o1]) = l1cc;
     vm = v0;
     v0 = vp;
     wzm = wcc.z;
@@ -263,39 +329,39 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
   int ia = (kb + 2) % 3, ib = kb % 3, ic = (kb + 1) % 3;
   size_t g = (size_t)(kb - 1) * S + (size_t)gy * P + gx;
   // Unrolled by the intermediate ring's period (3): the slot indices and the
-  // shift of the carried values resolve to fixed registers in each copy
-  // (512^3: 325 GLUP/s unrolled by 3, 308 not unrolled, 286 by 2, 321 by 6,
-  // 284 by 12, which spills).
+  // shift of the carried values resolve to fixed registers in each copy.
 #pragma unroll 3
   for (int k = kb; k <= ke && !failed; ++k, g += S) {
     wait_plane(k + 2);
     failed = __syncthreads_or(failed);
     if (failed) break;
     issue(k + 4);
-    W wn{};
-    float l1p = 0.f, c1p = 0.f;
-    if (k + 1 <= ke && l1_ok) {
-      const float vp = sm.ring[(k + 2) & (R - 1)].v[o];
-      level1(k + 1, vm, v0, vp, wzm, wn, l1p, c1p);
-      sm.v1[ic][tid] = l1p;
-      vm = v0;
-      v0 = vp;
-      wzm = wn.z;
-    }
-    if (k - 1 >= kb && out_ok) {
-      const float *vk = sm.v1[ia];
-      float d = 0.0f;
-      d = fmaf(wb.x, vk[tid + 1] - l1b, d);
-      d = fmaf(wb.xm, vk[tid - 1] - l1b, d);
-      d = fmaf(wb.y, vk[tid + L1X] - l1b, d);
-      d = fmaf(wb.ym, vk[tid - L1X] - l1b, d);
-      d = fmaf(wb.z, l1cc - l1b, d);
-      d = fmaf(wza, l1a - l1b, d);
-      const float yk = __fsub_rn(d, c1b);
-      const float t = __fadd_rn(l1b, yk);
-      const float cc = __fsub_rn(__fsub_rn(t, l1b), yk);
-      vn[g] = t;
-      cn[g] = walk::f2bf(cc);
+    // Both steps in one straight line, so that the second fills the first's
+    // waits; a step that this iteration does not have (the first plane's second,
+    // the last one's first) is computed from whatever is there and dropped.
+    W wn;
+    f2 l1p, c1p, c;
+    const float *vk = sm.v1[ia];
+    const f2 vp = ld2(&sm.ring[(k + 2) & (R - 1)].v[o]);
+    const f2 t = kahan(wb, wza, l1b, vk[o1 - 1], vk[o1 + 2], ld2(&vk[o1 + V1X]), ld2(&vk[o1 - V1X]),
+                       l1cc, l1a, c1b, c);
+    level1(k + 1, vm, v0, vp, wzm, wn, l1p, c1p);
+    if (l1_ok) *reinterpret_cast<f2 *>(&sm.v1[ic][o1]) = l1p;
+    vm = v0;
+    v0 = vp;
+    wzm = wn.z;
+    if (k > kb) {
+      const unsigned cb = bf16(c);
+      if (out0 && out1) {
+        *reinterpret_cast<f2 *>(&vn[g]) = t;
+        *reinterpret_cast<unsigned *>(&cn[g]) = cb;
+      } else if (out0) {
+        vn[g] = lo(t);
+        cn[g] = (uint16_t)cb;
+      } else if (out1) {
+        vn[g + 1] = hi(t);
+        cn[g + 1] = (uint16_t)(cb >> 16);
+      }
     }
     l1a = l1b;
     l1b = l1cc;
@@ -314,7 +380,7 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     if (tid == 0) atomicExch(err, 1);
     // Let the block's own loads in flight land before its shared memory goes
     // (each wait bounded).
-    if (waiter)
+    if (tid == 0)
       for (int s = 0; s < R; ++s)
         if (pending & (1u << s)) mbar_wait(&sm.bar[s], (phase >> s) & 1u);
   }
@@ -357,18 +423,35 @@ bool encode(CUtensorMap *m, const void *base, bool bf16, const heat_geom &g) {
                            bf16 ? 2 : 4, g, bf16 ? BXC : BXF, BY);
 }
 
+constexpr size_t kSmem = sizeof(Smem) + 128;
+
+// The kernels' shared memory allowed, once per process.
+bool ready() {
+  static const bool ok =
+      cudaFuncSetAttribute(k_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) ==
+          cudaSuccess &&
+      cudaFuncSetAttribute(k_batch_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kSmem) == cudaSuccess;
+  return ok;
+}
+
 }  // namespace
 
-size_t fp32c_tb2_smem() { return sizeof(Smem) + 128; }
+int fp32c_tile_rows() { return OY; }
+
+// A chunk's start costs about 4 planes' time: two planes of step t+1, their loads
+// and the halo planes.
+int fp32c_tb2_chunk(const heat_geom &g) {
+  const long tiles = (long)((g.nx - 2 + OX - 1) / OX) * ((g.ny - 2 + OY - 1) / OY);
+  static const long resident = ready() ? resident_blocks((const void *)k_fp32c_tb2, NT, kSmem) : 0;
+  return balanced_chunk(tiles, g.nz - 2, resident, 4, 0.95, 128);
+}
 
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                                    int flip, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  static bool attr =
-      cudaFuncSetAttribute(k_batch_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)fp32c_tb2_smem()) == cudaSuccess;
-  if (!attr) return cudaErrorInvalidConfiguration;
-  k_batch_fp32c_tb2<<<ntiles, NT, fp32c_tb2_smem(), st>>>(grids, tiles, flip);
+  if (!ready()) return cudaErrorInvalidConfiguration;
+  k_batch_fp32c_tb2<<<ntiles, NT, kSmem, st>>>(grids, tiles, flip);
   return cudaGetLastError();
 }
 
@@ -385,19 +468,10 @@ bool encode_fp32c_maps(CUtensorMap *m, float *const v[2], uint16_t *const cr[2],
 cudaError_t launch_fp32c_tb2(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
   if (wait_limit > tma::kWaitLimit) wait_limit = tma::kWaitLimit;
   const heat_geom &g = c->g;
-  static bool attr = cudaFuncSetAttribute(k_fp32c_tb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)fp32c_tb2_smem()) == cudaSuccess;
-  if (!attr) return cudaErrorInvalidConfiguration;
-  const int bx = (g.nx - 2 + OX - 1) / OX, by = (g.ny - 2 + OY - 1) / OY;
-  const int interior = g.nz - 2;
-  // Each chunk recomputes step t+1 on its halo planes, so chunks are deeper
-  // than the single-step launches': 96 planes at least (512^3: 330 GLUP/s,
-  // against 324 / 320 / 309 for 64 / 48 / 32 and 311 for 128, where 3 chunks
-  // leave 5.05 waves), 16 where a small grid needs more chunks to fill the GPU.
-  static const long resident = resident_blocks((const void *)k_fp32c_tb2, NT, fp32c_tb2_smem());
-  const int kchunk = wave_chunk(g, OX, OY, resident, 24, 96, 16);
-  dim3 grid(bx, by, (interior + kchunk - 1) / kchunk);
-  return launch_chained(k_fp32c_tb2, grid, NT, fp32c_tb2_smem(), st,
+  if (!ready()) return cudaErrorInvalidConfiguration;
+  const int kchunk = c->kchunk;
+  dim3 grid((g.nx - 2 + OX - 1) / OX, (g.ny - 2 + OY - 1) / OY, (g.nz - 2 + kchunk - 1) / kchunk);
+  return launch_chained(k_fp32c_tb2, grid, NT, kSmem, st,
                         Maps{c->maps[cur], c->maps[2 + cur], c->maps[4], c->maps[5], c->maps[6]},
                         c->v[cur ^ 1], c->carry[cur ^ 1], g.nx, g.ny, g.nz, g.pitch, g.plane,
                         kchunk, c->err, wait_limit);

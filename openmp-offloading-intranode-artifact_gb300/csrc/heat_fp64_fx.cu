@@ -640,9 +640,7 @@ long resident() {
 template <bool RHS>
 cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
   const heat_geom &g = c->g;
-  const int interior = g.nz - 2;
-  int kc = fx_fill_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny) * interior, RHS);
-  kc = kc >= 16 ? wave_chunk(g, TX, TY, resident<RHS>()) : kc < interior ? kc : interior;
+  const int kc = c->kchunk;
   dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
   return launch_chained(k_fx<RHS>, gr, NT, smem_bytes<RHS>(), st,
                         Maps{c->maps[cur], c->maps[2], c->maps[3]}, c->u[cur ^ 1],
@@ -657,15 +655,18 @@ cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_li
 int fx_tiles_x(int nx) { return (nx - 1 + TX - 1) / TX; }
 int fx_tiles_y(int ny) { return (ny - 2 + TY - 1) / TY; }
 
-// A lone block needs about 1 us a plane and 4 us to start and finish a launch,
-// a full SM (4 blocks) 2 us a plane of each: small grids want short chunks until
-// the GPU holds 1.7 blocks for every resident one (64^3: 7.1 us a step at 1
-// plane, 12.3 at 8; 128^3: 18.5 at 4, 20.5 at 8 and at 2).  From 16 planes on a
-// launch takes whole waves (512^3: 789 to 800 us between 17 and 64 planes, 820
-// and more beyond).
+// Short tiles until a table holds 1.7 blocks for every resident one, as a small
+// grid alone wants (64^3: 4.8 us a step at 1 plane, 6.7 at 2, 9.9 at 8).
 int fx_fill_chunk(long tile_planes, bool rhs) {
   const long n = rhs ? resident<true>() : resident<false>();
   return n > 0 ? (int)((3 * tile_planes + 5 * n - 1) / (5 * n)) : 16;
+}
+
+// A chunk's start, its first loads, costs about a plane's time; 384^3 runs 329 us
+// a step at 20 planes, 355 at 191.
+int fx_chunk(const heat_geom &g, bool rhs) {
+  return balanced_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny), g.nz - 2,
+                        rhs ? resident<true>() : resident<false>(), 1, 0.53, 32);
 }
 
 bool fx_usable(bool rhs) { return rhs ? usable<true>() : usable<false>(); }

@@ -3,6 +3,7 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -49,6 +50,7 @@ struct heat_ctx {
   // FP32C two-step form v0 v1 carry0 carry1 wx wy wz.
   CUtensorMap maps[7];
   bool have_maps;
+  int kchunk;  // planes per block of those steps
 
   // Device flag a kernel sets when a bounded wait ran out (HEAT_ETIMEOUT).
   int *err;
@@ -165,6 +167,38 @@ inline int wave_chunk(const heat_geom &g, int tile_x, int tile_y, long resident,
   return (int)((interior + chunks - 1) / chunks);
 }
 
+// Planes per block for a launch of `tiles` tiles over `interior` planes whose
+// blocks run `resident` at a time: the chunk count with the least estimated
+// time.  A round of blocks takes (planes + overhead) plane times; `alone` is a
+// plane's time with one block on an SM as a fraction of its time on a full one
+// (latency keeps it from falling with the load), between which it rises steeply
+// at first (k_fx: 0.53, 0.88, 0.94, 1 for 1 to 4 blocks).  At most `most` planes:
+// few long rounds end less evenly than this counts on.  Worked out once per
+// context.  Against the chunk that measured best of 19 it costs 2 to 8 % on
+// grids from 40 x 33 x 28 to 512^3.
+inline int balanced_chunk(long tiles, int interior, long resident, int overhead, double alone,
+                          int most) {
+  if (resident <= 0) return interior < 32 ? interior : 32;
+  const long per_sm = (resident + 151) / 152;
+  const int first = (interior + most - 1) / most;
+  double best = 0;
+  int best_kc = interior;
+  for (int c = first; c <= interior && c < first + 256; ++c) {
+    const int kc = (interior + c - 1) / c;
+    const long blocks = tiles * ((interior + kc - 1) / kc);
+    const long rest = (blocks % resident + 151) / 152;  // blocks per SM in the last round
+    double rounds = (double)(blocks / resident);
+    if (rest)
+      rounds += alone + (1.0 - alone) * std::sqrt((double)(rest - 1) / (per_sm > 1 ? per_sm - 1 : 1));
+    const double cost = rounds * (kc + overhead);
+    if (c == first || cost < best) {
+      best = cost;
+      best_kc = kc;
+    }
+  }
+  return best_kc;
+}
+
 // heat_fp64_exact.cu (compiled with --fmad=false)
 cudaError_t launch_exact_raw(double *u_new, const double *u_old, const double *rhs,
                              const double *kappa, const heat_geom &g, double factor,
@@ -194,6 +228,7 @@ cudaError_t launch_kq_setup(unsigned long long *K, int *bad, const double *kappa
 // context c from buffer `cur`.  encode_fx_maps fills m with the maps of a
 // field pair, its weights and source term (NULL: none).
 bool fx_usable(bool rhs);
+int fx_chunk(const heat_geom &g, bool rhs);
 bool encode_fx_maps(CUtensorMap *m, double *const u[2], const unsigned long long *K,
                     const double *rhs, const heat_geom &g);
 cudaError_t launch_fx(const heat_ctx *c, int cur, cudaStream_t st,
@@ -224,6 +259,7 @@ cudaError_t launch_to_f32(float *o, const double *a, size_t total, cudaStream_t 
 // launch (kWaitLimit in product use; smaller only to exercise the failure path).
 bool encode_fp32c_maps(CUtensorMap *m, float *const v[2], uint16_t *const cr[2],
                        float *const w[3], const heat_geom &g);
+int fp32c_tb2_chunk(const heat_geom &g);
 cudaError_t launch_fp32c_tb2(const heat_ctx *c, int cur, cudaStream_t st,
                              unsigned wait_limit = kWaitLimit);
 // Whether a context steps with launch_fp32c_tb2.

@@ -9,7 +9,7 @@
 //   minb   : the table kernel compiled for 2, 3 or 4 resident blocks per SM
 //            (its register cap per thread: 128, 80 or 64),
 //   depth  : time steps per launch, 1, or 2 for FP32C grids (the two-step TMA
-//            kernel on 32 x 16 tiles),
+//            kernel and its own tiles),
 // one after another (coordinate descent from the defaults 32 / 1 / the form's
 // default / 1).  For a class it builds a batch that fills the GPU the way a
 // real batch does: copies of one synthetic grid of that depth
