@@ -304,7 +304,7 @@ int rebuild(heat_batch *b) {
       maps.resize(maps.size() + 4);
       std::copy(c->maps, c->maps + 4, maps.end() - 4);
       // A small table fills the GPU with shorter tiles than the tuned ones.
-      kc = std::min(kc, std::max(1, heat::fx_fill_chunk(fx_planes[c->rhs != nullptr], c->rhs)));
+      kc = std::min(kc, heat::fx_fill_chunk(fx_planes[c->rhs != nullptr], c->rhs));
       rows = 1;
       ntx = heat::fx_tiles_x(c->g.nx);
       nty = heat::fx_tiles_y(c->g.ny);

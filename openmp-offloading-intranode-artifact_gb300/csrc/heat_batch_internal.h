@@ -67,8 +67,7 @@ cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int 
                             int flip, cudaStream_t st);
 int fx_tiles_x(int nx);
 int fx_tiles_y(int ny);
-// Planes per block that fill the GPU with blocks for a launch of tile_planes
-// planes of tiles in all; long launches want no longer chunks than 16 or so.
+// Most planes per tile of a table of tile_planes planes of such tiles in all.
 int fx_fill_chunk(long tile_planes, bool rhs);
 // heat_fp32c_tma.cu: the two-step FP32C table kernel.
 int fp32c_tile_rows();

@@ -18,10 +18,10 @@
 //     is negative, rounded up to an even number) gives the scale E: a value
 //     becomes the integer A = value * 2^(1083 - E), |A| < 2^61.
 //   * If no nonzero value of the patch itself (three planes) lies more than
-//     kSlack = 8 binary orders below E, those A are exact.  A neighbour further
-//     below is cut to whole units, an error of one unit times its weight; a
-//     result below 2^53 units, where a unit is more than 1/2 ulp, is formed anew
-//     point by point.
+//     kSlack = 8 binary orders below E, those A are exact, and are carried along
+//     z.  Other values are cut to whole units, an error of one unit times the
+//     weight.  A result below 2^53 units, where a unit is more than 1/2 ulp, is
+//     formed anew on its own.
 //   * Weights come from the per-point K = factor * kappa, kept as two limbs
 //     K = k1 2^-32 + k0 2^-63 with |k0| <= 2^30: a face weight is the two limb
 //     sums, no carry, and its low limb is a signed 32-bit number.
@@ -36,17 +36,17 @@
 // FP64 multiply-adds has seven roundings, and rounded weights besides.  A
 // constant region stays exactly constant (every D is 0).
 //
-// Patches outside those bounds (a wider range of magnitudes, exponents near
-// either end, infinities, NaNs) go point by point, each at the largest exponent
-// of its own seven values.  Which of the two a patch takes, and E, depend only on
-// the field's values in its region, never on tiles or z-chunks, so a grid's
-// results are the same bits in any launch.
-// (Patches are small so that steep fields fit: of a Gaussian of width 0.05 on
-// 512^3, whose tails fall by up to one binary order per point, no patch is
-// outside the bounds; of 16 x 8-point patches 40 % would be.)
+// Points formed on their own (results too small for their patch's units,
+// exponents near either end, infinities, NaNs) are aligned to the largest
+// exponent of their own seven values.  Which way a point goes, and E, depend only
+// on the field's values in the patch's region, never on tiles or z-chunks, so a
+// grid's results are the same bits in any launch.
 //
 // The integers carried along z move to a new scale by shifting, which is exact
-// because both scales hold the patch exactly.
+// where both scales hold the patch exactly; elsewhere they are taken from the
+// values again.  (Patches are small so that steep fields fit: of a Gaussian of
+// width 0.05 on 512^3, whose tails fall by up to one binary order per point, no
+// patch is outside the slack; of 16 x 8-point patches 40 % would be.)
 //
 // Staging: a block is 32 x 16 columns (128 threads, 16 x 8 patches).  Planes of
 // u and K (and the source term) land by TMA in a ring 4 deep (3), boxes 36 x 18
@@ -54,17 +54,18 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 165 GLUP/s (0.80 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 168 GLUP/s (0.79 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 146 (115.7).
-// About 139 warp instructions per point (300 for an integer row of that
+// the launch before this one), with the reference's source term 149 (115.7);
+// 192^3 with a narrow Gaussian 134, 160 without.
+// About 140 warp instructions per point (300 for an integer row of that
 // launch); ALU, FMA-heavy (18 of its instructions the wide multiply-adds, twice
 // the cost of the others) and issue are each about 60 % busy, DRAM 55 %.
-// Measured and not kept: the neighbours above and below converted by the FP64
-// pipe as the patch's own are (157 when this was 167; that pipe is then at 75 %
-// and the others wait for it), no value converted by it (164), five blocks per SM
-// at 96 registers (165), 32 x 32 tiles (156), 64 x 8 (166), the plane loop
-// unrolled by 2 (162).
+// Measured and not kept (512^3, GLUP/s): the neighbours above and below converted
+// by the FP64 pipe as the patch's own are, 157 for 167 (that pipe is then at 75 %
+// and the others wait for it); no value converted by it 164; five blocks per SM
+// at 96 registers 162; 32 x 32 tiles 156; 64 x 8 166; the plane loop unrolled by
+// 2 162.
 //
 // Every mbarrier wait is bounded: a wait that runs out stops the block at the
 // next barrier (the flag is OR-reduced), thread 0 waits (bounded) for its loads
@@ -93,6 +94,7 @@ constexpr int BX = TX + 4, BY = TY + 2;  // box: columns i0 - 2 .. i0 + 33, rows
 // slots are larger (four blocks of 4 would not fit an SM).
 template <bool RHS>
 constexpr int kRing = RHS ? 3 : 4;
+constexpr int kMaxPlanes = 32;  // of a chunk: a bit each in `again`
 constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills
 
 constexpr unsigned kExp = 1u << 20;      // one binary order in the high word of a double
@@ -126,6 +128,7 @@ static_assert(sizeof(Slot<false>) % 128 == 0 && sizeof(Slot<true>) % 128 == 0 &&
 template <bool RHS>
 struct Smem {
   Slot<RHS> ring[kRing<RHS>];
+  ulonglong2 below[2][NT];  // each thread's patch at the plane below, where its registers do not hold it
   u64 bar[kRing<RHS>];
 };
 
@@ -176,7 +179,8 @@ struct Range {
     const unsigned up = (int)sg < 0 ? 2 * kExp : kExp;
     return max((mx + up) & ~(2 * kExp - 1), kLowE);
   }
-  __device__ __forceinline__ bool fits(unsigned E) const {
+  // Whether the scale holds every value seen exactly.
+  __device__ __forceinline__ bool held(unsigned E) const {
     return E - min(mn, E) <= kSlack + 1 && E <= kHighE && mx != 0;
   }
 };
@@ -254,60 +258,46 @@ struct Acc {
   }
 };
 
-// A point of a patch outside the shared scale's bounds: box offset p, the value
-// vd below it and the limbs of the weight to it.  The same arithmetic at the
-// point's own scale, the largest exponent of its seven values (and the source
-// term), every value cut to that scale's units; exponents near either end,
-// infinities and NaNs take walk::int_point.  PLAIN: no value is negative.  A
-// whole grid of such points runs at 99 GLUP/s (512^3; 87 with signs always).  A
-// function of its own: inlined, or four points to a call, they run at 119 and
-// 112, but the fast form, scheduled around them, at 144 and 142 for 164.  pd: the value below in global
-// memory (vd may have read a subnormal as 0).
-template <bool RHS, bool PLAIN>
-__device__ __noinline__ double point(const Slot<RHS> &sk, const Slot<RHS> &sn, int p, int prhs,
-                                     u64 vd, unsigned w0, unsigned w1, const u64 *pd) {
-  const u64 c = sk.u[p], f[6] = {sn.u[p], vd, sk.u[p - 1], sk.u[p + 1], sk.u[p - BX], sk.u[p + BX]};
+// One point from global memory (u, K and the source term at it): the same
+// arithmetic at the point's own scale, the largest exponent of its seven values
+// (and the source term), every value cut to that scale's units; exponents near
+// either end, infinities and NaNs take walk::int_point.
+template <bool RHS>
+__device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *rhs, int P, size_t S) {
+  const u64 c = __ldcg(u);
+  const u64 f[6] = {__ldcg(u + S), __ldcg(u - S), __ldcg(u - 1),
+                    __ldcg(u + 1), __ldcg(u - P), __ldcg(u + P)};
+  const u64 kc = __ldcg(K);
+  const u64 k[6] = {__ldcg(K + S), __ldcg(K - S), __ldcg(K - 1),
+                    __ldcg(K + 1), __ldcg(K - P), __ldcg(K + P)};
   Range r;
   r.bound(c);
 #pragma unroll
   for (int q = 0; q < 6; ++q) r.bound(f[q]);
   u64 vr = 0;
   if constexpr (RHS) {
-    vr = sk.r[prhs];
+    vr = __ldcg(rhs);
     r.bound(vr);
   }
-  const u64 kc = sk.k[p];
-  const u64 k[6] = {sn.k[p], 0, sk.k[p - 1], sk.k[p + 1], sk.k[p - BX], sk.k[p + BX]};
-  const unsigned E = r.mx + (!PLAIN && (int)r.sg < 0 ? kExp : 0u);
+  const unsigned E = r.mx + ((int)r.sg < 0 ? kExp : 0u);
   if (E - kLowE <= kHighE - kLowE) {
-    auto load = [&](u64 v) {
-      const u64 m = magnitude(v, E);
-      return PLAIN ? m : with_sign(m, v);
-    };
+    auto load = [&](u64 v) { return with_sign(magnitude(v, E), v); };
     const u64 A = load(c);
     Acc a(A);
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      if (q == 1)
-        a.face(load(f[q]) - A, w0, w1);
-      else
-        a.face(load(f[q]) - A, kc, k[q]);
-    }
+    for (int q = 0; q < 6; ++q) a.face(load(f[q]) - A, kc, k[q]);
     if constexpr (RHS) a.add(vr, E);
     return scaled(a.rounded(), E);
   }
-  const u64 ud = __ldcg(pd);
-  if (((c | f[0] | ud | f[2] | f[3] | f[4] | f[5] | vr) << 1) == 0) return 0.0;
-  // K in units of 2^-64, as int_point takes it; the one below from the face's limbs
-  auto weight = [](unsigned k0, unsigned k1) {
-    return ((u64)k1 << 32) + 2ull * (u64)(i64)(int)k0;
+  if (((c | f[0] | f[1] | f[2] | f[3] | f[4] | f[5] | vr) << 1) == 0) return 0.0;
+  auto w = [](u64 x) {  // K in units of 2^-64, as int_point takes it
+    return (x & 0xffffffff00000000ull) + 2ull * (u64)(i64)(int)(unsigned)x;
   };
-  auto w = [&](u64 x) { return weight((unsigned)x, (unsigned)(x >> 32)); };
-  return walk::int_point<RHS>(
-      walk::decode(c), walk::decode(f[0]), walk::decode(ud), walk::decode(f[3]), walk::decode(f[2]),
-      walk::decode(f[5]), walk::decode(f[4]), w(kc), w(k[0]),
-      weight(w0 - (unsigned)kc, w1 - (unsigned)(kc >> 32)), w(k[3]), w(k[2]), w(k[5]), w(k[4]), vr,
-      [=] { return walk::Raw7{c, f[3], f[2], f[5], f[4], f[0], ud}; });
+  return walk::int_point<RHS>(walk::decode(c), walk::decode(f[0]), walk::decode(f[1]),
+                              walk::decode(f[3]), walk::decode(f[2]), walk::decode(f[5]),
+                              walk::decode(f[4]), w(kc), w(k[0]), w(k[1]), w(k[3]), w(k[2]), w(k[5]),
+                              w(k[4]), vr,
+                              [=] { return walk::Raw7{c, f[3], f[2], f[5], f[4], f[0], f[1]}; });
 }
 
 // Keeps the compiler from holding values read before this point in registers.
@@ -318,11 +308,11 @@ __device__ __forceinline__ ulonglong2 ld2(const u64 *p) {
 }
 
 // One step over the (32 x 16)-column tile (tx, ty), planes [kb, ke), of the
-// field u into un.  Returns true if a wait ran out.
+// field u into un; at most kMaxPlanes planes.  Returns true if a wait ran out.
 template <bool RHS, class M>
 __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__restrict__ un,
                                         const u64 *__restrict__ u, const u64 *__restrict__ K,
-                                        int tx, int ty, int nx, int ny, int P, size_t S, int kb,
+                                        const u64 *__restrict__ rhs, int tx, int ty, int nx, int ny, int P, size_t S, int kb,
                                         int ke, unsigned wait_limit) {
   const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
   const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly;  // patch: i, i + 1; j, j + 1
@@ -351,8 +341,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
 
   // Carried along z, points in the order (i, j), (i + 1, j), (i, j + 1),
   // (i + 1, j + 1): the patch at plane k (A1) and its difference to plane k - 1
-  // (Dd) at scale E (0: not held), the weight limbs of the face below, K and
-  // the ranges.
+  // (Dd) at scale E (0: not held), the weight limbs of the face below and the
+  // ranges.
   u64 Dd[4], A1[4];
   unsigned W0[4], W1[4];
   Range r0, r1;
@@ -387,10 +377,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
       A1[q] = with_sign(magnitude(b[q], E), b[q]);
       Dd[q] = with_sign(magnitude(a[q], E), a[q]) - A1[q];
     }
-    if (!r.fits(E)) {
+    if (!r.held(E)) {
       E = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) A1[q] = a[q];
+      sm.below[0][t] = make_ulonglong2(a[0], a[1]);
+      sm.below[1][t] = make_ulonglong2(a[2], a[3]);
     }
   }
 
@@ -399,6 +389,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   int s0 = 0, s1 = 1;
   unsigned parity = 0;
   double *w = un + (size_t)kb * S + (size_t)j * P + i;  // the patch at plane k
+  // Keeps points that are not written out of `least`.
+  const int skip[4] = {x0 && y0 ? 0 : 0x7fffffff, x1 && y0 ? 0 : 0x7fffffff,
+                       x0 && y1 ? 0 : 0x7fffffff, x1 && y1 ? 0 : 0x7fffffff};
+  unsigned again = 0;  // bit p: the patch at plane kb + p is to be formed point by point
   int k = kb;
   for (; k < ke; ++k, w += S) {
     const int s2 = s1 == kRing<RHS> - 1 ? 0 : s1 + 1;
@@ -442,16 +436,11 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
       }
     }
     const unsigned En = r.scale();
-    if (r.fits(En)) {
+    const bool held = r.held(En);
+    int least = 0;  // high word of the smallest result (its size), in units
+    if (r.mx != 0 && En <= kHighE) {
       if (E != En) {
-        if (E == 0) {  // the plane before went point by point
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const u64 a = A1[q], b = sk.u[o + (q >> 1) * BX + (q & 1)];
-            A1[q] = with_sign(magnitude(b, En), b);
-            Dd[q] = with_sign(magnitude(a, En), a) - A1[q];
-          }
-        } else {
+        if (E != 0 && held) {
           const int d = (int)(En - E) >> 20;
           const unsigned dn = (unsigned)max(d, 0), ups = (unsigned)max(-d, 0);
 #pragma unroll
@@ -459,59 +448,73 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             Dd[q] = sar(shl(Dd[q], ups), dn);
             A1[q] = sar(shl(A1[q], ups), dn);
           }
+        } else {  // from the values: those below are A1 + Dd units, or in shared memory
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            u64 a = (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E));
+            if (E == 0) a = q & 1 ? sm.below[q >> 1][t].y : sm.below[q >> 1][t].x;
+            const u64 b = sk.u[o + (q >> 1) * BX + (q & 1)];
+            A1[q] = with_sign(magnitude(b, En), b);
+            Dd[q] = with_sign(magnitude(a, En), a) - A1[q];
+          }
         }
         E = En;
       }
       // The values are read from shared memory again here, row by row, rather
       // than kept in registers from the range pass.
       u64 A2[4];
-      int least = 0x7fffffff;  // high word of the smallest result (its size), in units
+      least = 0x7fffffff;
+      double out[4];
       auto patch = [&](auto plain) {
+        // One straight line, no branch in it: with one between the points the
+        // compiler forms them one after the other (512^3: 870 to 960 us a step for
+        // 788).
         auto load = [&](u64 v) {
           const u64 m = magnitude(v, E);
           return plain.value ? m : with_sign(m, v);
-      };
+        };
+        reload();
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
-          reload();
-          double out[2];
           const int oy = o + y * BX, oo = y ? o + 2 * BX : o - BX;
+          // of the row: the plane above (U), beside it (S), the other row of the
+          // patch (I) and the one outside it (O)
           const ulonglong2 vU = ld2(&sn.u[oy]), vO = ld2(&sk.u[oo]);
           const ulonglong2 kC = ld2(&sk.k[oy]), kI = ld2(&sk.k[y ? o : o + BX]), kO = ld2(&sk.k[oo]),
                            kU = ld2(&sn.k[oy]);
-          A2[2 * y] = plain.value ? convert(vU.x, E) : load(vU.x);
-          A2[2 * y + 1] = plain.value ? convert(vU.y, E) : load(vU.y);
+          const u64 vS[2] = {sk.u[oy - 1], sk.u[oy + 2]}, kS[2] = {sk.k[oy - 1], sk.k[oy + 2]};
+          const u64 kc[2] = {kC.x, kC.y}, ki[2] = {kI.x, kI.y}, ko[2] = {kO.x, kO.y};
+          const u64 ku[2] = {kU.x, kU.y}, vo[2] = {vO.x, vO.y};
+          const int q0 = 2 * y;
+          A2[q0] = plain.value ? convert(vU.x, E) : load(vU.x);
+          A2[q0 + 1] = plain.value ? convert(vU.y, E) : load(vU.y);
+          Acc a[2] = {Acc(A1[q0]), Acc(A1[q0 + 1])};
+#pragma unroll
+          for (int x = 0; x < 2; ++x) a[x].face(Dd[q0 + x], W0[q0 + x], W1[q0 + x]);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) a[x].face(A1[q0 + (x ^ 1)] - A1[q0 + x], kc[x], kc[x ^ 1]);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) a[x].face(A1[(q0 + x) ^ 2] - A1[q0 + x], kc[x], ki[x]);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) a[x].face(load(vS[x]) - A1[q0 + x], kc[x], kS[x]);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) a[x].face(load(vo[x]) - A1[q0 + x], kc[x], ko[x]);
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            const int q = 2 * y + x, side = x ? oy + 2 : oy - 1;
-            const u64 Kc = x ? kC.y : kC.x, Ku = x ? kU.y : kU.x;
-            const unsigned U0 = (unsigned)Kc + (unsigned)Ku;
-            const unsigned U1 = (unsigned)(Kc >> 32) + (unsigned)(Ku >> 32);
-            Acc a(A1[q]);
-            a.face(A2[q] - A1[q], U0, U1);
-            a.face(Dd[q], W0[q], W1[q]);
-            a.face(A1[q ^ 1] - A1[q], Kc, x ? kC.x : kC.y);
-            a.face(load(sk.u[side]) - A1[q], Kc, sk.k[side]);
-            a.face(A1[q ^ 2] - A1[q], Kc, x ? kI.y : kI.x);
-            a.face(load(x ? vO.y : vO.x) - A1[q], Kc, x ? kO.y : kO.x);
-            if constexpr (RHS) a.add(rr[q], E);
-            const double v = a.rounded();
-          if ((x ? x1 : x0) && (y ? y1 : y0)) {
-            const int h = (int)(a.H >> 32);
-            least = min(least, plain.value ? h : h ^ (h >> 31));
-          }
-          out[x] = scaled(v, E);
+            const int q = q0 + x;
+            W0[q] = (unsigned)kc[x] + (unsigned)ku[x];
+            W1[q] = (unsigned)(kc[x] >> 32) + (unsigned)(ku[x] >> 32);
+            a[x].face(A2[q] - A1[q], W0[q], W1[q]);
             Dd[q] = A1[q] - A2[q];
-            W0[q] = U0, W1[q] = U1;
+            if constexpr (RHS) a[x].add(rr[q], E);
           }
-          if (y ? y1 : y0) {
-            double *wy = w + (y ? P : 0);
-            if (x0 && x1) {
-              *reinterpret_cast<double2 *>(wy) = make_double2(out[0], out[1]);
-            } else {
-              if (x0) wy[0] = out[0];
-              if (x1) wy[1] = out[1];
-            }
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int q = q0 + x;
+            const double v = a[x].rounded();
+            const int h = (int)(a[x].H >> 32);
+            least = min(least, (plain.value ? h : h ^ (h >> 31)) | skip[q]);
+            out[q] = scaled(v, E);
           }
         }
       };
@@ -521,43 +524,34 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
         patch(Bool<false>{});
 #pragma unroll
       for (int q = 0; q < 4; ++q) A1[q] = A2[q];
-      if (least < kLeast) {
-        // A result too small for the scale's units (zeros in the patch, small
-        // neighbours): point by point, planes below from global memory.
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          if (!((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0))) continue;
-          const int p = o + (q >> 1) * BX + (q & 1);
-          double *wq = w + ((q & 2 ? P : 0) + (q & 1));
-          const u64 *pd = u + (wq - un) - S;
-          const u64 Kc = sk.k[p], Kd = __ldcg(K + (pd - u));
-          *wq = point<RHS, false>(sk, sn, p, (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1), __ldcg(pd),
-                           (unsigned)Kc + (unsigned)Kd,
-                           (unsigned)(Kc >> 32) + (unsigned)(Kd >> 32), pd);
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        if (!(y ? y1 : y0)) continue;
+        double *wy = w + (y ? P : 0);
+        if (x0 && x1) {
+          *reinterpret_cast<double2 *>(wy) = make_double2(out[2 * y], out[2 * y + 1]);
+        } else {
+          if (x0) wy[0] = out[2 * y];
+          if (x1) wy[1] = out[2 * y + 1];
         }
       }
     } else {
-      // Point by point.  E = 0: A1 then holds the patch's values (bits) at the
-      // plane below.
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int p = o + (q >> 1) * BX + (q & 1);
-        const u64 below =
-            E ? (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E)) : A1[q];
-        if ((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0)) {
-          double *wq = w + ((q & 2 ? P : 0) + (q & 1));
-          const int pr = (2 * ly + (q >> 1)) * TX + 2 * lx + (q & 1);
-          const u64 *pd = u + (wq - un) - S;
-          *wq = (int)r.sg >= 0 ? point<RHS, true>(sk, sn, p, pr, below, W0[q], W1[q], pd)
-                               : point<RHS, false>(sk, sn, p, pr, below, W0[q], W1[q], pd);
-        }
-        A1[q] = sk.u[p];
         const u64 Kc = sk.k[p], Ku = sn.k[p];
         W0[q] = (unsigned)Kc + (unsigned)Ku;
         W1[q] = (unsigned)(Kc >> 32) + (unsigned)(Ku >> 32);
       }
-      E = 0;
     }
+    if (!held) {
+      E = 0;
+      sm.below[0][t] = ld2(&sk.u[o]);
+      sm.below[1][t] = ld2(&sk.u[o + BX]);
+    }
+    // No scale, or a result too small for its units (zeros in the patch, small
+    // neighbours).
+    if (least < kLeast) again |= 1u << (k - kb);
     r0 = r1;
     r1 = r2;
   }
@@ -565,6 +559,17 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   if (failed && t == 0)
     for (int p = k - 1; p <= min(k + kRing<RHS> - 2, ke); ++p)
       tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing<RHS>], (p - kb + 1) / kRing<RHS> & 1u);
+  // Marked and formed after the walk: inside it, inlined or called, it costs the
+  // loop its schedule (512^3: 808 to 930 us a step for 788).
+  for (; again && !failed; again &= again - 1) {
+    const size_t c = (size_t)(kb + __ffs(again) - 1) * S + (size_t)j * P + i;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      if (!((q & 1 ? x1 : x0) && (q & 2 ? y1 : y0))) continue;
+      const size_t g = c + (q & 2 ? P : 0) + (q & 1);
+      un[g] = point<RHS>(u + g, K + g, RHS ? rhs + g : nullptr, P, S);
+    }
+  }
   return failed;
 }
 
@@ -577,13 +582,13 @@ __device__ __forceinline__ Smem<RHS> &smem() {
 template <bool RHS>
 __global__ void __launch_bounds__(NT, kMinB)
     k_fx(const __grid_constant__ Maps maps, double *__restrict__ un, const u64 *__restrict__ u,
-         const u64 *__restrict__ K, int nx, int ny, int nz, int P, size_t S, int kchunk, int *__restrict__ err,
-         unsigned wait_limit) {
+         const u64 *__restrict__ K, const u64 *__restrict__ rhs, int nx, int ny, int nz, int P,
+         size_t S, int kchunk, int *__restrict__ err, unsigned wait_limit) {
   const int kb = 1 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
   if (kb >= ke) return;  // whole block
-  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, blockIdx.x, blockIdx.y, nx, ny, P, S, kb,
-                   ke, wait_limit) &&
+  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P, S,
+                   kb, ke, wait_limit) &&
       threadIdx.x == 0)
     atomicExch(err, 1);
 }
@@ -603,8 +608,8 @@ __global__ void __launch_bounds__(NT, kMinB)
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm + threadIdx.x)
                  : "memory");
   __syncthreads();
-  if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq, tl.tx,
-                   tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1, kWaitLimit) &&
+  if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq,
+                   (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1, kWaitLimit) &&
       threadIdx.x == 0)
     atomicExch(g.err, 1);
 }
@@ -644,7 +649,7 @@ cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_li
   dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
   return launch_chained(k_fx<RHS>, gr, NT, smem_bytes<RHS>(), st,
                         Maps{c->maps[cur], c->maps[2], c->maps[3]}, c->u[cur ^ 1],
-                        (const u64 *)c->u[cur], c->kq, g.nx, g.ny, g.nz, g.pitch, g.plane, kc,
+                        (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny, g.nz, g.pitch, g.plane, kc,
                         c->err, wait_limit);
 }
 
@@ -656,17 +661,19 @@ int fx_tiles_x(int nx) { return (nx - 1 + TX - 1) / TX; }
 int fx_tiles_y(int ny) { return (ny - 2 + TY - 1) / TY; }
 
 // Short tiles until a table holds 1.7 blocks for every resident one, as a small
-// grid alone wants (64^3: 4.8 us a step at 1 plane, 6.7 at 2, 9.9 at 8).
+// grid alone wants (64^3: 4.8 us a step at 1 plane, 6.7 at 2, 9.9 at 8); never
+// more than kMaxPlanes.
 int fx_fill_chunk(long tile_planes, bool rhs) {
   const long n = rhs ? resident<true>() : resident<false>();
-  return n > 0 ? (int)((3 * tile_planes + 5 * n - 1) / (5 * n)) : 16;
+  const long kc = n > 0 ? (3 * tile_planes + 5 * n - 1) / (5 * n) : 16;
+  return kc < 1 ? 1 : kc < kMaxPlanes ? (int)kc : kMaxPlanes;
 }
 
 // A chunk's start, its first loads, costs about a plane's time; 384^3 runs 329 us
 // a step at 20 planes, 355 at 191.
 int fx_chunk(const heat_geom &g, bool rhs) {
   return balanced_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny), g.nz - 2,
-                        rhs ? resident<true>() : resident<false>(), 1, 0.53, 32);
+                        rhs ? resident<true>() : resident<false>(), 1, 0.53, kMaxPlanes);
 }
 
 bool fx_usable(bool rhs) { return rhs ? usable<true>() : usable<false>(); }

@@ -141,7 +141,7 @@ __device__ __forceinline__ double encode(i64 acc, int E) {
   return ldexp((double)acc, E - 1084);  // subnormal or overflowing result
 }
 
-__device__ __noinline__ double slow_point(double uc, double ue, double uw, double un, double us,
+__device__ __forceinline__ double slow_point(double uc, double ue, double uw, double un, double us,
                                           double uu, double ud, double r, u64 Kc, u64 Ke,
                                           u64 Kw, u64 Kn, u64 Ks, u64 Ku, u64 Kd) {
   const double s = 0x1p-64;
