@@ -21,6 +21,7 @@
 namespace heat {
 namespace {
 
+typedef unsigned long long u64;
 using walk::combine;
 using walk::flux;
 
@@ -45,50 +46,82 @@ __global__ void k_naive(double *__restrict__ un, const double *__restrict__ u,
   un[c] = combine(RHS ? __dadd_rn(uc, rhs[c]) : uc, factor, A, B, C, D, E, F);
 }
 
-// z-marching kernel.  A (32 x 8) thread tile walks a chunk of planes; each
-// thread owns one column i of RY adjacent rows, and the lower flux and the
-// z-neighbours of each row stay in registers.  Two face fluxes are shared
-// instead of recomputed (a face flux is the same rounded value seen from both
-// cells that share the face):
+// fl(k d) on the integer pipes, for k in [2^-200, 2^200) and d zero or of a size in
+// [2^-723, 2^677); otherwise odd is set.  The 106-bit product of the significands
+// keeps its first 53 bits; the next 32, and an or of the rest below them, round to
+// nearest even through a carry that may run on into the exponent field.
+__device__ __forceinline__ double product(double k, double d, bool &odd) {
+  const unsigned kh = (unsigned)__double2hiint(k), kl = (unsigned)__double2loint(k);
+  const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
+  const unsigned tk = kh & 0x7ff00000u, td = dh & 0x7ff00000u;
+  const unsigned b1 = __funnelshift_l(kl, kh, 11) | 0x80000000u, b0 = kl << 11;
+  const unsigned a1 = (dh & 0xfffffu) | 0x100000u, a0 = dl;
+  const u64 p00 = (u64)a0 * b0, p01 = (u64)a0 * b1 + (p00 >> 32);
+  const u64 p10 = (u64)a1 * b0 + (unsigned)p01;
+  const u64 p11 = (u64)a1 * b1 + (p01 >> 32) + (p10 >> 32);
+  const unsigned h1 = (unsigned)(p11 >> 32), h0 = (unsigned)p11, l1 = (unsigned)p10;
+  const unsigned top = h1 & 0x100000u, n = (top >> 20) ^ 1;
+  const unsigned m1 = __funnelshift_l(h0, h1, n), m0 = __funnelshift_l(l1, h0, n);
+  const unsigned x = __funnelshift_l((unsigned)p00, l1, n) | ((unsigned)p00 >> 11);
+  const u64 carry = (u64)x + 0x7fffffffu + (m0 & 1) >> 32;
+  u64 r = (((u64)m1 << 32) | m0) + carry + ((u64)(td + tk + top - (1024u << 20)) << 32);
+  if (td == 0) r = 0;
+  odd |= kh - (823u << 20) >= (400u << 20) ||
+         (td - (300u << 20) > (1400u << 20) && ((dh << 1) | dl) != 0);
+  return __hiloint2double((int)((unsigned)(r >> 32) | (dh & 0x80000000u)), (int)(unsigned)r);
+}
+
+// z-marching kernel.  A thread walks a chunk of planes; it owns one column i of RY
+// adjacent rows, and the lower flux and the z-neighbours of each row stay in
+// registers.  Two face fluxes are shared instead of recomputed (a face flux is the
+// same rounded value seen from both cells that share the face):
 //   - x: B at column i is A of column i-1 (same operands, same order), taken
-//     from the neighbouring lane.  A warp covers 31 output columns; its lane 0
-//     walks the column west of them only to hand over its A.  Lanes past the
-//     grid's interior walk the last interior column (in-bounds loads) and
-//     store nothing.
+//     from the neighbouring lane.
 //   - y: C of row j is D of row j+1, so a thread computes RY+1 y-fluxes for
 //     its RY outputs instead of 2 RY.  Row t of a thread (t = 0 .. RY+1) is
 //     grid row j0-1+t; rows past the grid are clamped to the last row so every
 //     load stays in bounds, and only interior rows store (an interior row reads
 //     rows j-1, j, j+1 only, none of them clamped).
+// Columns 0 .. nx-2 of each group of RY rows (column 0 only hands over its A) are
+// laid end to end and cut into warps of 31, the last lane of one repeated as lane
+// 0 of the next: tiles of 31 columns leave 15 % of the lanes idle at 160 columns,
+// 9 % at 256.  (Lane counts fit an int for any field that fits the GPU.)
 // RAW forms the face kappa sums from kappa as the reference does each step
 // (the drop-in heat_update); otherwise they are read precomputed, once per
 // context: kx[c] = kappa[c] + kappa[c+1], ky[c] = kappa[c] + kappa[c+P],
 // kz[c] = kappa[c] + kappa[c+S] -- the same values, fewer additions per point.
-// Three rows per thread measured best at 512^3 (GLUP/s, drop-in / context
-// form): one row 24.0 / 31.9, two 26.4 / 34.6, three 26.7 / 35.1, four
-// 26.3 / 34.5 (123 registers).
-constexpr int TX = 32, TY = 8;
-constexpr int SX = 31;
+//
+// Bound: the FP64 pipe, which retires about 530 G operations/s, 1/32 of the
+// integer pipes' rate.  A point takes 13.7 of them in the reference's order (1 more
+// with a source term, 3.3 more for RAW); its 3.3 products are formed on the integer
+// pipes instead, about 40 instructions each.  Where a lane's product is out of
+// product()'s range the lane forms the plane's fluxes again in FP64.
+// GLUP/s, all products in FP64 -> this: context form 160^3 with source 22 -> 32, 256^3 30
+// -> 46, 512^3 35.5 -> 48.4; drop-in 256^3 with source 24 -> 33, 512^3 28.5 -> 36.4.
+// Three rows per thread at 128 threads and 3 blocks per SM (168 registers) measured
+// best; two rows 36.3 at 512^3, four 48.1; 4 blocks 47.6, 5 blocks 48.0, 8-warp blocks
+// of 160 registers 40.6.
+constexpr int NW = 4;
 constexpr int RY = 3;
+constexpr int MINB = 3;
 
 template <bool RHS, bool RAW>
-__global__ void __launch_bounds__(TX *TY)
+__global__ void __launch_bounds__(32 * NW, MINB)
     k_exact_rows(double *__restrict__ un, const double *__restrict__ u,
                  const double *__restrict__ rhs, const double *__restrict__ kap,
                  const double *__restrict__ kx, const double *__restrict__ ky,
                  const double *__restrict__ kz, int nx, int ny, int nz, int P, size_t S,
                  double factor, int kchunk) {
-  const int lane = threadIdx.x;
-  const int i = blockIdx.x * SX + lane;  // lane 0: the column west of the outputs
-  const int j0 = 1 + (blockIdx.y * TY + threadIdx.y) * RY;
+  const int lane = threadIdx.x % 32;
+  // Lane 0 repeats the last column of the warp before.
+  const int at = (blockIdx.x * NW + threadIdx.x / 32) * 31 + lane;
+  const int i = at % (nx - 1), j0 = 1 + at / (nx - 1) * RY;
   const int kb = 1 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
-  if (j0 >= ny - 1 || kb >= ke) return;  // uniform across the warp
-  const bool xs = lane >= 1 && i <= nx - 2;
-  const int ic = min(i, nx - 2);
+  const bool xs = lane >= 1 && i >= 1;
   size_t ro[RY + 2];
 #pragma unroll
-  for (int t = 0; t < RY + 2; ++t) ro[t] = (size_t)min(j0 - 1 + t, ny - 1) * P + ic;
+  for (int t = 0; t < RY + 2; ++t) ro[t] = (size_t)min(j0 - 1 + t, ny - 1) * P + i;
   size_t pl = (size_t)kb * S;
   double uc[RY + 2], kc[RY + 2], F[RY];
 #pragma unroll
@@ -103,29 +136,37 @@ __global__ void __launch_bounds__(TX *TY)
                : flux(kz[q], uc[r + 1], u[q]);
   }
   for (int k = kb; k < ke; ++k, pl += S) {
-    double uu[RY + 2], ku[RY + 2], G[RY + 1];
+    double uu[RY + 2], ku[RY + 2], A[RY], E[RY], G[RY + 1];
 #pragma unroll
     for (int t = 0; t < RY + 2; ++t) {
       uu[t] = u[pl + S + ro[t]];
       ku[t] = RAW ? kap[pl + S + ro[t]] : 0.0;
     }
-    // G[t]: the flux through the face between rows t and t+1
+    // A and E of each row; G[t]: the flux through the face between rows t and t+1
+    auto fluxes = [&](auto mul) {
 #pragma unroll
-    for (int t = 0; t <= RY; ++t)
-      G[t] = RAW ? flux(__dadd_rn(kc[t + 1], kc[t]), uc[t + 1], uc[t])
-                 : flux(ky[pl + ro[t]], uc[t + 1], uc[t]);
+      for (int t = 0; t <= RY; ++t)
+        G[t] = mul(RAW ? __dadd_rn(kc[t + 1], kc[t]) : ky[pl + ro[t]], __dsub_rn(uc[t + 1], uc[t]));
+#pragma unroll
+      for (int r = 0; r < RY; ++r) {
+        const int t = r + 1;
+        const size_t q = pl + ro[t];
+        A[r] = mul(RAW ? __dadd_rn(kap[q + 1], kc[t]) : kx[q], __dsub_rn(u[q + 1], uc[t]));
+        E[r] = mul(RAW ? __dadd_rn(ku[t], kc[t]) : kz[q], __dsub_rn(uu[t], uc[t]));
+      }
+    };
+    bool odd = false;
+    fluxes([&](double k, double d) { return product(k, d, odd); });
+    if (odd) fluxes([&](double k, double d) { return __dmul_rn(k, d); });
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
       const int t = r + 1;
       const size_t q = pl + ro[t];
-      const double A = RAW ? flux(__dadd_rn(kap[q + 1], kc[t]), u[q + 1], uc[t])
-                           : flux(kx[q], u[q + 1], uc[t]);
-      const double B = __shfl_up_sync(0xffffffffu, A, 1);
-      const double E = RAW ? flux(__dadd_rn(ku[t], kc[t]), uu[t], uc[t]) : flux(kz[q], uu[t], uc[t]);
+      const double B = __shfl_up_sync(0xffffffffu, A[r], 1);
       if (xs && j0 + r <= ny - 2)
-        un[q] = combine(RHS ? __dadd_rn(uc[t], rhs[q]) : uc[t], factor, A, B, G[t], G[t - 1], E,
+        un[q] = combine(RHS ? __dadd_rn(uc[t], rhs[q]) : uc[t], factor, A[r], B, G[t], G[t - 1], E[r],
                         F[r]);
-      F[r] = E;
+      F[r] = E[r];
     }
 #pragma unroll
     for (int t = 0; t < RY + 2; ++t) {
@@ -138,11 +179,12 @@ __global__ void __launch_bounds__(TX *TY)
 template <bool RHS, bool RAW>
 void launch_rows(double *u_new, const double *u_old, const double *rhs, const double *kappa,
                  double *const ks[3], const heat_geom &g, double factor, cudaStream_t st) {
-  static const long resident = resident_blocks((const void *)k_exact_rows<RHS, RAW>, TX * TY, 0);
-  const int kc = wave_chunk(g, SX, TY * RY, resident);
-  dim3 gr((g.nx - 2 + SX - 1) / SX, (g.ny - 2 + TY * RY - 1) / (TY * RY),
-          (g.nz - 2 + kc - 1) / kc);
-  k_exact_rows<RHS, RAW><<<gr, dim3(TX, TY), 0, st>>>(
+  static const long resident = resident_blocks((const void *)k_exact_rows<RHS, RAW>, 32 * NW, 0);
+  const long lanes = (long)((g.ny - 2 + RY - 1) / RY) * (g.nx - 1);
+  const int blocks = (int)((lanes + 31 * NW - 1) / (31 * NW));
+  const int kc = balanced_chunk(blocks, g.nz - 2, resident, 2, 0.6, 32);
+  dim3 gr(blocks, 1, (g.nz - 2 + kc - 1) / kc);
+  k_exact_rows<RHS, RAW><<<gr, 32 * NW, 0, st>>>(
       u_new, u_old, rhs, kappa, ks ? ks[0] : nullptr, ks ? ks[1] : nullptr,
       ks ? ks[2] : nullptr, g.nx, g.ny, g.nz, g.pitch, g.plane, factor, kc);
 }

@@ -180,18 +180,18 @@ inline int balanced_chunk(long tiles, int interior, long resident, int overhead,
                           int most) {
   if (resident <= 0) return interior < 32 ? interior : 32;
   const long per_sm = (resident + 151) / 152;
-  const int first = (interior + most - 1) / most;
   double best = 0;
-  int best_kc = interior;
-  for (int c = first; c <= interior && c < first + 256; ++c) {
-    const int kc = (interior + c - 1) / c;
-    const long blocks = tiles * ((interior + kc - 1) / kc);
+  int best_kc = 0;
+  for (int most_kc = interior < most ? interior : most; most_kc >= 1; --most_kc) {
+    const int chunks = (interior + most_kc - 1) / most_kc;
+    const int kc = (interior + chunks - 1) / chunks;
+    const long blocks = tiles * chunks;
     const long rest = (blocks % resident + 151) / 152;  // blocks per SM in the last round
     double rounds = (double)(blocks / resident);
     if (rest)
       rounds += alone + (1.0 - alone) * std::sqrt((double)(rest - 1) / (per_sm > 1 ? per_sm - 1 : 1));
     const double cost = rounds * (kc + overhead);
-    if (c == first || cost < best) {
+    if (best_kc == 0 || cost < best) {
       best = cost;
       best_kc = kc;
     }
