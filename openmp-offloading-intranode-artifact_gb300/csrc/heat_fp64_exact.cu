@@ -46,29 +46,64 @@ __global__ void k_naive(double *__restrict__ un, const double *__restrict__ u,
   un[c] = combine(RHS ? __dadd_rn(uc, rhs[c]) : uc, factor, A, B, C, D, E, F);
 }
 
-// fl(k d) on the integer pipes, for k in [2^-200, 2^200) and d zero or of a size in
-// [2^-723, 2^677); otherwise odd is set.  The 106-bit product of the significands
-// keeps its first 53 bits; the next 32, and an or of the rest below them, round to
-// nearest even through a carry that may run on into the exponent field.
-__device__ __forceinline__ double product(double k, double d, bool &odd) {
-  const unsigned kh = (unsigned)__double2hiint(k), kl = (unsigned)__double2loint(k);
-  const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
-  const unsigned tk = kh & 0x7ff00000u, td = dh & 0x7ff00000u;
-  const unsigned b1 = __funnelshift_l(kl, kh, 11) | 0x80000000u, b0 = kl << 11;
-  const unsigned a1 = (dh & 0xfffffu) | 0x100000u, a0 = dl;
-  const u64 p00 = (u64)a0 * b0, p01 = (u64)a0 * b1 + (p00 >> 32);
-  const u64 p10 = (u64)a1 * b0 + (unsigned)p01;
-  const u64 p11 = (u64)a1 * b1 + (p01 >> 32) + (p10 >> 32);
+__device__ __forceinline__ u64 shr(u64 a, unsigned n) {  // 0 for n >= 64
+  u64 r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
+  return r;
+}
+// A conductivity as an integer with its leading bit at 62, so that a sum of two
+// fits, and its exponent field.  Zeros and subnormals (a plain significand beside
+// the field 0) need no care in a sum that is in range; negative values are odd.
+struct Int {
+  u64 m;
+  unsigned e;
+};
+__device__ __forceinline__ Int integer(double v, bool &odd) {
+  const unsigned hi = (unsigned)__double2hiint(v);
+  odd |= (int)hi < 0;
+  const unsigned h = (hi & 0xfffffu) | min(hi & 0x7ff00000u, 0x100000u);
+  return {(((u64)h << 32) | (unsigned)__double2loint(v)) << 10, hi >> 20};
+}
+
+// A sum of two conductivities in [2^-200, 2^200): exponent field (in place) and
+// significand, its leading bit at 63.
+struct Weight {
+  unsigned h, l, t;
+};
+__device__ __forceinline__ Weight weight(double k, bool &odd) {
+  const unsigned hi = (unsigned)__double2hiint(k), lo = (unsigned)__double2loint(k);
+  odd |= hi - (823u << 20) >= (400u << 20);
+  return {__funnelshift_l(lo, hi, 11) | 0x80000000u, lo << 11, hi & 0x7ff00000u};
+}
+// fl(a + b).  Where an operand is shifted by more than its 10 zero bits the sum
+// lacks less than a unit, which matters to the rounding of a tie only: odd, as a
+// sum that rounds up to a power of two.
+__device__ __forceinline__ Weight sum(const Int &a, const Int &b, bool &odd) {
+  const unsigned e = max(a.e, b.e), da = e - a.e, db = e - b.e;
+  const u64 s = shr(a.m, da) + shr(b.m, db);
+  const unsigned n = (unsigned)(s >> 63) ^ 1, t = (e + 1 - n) << 20;
+  const u64 x = s << n, y = x + 0x3ff + (x >> 11 & 1);
+  odd |= y < x || (da + db > 10 && (x & 0x7ff) == 0x400) || t - (823u << 20) >= (400u << 20);
+  return {(unsigned)(y >> 32), (unsigned)y & ~0x7ffu, t};
+}
+// fl(k d), for d zero or of a size in [2^-723, 2^677).  The 106-bit product of the significands keeps its first 53 bits; the
+// next 32, and an or of the rest below them, round to nearest even through a
+// carry that may run on into the exponent field.
+__device__ __forceinline__ double product(const Weight &k, double d, bool &odd) {
+  const unsigned hi = (unsigned)__double2hiint(d), a0 = (unsigned)__double2loint(d);
+  const unsigned t = hi & 0x7ff00000u, a1 = (hi & 0xfffffu) | 0x100000u;
+  const u64 p00 = (u64)a0 * k.l, p01 = (u64)a0 * k.h + (p00 >> 32);
+  const u64 p10 = (u64)a1 * k.l + (unsigned)p01;
+  const u64 p11 = (u64)a1 * k.h + (p01 >> 32) + (p10 >> 32);
   const unsigned h1 = (unsigned)(p11 >> 32), h0 = (unsigned)p11, l1 = (unsigned)p10;
   const unsigned top = h1 & 0x100000u, n = (top >> 20) ^ 1;
   const unsigned m1 = __funnelshift_l(h0, h1, n), m0 = __funnelshift_l(l1, h0, n);
   const unsigned x = __funnelshift_l((unsigned)p00, l1, n) | ((unsigned)p00 >> 11);
-  const u64 carry = (u64)x + 0x7fffffffu + (m0 & 1) >> 32;
-  u64 r = (((u64)m1 << 32) | m0) + carry + ((u64)(td + tk + top - (1024u << 20)) << 32);
-  if (td == 0) r = 0;
-  odd |= kh - (823u << 20) >= (400u << 20) ||
-         (td - (300u << 20) > (1400u << 20) && ((dh << 1) | dl) != 0);
-  return __hiloint2double((int)((unsigned)(r >> 32) | (dh & 0x80000000u)), (int)(unsigned)r);
+  const u64 carry = ((u64)x + 0x7fffffffu + (m0 & 1)) >> 32;
+  u64 r = (((u64)m1 << 32) | m0) + carry + ((u64)(t + k.t + top - (1024u << 20)) << 32);
+  if (t == 0) r = 0;
+  odd |= t - (300u << 20) > (1400u << 20) && ((hi << 1) | a0) != 0;
+  return __hiloint2double((int)((unsigned)(r >> 32) | (hi & 0x80000000u)), (int)(unsigned)r);
 }
 
 // z-marching kernel.  A thread walks a chunk of planes; it owns one column i of RY
@@ -93,28 +128,31 @@ __device__ __forceinline__ double product(double k, double d, bool &odd) {
 //
 // Bound: the FP64 pipe, which retires about 530 G operations/s, 1/32 of the
 // integer pipes' rate.  A point takes 13.7 of them in the reference's order (1 more
-// with a source term, 3.3 more for RAW); its 3.3 products are formed on the integer
-// pipes instead, about 40 instructions each.  Where a lane's product is out of
-// product()'s range the lane forms the plane's fluxes again in FP64.
-// GLUP/s, all products in FP64 -> this: context form 160^3 with source 22 -> 32, 256^3 30
-// -> 46, 512^3 35.5 -> 48.4; drop-in 256^3 with source 24 -> 33, 512^3 28.5 -> 36.4.
-// Three rows per thread at 128 threads and 3 blocks per SM (168 registers) measured
-// best; two rows 36.3 at 512^3, four 48.1; 4 blocks 47.6, 5 blocks 48.0, 8-warp blocks
-// of 160 registers 40.6.
-constexpr int NW = 4;
+// with a source term, 3.3 more for RAW).  Its 3.3 products, and RAW's sums of
+// conductivities, are formed on the integer pipes instead (about 40 instructions
+// for a product, 30 for a sum), which leaves 10.3: 51 GLUP/s, 47 with a source
+// term.  Where an operand is out of their range the lane forms the plane's fluxes
+// again in FP64.  The differences stay on the FP64 pipe: in integers they must be
+// normalised (512^3, GLUP/s: those along z 42 for 48, all 28).
+// GLUP/s, all operations in FP64 -> this: context form 160^3 with source 22 -> 38,
+// 256^3 30 -> 46, 512^3 35.5 -> 48.4; drop-in 256^3 with source 24 -> 41, 512^3
+// 28.5 -> 46.8 (36.4 with its sums in FP64).
+// Blocks are single warps, 12 per SM (168 registers), so that few are left over at
+// the end: 160^3 110 us a step for 126 with 4 warps.  Four rows per thread 38.6 for
+// 41.6 (drop-in 256^3), two 36 for 48 (512^3).
 constexpr int RY = 3;
-constexpr int MINB = 3;
+constexpr int MINB = 12;
 
 template <bool RHS, bool RAW>
-__global__ void __launch_bounds__(32 * NW, MINB)
+__global__ void __launch_bounds__(32, MINB)
     k_exact_rows(double *__restrict__ un, const double *__restrict__ u,
                  const double *__restrict__ rhs, const double *__restrict__ kap,
                  const double *__restrict__ kx, const double *__restrict__ ky,
                  const double *__restrict__ kz, int nx, int ny, int nz, int P, size_t S,
                  double factor, int kchunk) {
-  const int lane = threadIdx.x % 32;
+  const int lane = threadIdx.x;
   // Lane 0 repeats the last column of the warp before.
-  const int at = (blockIdx.x * NW + threadIdx.x / 32) * 31 + lane;
+  const int at = blockIdx.x * 31 + lane;
   const int i = at % (nx - 1), j0 = 1 + at / (nx - 1) * RY;
   const int kb = 1 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
@@ -124,10 +162,13 @@ __global__ void __launch_bounds__(32 * NW, MINB)
   for (int t = 0; t < RY + 2; ++t) ro[t] = (size_t)min(j0 - 1 + t, ny - 1) * P + i;
   size_t pl = (size_t)kb * S;
   double uc[RY + 2], kc[RY + 2], F[RY];
+  Int wc[RY + 2];     // kc again
+  bool below = false;  // a conductivity below zero was seen
 #pragma unroll
   for (int t = 0; t < RY + 2; ++t) {
     uc[t] = u[pl + ro[t]];
     kc[t] = RAW ? kap[pl + ro[t]] : 0.0;
+    wc[t] = integer(kc[t], below);
   }
 #pragma unroll
   for (int r = 0; r < RY; ++r) {
@@ -137,27 +178,39 @@ __global__ void __launch_bounds__(32 * NW, MINB)
   }
   for (int k = kb; k < ke; ++k, pl += S) {
     double uu[RY + 2], ku[RY + 2], A[RY], E[RY], G[RY + 1];
+    Int wu[RY + 2];
 #pragma unroll
     for (int t = 0; t < RY + 2; ++t) {
       uu[t] = u[pl + S + ro[t]];
       ku[t] = RAW ? kap[pl + S + ro[t]] : 0.0;
+      wu[t] = integer(ku[t], below);
     }
     // A and E of each row; G[t]: the flux through the face between rows t and t+1
-    auto fluxes = [&](auto mul) {
+    bool odd = false;
+#pragma unroll
+    for (int t = 0; t <= RY; ++t)
+      G[t] = product(RAW ? sum(wc[t + 1], wc[t], odd) : weight(ky[pl + ro[t]], odd),
+                     __dsub_rn(uc[t + 1], uc[t]), odd);
+#pragma unroll
+    for (int r = 0; r < RY; ++r) {
+      const int t = r + 1;
+      const size_t q = pl + ro[t];
+      A[r] = product(RAW ? sum(integer(kap[q + 1], below), wc[t], odd) : weight(kx[q], odd),
+                     __dsub_rn(u[q + 1], uc[t]), odd);
+      E[r] = product(RAW ? sum(wu[t], wc[t], odd) : weight(kz[q], odd), __dsub_rn(uu[t], uc[t]), odd);
+    }
+    if (odd || below) {
 #pragma unroll
       for (int t = 0; t <= RY; ++t)
-        G[t] = mul(RAW ? __dadd_rn(kc[t + 1], kc[t]) : ky[pl + ro[t]], __dsub_rn(uc[t + 1], uc[t]));
+        G[t] = flux(RAW ? __dadd_rn(kc[t + 1], kc[t]) : ky[pl + ro[t]], uc[t + 1], uc[t]);
 #pragma unroll
       for (int r = 0; r < RY; ++r) {
         const int t = r + 1;
         const size_t q = pl + ro[t];
-        A[r] = mul(RAW ? __dadd_rn(kap[q + 1], kc[t]) : kx[q], __dsub_rn(u[q + 1], uc[t]));
-        E[r] = mul(RAW ? __dadd_rn(ku[t], kc[t]) : kz[q], __dsub_rn(uu[t], uc[t]));
+        A[r] = flux(RAW ? __dadd_rn(kap[q + 1], kc[t]) : kx[q], u[q + 1], uc[t]);
+        E[r] = flux(RAW ? __dadd_rn(ku[t], kc[t]) : kz[q], uu[t], uc[t]);
       }
-    };
-    bool odd = false;
-    fluxes([&](double k, double d) { return product(k, d, odd); });
-    if (odd) fluxes([&](double k, double d) { return __dmul_rn(k, d); });
+    }
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
       const int t = r + 1;
@@ -172,6 +225,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     for (int t = 0; t < RY + 2; ++t) {
       uc[t] = uu[t];
       kc[t] = ku[t];
+      wc[t] = wu[t];
     }
   }
 }
@@ -179,12 +233,14 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 template <bool RHS, bool RAW>
 void launch_rows(double *u_new, const double *u_old, const double *rhs, const double *kappa,
                  double *const ks[3], const heat_geom &g, double factor, cudaStream_t st) {
-  static const long resident = resident_blocks((const void *)k_exact_rows<RHS, RAW>, 32 * NW, 0);
+  static const long resident = resident_blocks((const void *)k_exact_rows<RHS, RAW>, 32, 0);
   const long lanes = (long)((g.ny - 2 + RY - 1) / RY) * (g.nx - 1);
-  const int blocks = (int)((lanes + 31 * NW - 1) / (31 * NW));
-  const int kc = balanced_chunk(blocks, g.nz - 2, resident, 2, 0.6, 32);
+  const int blocks = (int)((lanes + 30) / 31);
+  // Short chunks cost little here (at 192^3 162 us a step with 6 planes, 169 with 16,
+  // 198 with 32), and long ones leave SMs idle at the end.
+  const int kc = balanced_chunk(blocks, g.nz - 2, resident, 1, 0.4, 10);
   dim3 gr(blocks, 1, (g.nz - 2 + kc - 1) / kc);
-  k_exact_rows<RHS, RAW><<<gr, 32 * NW, 0, st>>>(
+  k_exact_rows<RHS, RAW><<<gr, 32, 0, st>>>(
       u_new, u_old, rhs, kappa, ks ? ks[0] : nullptr, ks ? ks[1] : nullptr,
       ks ? ks[2] : nullptr, g.nx, g.ny, g.nz, g.pitch, g.plane, factor, kc);
 }
