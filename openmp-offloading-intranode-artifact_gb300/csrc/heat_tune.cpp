@@ -171,12 +171,16 @@ double time_candidate(std::vector<heat_ctx *> &cs, heat_batch *b, const heat::Tu
 
 namespace heat {
 
-TuneChoice tuned_choice(int form, int nz) {
+TuneChoice tuned_choice(int form, int nz, bool *tuned) {
   std::lock_guard<std::mutex> lk(g_mu);
   load_locked();
   const int cls = class_of(nz);
   for (const TuneEntry &t : g_table)
-    if (t.form == form && t.nz_max == cls) return t.ch;
+    if (t.form == form && t.nz_max == cls) {
+      if (tuned) *tuned = true;
+      return t.ch;
+    }
+  if (tuned) *tuned = false;
   return default_choice(form);
 }
 
