@@ -126,22 +126,26 @@ __device__ __forceinline__ double product(const Weight &k, double d, bool &odd) 
 // context: kx[c] = kappa[c] + kappa[c+1], ky[c] = kappa[c] + kappa[c+P],
 // kz[c] = kappa[c] + kappa[c+S] -- the same values, fewer additions per point.
 //
-// Bound: the FP64 pipe, which retires about 530 G operations/s, 1/32 of the
-// integer pipes' rate.  A point takes 13.7 of them in the reference's order (1 more
+// Bound: the FP64 pipe (83 % busy, which is all that additions reach), which
+// retires about 530 G operations/s, 1/32 of the integer pipes' rate.  A point takes 13.7 of them in the reference's order (1 more
 // with a source term, 3.3 more for RAW).  Its 3.3 products, and RAW's sums of
 // conductivities, are formed on the integer pipes instead (about 40 instructions
-// for a product, 30 for a sum), which leaves 10.3: 51 GLUP/s, 47 with a source
-// term.  Where an operand is out of their range the lane forms the plane's fluxes
-// again in FP64.  The differences stay on the FP64 pipe: in integers they must be
-// normalised (512^3, GLUP/s: those along z 42 for 48, all 28).
+// for a product, 30 for a sum), and so is the one of the step factor but where RAW
+// and a source term leave no registers (drop-in 256^3 with source 406 us a step so,
+// 400 with it in FP64; without source 2.76 ms for 2.86 at 512^3).  That leaves 9.3
+// additions.  Where an operand is out of their range the lane forms the plane's
+// products again in FP64.  The differences stay on the FP64 pipe: in integers they
+// must be normalised (512^3, GLUP/s: those along z 42 for 48, all 28).
 // GLUP/s, all operations in FP64 -> this: context form 160^3 with source 22 -> 38,
-// 256^3 30 -> 46, 512^3 35.5 -> 48.4; drop-in 256^3 with source 24 -> 41, 512^3
-// 28.5 -> 46.8 (36.4 with its sums in FP64).
+// 256^3 30 -> 49.5, 512^3 35.5 -> 52.6; drop-in 256^3 with source 24 -> 41, 512^3
+// 28.5 -> 48.
 // Blocks are single warps, 12 per SM (168 registers), so that few are left over at
 // the end: 160^3 110 us a step for 126 with 4 warps.  Four rows per thread 38.6 for
 // 41.6 (drop-in 256^3), two 36 for 48 (512^3).
 constexpr int RY = 3;
 constexpr int MINB = 12;
+template <bool RHS, bool RAW>
+constexpr bool kScaled = !(RHS && RAW);
 
 template <bool RHS, bool RAW>
 __global__ void __launch_bounds__(32, MINB)
@@ -160,6 +164,8 @@ __global__ void __launch_bounds__(32, MINB)
   size_t ro[RY + 2];
 #pragma unroll
   for (int t = 0; t < RY + 2; ++t) ro[t] = (size_t)min(j0 - 1 + t, ny - 1) * P + i;
+  bool wide = false;  // the factor is out of product()'s range
+  const Weight w = weight(factor, wide);
   size_t pl = (size_t)kb * S;
   double uc[RY + 2], kc[RY + 2], F[RY];
   Int wc[RY + 2];     // kc again
@@ -211,15 +217,25 @@ __global__ void __launch_bounds__(32, MINB)
         E[r] = flux(RAW ? __dadd_rn(ku[t], kc[t]) : kz[q], uu[t], uc[t]);
       }
     }
+    double s[RY], ds[RY];
+    bool far = wide;
+#pragma unroll
+    for (int r = 0; r < RY; ++r) {
+      const double B = __shfl_up_sync(0xffffffffu, A[r], 1);
+      s[r] = walk::net(A[r], B, G[r + 1], G[r], E[r], F[r]);
+      ds[r] = kScaled<RHS, RAW> ? product(w, s[r], far) : __dmul_rn(factor, s[r]);
+      F[r] = E[r];
+    }
+    if (kScaled<RHS, RAW> && far) {
+      __threadfence_block();  // or the compiler forms these for every lane and selects
+#pragma unroll
+      for (int r = 0; r < RY; ++r) ds[r] = __dmul_rn(factor, s[r]);
+    }
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
       const int t = r + 1;
       const size_t q = pl + ro[t];
-      const double B = __shfl_up_sync(0xffffffffu, A[r], 1);
-      if (xs && j0 + r <= ny - 2)
-        un[q] = combine(RHS ? __dadd_rn(uc[t], rhs[q]) : uc[t], factor, A[r], B, G[t], G[t - 1], E[r],
-                        F[r]);
-      F[r] = E[r];
+      if (xs && j0 + r <= ny - 2) un[q] = __dadd_rn(RHS ? __dadd_rn(uc[t], rhs[q]) : uc[t], ds[r]);
     }
 #pragma unroll
     for (int t = 0; t < RY + 2; ++t) {

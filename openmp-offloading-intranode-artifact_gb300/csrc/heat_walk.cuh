@@ -54,12 +54,16 @@ __device__ __forceinline__ double flux(double ksum, double ub, double ua) {
   return __dmul_rn(ksum, __dsub_rn(ub, ua));
 }
 
+// The sum of the face fluxes in the reference's order.
+__device__ __forceinline__ double net(double A, double B, double C, double D, double E, double F) {
+  return __dsub_rn(__dadd_rn(__dsub_rn(__dadd_rn(__dsub_rn(A, B), C), D), E), F);
+}
+
 // base is u + rhs (or u alone when the problem has no source term: u + 0.0
 // equals u for every value but -0.0, which these fields never hold).
 __device__ __forceinline__ double combine(double base, double factor, double A, double B,
                                           double C, double D, double E, double F) {
-  double s = __dsub_rn(__dadd_rn(__dsub_rn(__dadd_rn(__dsub_rn(A, B), C), D), E), F);
-  return __dadd_rn(base, __dmul_rn(factor, s));
+  return __dadd_rn(base, __dmul_rn(factor, net(A, B, C, D, E, F)));
 }
 
 template <bool RHS>
