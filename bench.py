@@ -207,13 +207,27 @@ def reference_gpu_leg(n=512, steps=300):
             "build": f"nvcc {REF_CUDA_FLAGS} -lm"}
 
 
-TRAFFIC_RECORD = ROOT / "profiles" / "fp64_default_traffic.json"
+TRAFFIC_RECORD = ROOT / "profiles" / "fp64_default_traffic.json"  # of the row-split launch before k_fx
+FX_TRAFFIC_RECORD = ROOT / "profiles" / "fp64_fx_traffic.json"
+
+
+def fx_pipe_record(n, launch_ms, peak_gops):
+    """The default form's FP64-pipe work beside the HBM roofline: two conversions
+    between FP64 and 64-bit integers per point; everything else is on the
+    integer pipes."""
+    ops = (n - 2) ** 3 * 2
+    achieved = ops / (launch_ms * 1e-3) / 1e9
+    return {"achieved_gops": round(achieved, 1), "peak_gops": round(peak_gops, 1),
+            "frac": round(achieved / peak_gops, 4) if peak_gops > 0 else None,
+            "ops_per_launch": ops,
+            "note": "2 conversions per point, the rest on the integer pipes; peak = measured FP64 FMA "
+                    "rate of this GPU (heat_diag_fp64_rate, eight independent chains per thread)"}
 
 
 def fp64_pipe_record(n, launch_ms, peak_gops):
-    """The default form's FP64-pipe work beside the HBM roofline: rows j with
-    (j - 1) mod 8 < 4 take the FP64 pipe at 7 operations per point (one multiply,
-    six fused multiply-adds), the rest the integer pipes."""
+    """The same of the row-split launch before it: rows j with (j - 1) mod 8 < 4
+    took the FP64 pipe at 7 operations per point (one multiply, six fused
+    multiply-adds), the rest the integer pipes."""
     rows = sum(1 for j in range(1, n - 1) if (j - 1) % 8 < 4)
     ops = (n - 2) * (n - 2) * rows * 7
     achieved = ops / (launch_ms * 1e-3) / 1e9
@@ -224,14 +238,14 @@ def fp64_pipe_record(n, launch_ms, peak_gops):
                     "rate of this GPU (heat_diag_fp64_rate, eight independent chains per thread)"}
 
 
-def profile_traffic(updates_per_launch):
+def profile_traffic(updates_per_launch, record=TRAFFIC_RECORD):
     """DRAM bytes (read + write) per launch of the dominant kernel: the
     machine-readable record of one ncu capture (its command and raw
     dram__bytes_read.sum / dram__bytes_write.sum of the captured launch),
     scaled from the captured launch's updates to this launch's."""
-    if not TRAFFIC_RECORD.exists():
+    if not record.exists():
         return None, None
-    rec = json.loads(TRAFFIC_RECORD.read_text())
+    rec = json.loads(record.read_text())
     cap = rec["capture"]
     per_update = (cap["dram_bytes_read"] + cap["dram_bytes_write"]) / cap["updates"]
     return per_update * updates_per_launch, {"kernel": rec["kernel"], "bytes_per_update": round(per_update, 2),
@@ -424,7 +438,7 @@ def our_arm(a):
     if rank == 0:
         peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
         hbm_peak = peaks.get("hbm_gbs", 6800.0)
-        traffic, traffic_src = profile_traffic(updates(n, 1))
+        traffic, traffic_src = profile_traffic(updates(n, 1), FX_TRAFFIC_RECORD)
         out = {
             "metric": METRIC, "value": round(value, 3), "unit": UNIT, "n_gpus": world,
             "steps": a.steps, "warmup": a.warmup, "ms_per_step": round(t_max / a.steps, 3),
@@ -440,7 +454,7 @@ def our_arm(a):
                          "traffic": traffic, "traffic_source": traffic_src,
                          "bytes_per_update": BYTES_PER_UPDATE,
                          "kernel_ms_per_launch": round(launch_ms, 4),
-                         "fp64_pipe": fp64_pipe_record(n, launch_ms, fp64_peak)},
+                         "fp64_pipe": fx_pipe_record(n, launch_ms, fp64_peak)},
             "e2e": {"value": round(e2e_value, 3), "unit": UNIT,
                     "h2d_bytes_per_step": int(pk.numel() * 8 + pu.numel() * 8),
                     "d2h_bytes_per_step": int(pout.numel() * 8),

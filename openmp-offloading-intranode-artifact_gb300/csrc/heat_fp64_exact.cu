@@ -86,9 +86,10 @@ __device__ __forceinline__ Weight sum(const Int &a, const Int &b, bool &odd) {
   odd |= y < x || (da + db > 10 && (x & 0x7ff) == 0x400) || t - (823u << 20) >= (400u << 20);
   return {(unsigned)(y >> 32), (unsigned)y & ~0x7ffu, t};
 }
-// fl(k d), for d zero or of a size in [2^-723, 2^677).  The 106-bit product of the significands keeps its first 53 bits; the
-// next 32, and an or of the rest below them, round to nearest even through a
-// carry that may run on into the exponent field.
+// fl(k d), for d zero or of a size in [2^-723, 2^677).  The 106-bit product of the
+// significands keeps its first 53 bits; the next 32, and an or of the rest below
+// them, round to nearest even through a carry that may run on into the exponent
+// field.
 __device__ __forceinline__ double product(const Weight &k, double d, bool &odd) {
   const unsigned hi = (unsigned)__double2hiint(d), a0 = (unsigned)__double2loint(d);
   const unsigned t = hi & 0x7ff00000u, a1 = (hi & 0xfffffu) | 0x100000u;
@@ -127,17 +128,18 @@ __device__ __forceinline__ double product(const Weight &k, double d, bool &odd) 
 // kz[c] = kappa[c] + kappa[c+S] -- the same values, fewer additions per point.
 //
 // Bound: the FP64 pipe (83 % busy, which is all that additions reach), which
-// retires about 530 G operations/s, 1/32 of the integer pipes' rate.  A point takes 13.7 of them in the reference's order (1 more
-// with a source term, 3.3 more for RAW).  Its 3.3 products, and RAW's sums of
-// conductivities, are formed on the integer pipes instead (about 40 instructions
-// for a product, 30 for a sum), and so is the one of the step factor but where RAW
-// and a source term leave no registers (drop-in 256^3 with source 406 us a step so,
-// 400 with it in FP64; without source 2.76 ms for 2.86 at 512^3).  That leaves 9.3
-// additions.  Where an operand is out of their range the lane forms the plane's
-// products again in FP64.  The differences stay on the FP64 pipe: in integers they
-// must be normalised (512^3, GLUP/s: those along z 42 for 48, all 28).
+// retires about 530 G operations/s, 1/32 of the integer pipes' rate.  A point takes
+// 13.7 of them in the reference's order (1 more with a source term, 3.3 more for
+// RAW).  Its 3.3 products, and RAW's sums of conductivities, are formed on the
+// integer pipes instead (about 40 instructions for a product, 30 for a sum), and so
+// is the product with the step factor, but where RAW and a source term leave no
+// registers (drop-in 256^3 with source 406 us a step so, 400 with it in FP64;
+// without source 2.75 ms for 2.86 at 512^3).  That leaves 9.3 additions.  Where an
+// operand is out of their range the lane forms the plane's products again in FP64.
+// The differences stay on the FP64 pipe: in integers they must be normalised
+// (512^3, GLUP/s: those along z 42 for 48, all 28).
 // GLUP/s, all operations in FP64 -> this: context form 160^3 with source 22 -> 38,
-// 256^3 30 -> 49.5, 512^3 35.5 -> 52.6; drop-in 256^3 with source 24 -> 41, 512^3
+// 256^3 30 -> 49.7, 512^3 35.5 -> 52.7; drop-in 256^3 with source 24 -> 41, 512^3
 // 28.5 -> 48.
 // Blocks are single warps, 12 per SM (168 registers), so that few are left over at
 // the end: 160^3 110 us a step for 126 with 4 warps.  Four rows per thread 38.6 for
@@ -203,7 +205,8 @@ __global__ void __launch_bounds__(32, MINB)
       const size_t q = pl + ro[t];
       A[r] = product(RAW ? sum(integer(kap[q + 1], below), wc[t], odd) : weight(kx[q], odd),
                      __dsub_rn(u[q + 1], uc[t]), odd);
-      E[r] = product(RAW ? sum(wu[t], wc[t], odd) : weight(kz[q], odd), __dsub_rn(uu[t], uc[t]), odd);
+      E[r] = product(RAW ? sum(wu[t], wc[t], odd) : weight(kz[q], odd), __dsub_rn(uu[t], uc[t]),
+                     odd);
     }
     if (odd || below) {
 #pragma unroll

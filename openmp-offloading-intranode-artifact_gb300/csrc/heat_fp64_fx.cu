@@ -54,13 +54,14 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 168 GLUP/s (0.79 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 167 GLUP/s (0.79 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 149 (115.7);
-// 192^3 with a narrow Gaussian 134, 160 without.
+// the launch before this one), with the reference's source term 148 (115.7);
+// 192^3 with a narrow Gaussian 133 at first, 123 over 200 steps.
 // About 140 warp instructions per point (300 for an integer row of that
-// launch); ALU, FMA-heavy (18 of its instructions the wide multiply-adds, twice
-// the cost of the others) and issue are each about 60 % busy, DRAM 55 %.
+// launch); at 320^3 the ALU pipe is 58 % busy, FMA-heavy (18 of its instructions the
+// wide multiply-adds, twice the cost of the others) the same, FP64 53 %, issue 61 %,
+// DRAM 24.6 bytes a point.
 // Measured and not kept (512^3, GLUP/s): the neighbours above and below converted
 // by the FP64 pipe as the patch's own are, 157 for 167 (that pipe is then at 75 %
 // and the others wait for it); no value converted by it 164; five blocks per SM
@@ -266,7 +267,8 @@ struct Acc {
 // (and the source term), every value cut to that scale's units; exponents near
 // either end, infinities and NaNs take walk::int_point.
 template <bool RHS>
-__device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *rhs, int P, size_t S) {
+__device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *rhs, int P,
+                                        size_t S) {
   const u64 c = __ldcg(u);
   const u64 f[6] = {__ldcg(u + S), __ldcg(u - S), __ldcg(u - 1),
                     __ldcg(u + 1), __ldcg(u - P), __ldcg(u + P)};
@@ -298,8 +300,8 @@ __device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *r
   };
   return walk::int_point<RHS>(walk::decode(c), walk::decode(f[0]), walk::decode(f[1]),
                               walk::decode(f[3]), walk::decode(f[2]), walk::decode(f[5]),
-                              walk::decode(f[4]), w(kc), w(k[0]), w(k[1]), w(k[3]), w(k[2]), w(k[5]),
-                              w(k[4]), vr,
+                              walk::decode(f[4]), w(kc), w(k[0]), w(k[1]), w(k[3]), w(k[2]),
+                              w(k[5]), w(k[4]), vr,
                               [=] { return walk::Raw7{c, f[3], f[2], f[5], f[4], f[0], f[1]}; });
 }
 
@@ -515,8 +517,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           // of the row: the plane above (U), beside it (S), the other row of the
           // patch (I) and the one outside it (O)
           const ulonglong2 vU = ld2(&sn.u[oy]), vO = ld2(&sk.u[oo]);
-          const ulonglong2 kC = ld2(&sk.k[oy]), kI = ld2(&sk.k[y ? o : o + BX]), kO = ld2(&sk.k[oo]),
-                           kU = ld2(&sn.k[oy]);
+          const ulonglong2 kC = ld2(&sk.k[oy]), kI = ld2(&sk.k[y ? o : o + BX]);
+          const ulonglong2 kO = ld2(&sk.k[oo]), kU = ld2(&sn.k[oy]);
           const u64 vS[2] = {sk.u[oy - 1], sk.u[oy + 2]}, kS[2] = {sk.k[oy - 1], sk.k[oy + 2]};
           const u64 kc[2] = {kC.x, kC.y}, ki[2] = {kI.x, kI.y}, ko[2] = {kO.x, kO.y};
           const u64 ku[2] = {kU.x, kU.y}, vo[2] = {vO.x, vO.y};
@@ -597,8 +599,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   // Marked and formed after the walk: inside it, inlined or called, it costs the
   // loop its schedule (512^3: 808 to 930 us a step for 788).
   if (__syncthreads_or(again != 0 && !failed))
-    form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs, tx,
-                    ty, kb, nx, ny, P, S);
+    form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs,
+                    tx, ty, kb, nx, ny, P, S);
   return failed;
 }
 
@@ -616,8 +618,8 @@ __global__ void __launch_bounds__(NT, kMinB)
   const int kb = 1 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
   if (kb >= ke) return;  // whole block
-  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P, S,
-                   kb, ke, wait_limit) &&
+  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P,
+                   S, kb, ke, wait_limit) &&
       threadIdx.x == 0)
     atomicExch(err, 1);
 }
@@ -638,7 +640,8 @@ __global__ void __launch_bounds__(NT, kMinB)
                  : "memory");
   __syncthreads();
   if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq,
-                   (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1, kWaitLimit) &&
+                   (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1,
+                   kWaitLimit) &&
       threadIdx.x == 0)
     atomicExch(g.err, 1);
 }
@@ -678,7 +681,8 @@ cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_li
   dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
   return launch_chained(k_fx<RHS>, gr, NT, smem_bytes<RHS>(), st,
                         Maps{c->maps[cur], c->maps[2], c->maps[3]}, c->u[cur ^ 1],
-                        (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny, g.nz, g.pitch, g.plane, kc,
+                        (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny, g.nz,
+                        g.pitch, g.plane, kc,
                         c->err, wait_limit);
 }
 

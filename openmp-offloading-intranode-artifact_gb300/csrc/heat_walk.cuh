@@ -4,10 +4,8 @@
 // same code runs alone and in a batch, so a grid's results do not depend on
 // how it was launched.
 //
-// Integer-pipe evaluation of the default FP64 form (walk_int):
-// GB300's FP64 pipe retires about 2 lane-operations per clock per SM, while
-// its integer pipes retire 64 (logic, shifts, IMAD) to 128 (IADD) lane-ops
-// per clock and run concurrently with it.  walk_int evaluates the update
+// Integer evaluation of a single point of the default FP64 form (int_point), which
+// the fixed-point kernel uses for points its patches cannot hold:
 //
 //   u_new = uC + rhs + sum_f w_f (u_f - uC),   w_f = factor (kappa_a + kappa_b)
 //
@@ -33,8 +31,8 @@
 //
 // The representation needs |acc| < 2^63, which holds when every centre weight
 // 1 - sum_f w_f is >= 0 (the explicit scheme's stability condition) and each
-// factor*kappa < 1/4.  k_kq_setup checks both; contexts that fail it use the
-// FP64-pipe kernel alone.  Infinite or NaN inputs in a stencil take a
+// factor*kappa < 1/4.  k_kq_check checks both (and a little more); contexts that
+// fail it use the FP64-pipe kernel.  Infinite or NaN inputs in a stencil take a
 // per-point FP64 path.
 
 #pragma once
@@ -90,7 +88,7 @@ __device__ __forceinline__ void walk_exact_faces(double *__restrict__ un,
   }
 }
 
-// ---- default FP64 form: integer pipes and FP64 pipe ----
+// ---- default FP64 form: one point in integers ----
 struct Dec {
   int e;    // biased exponent, subnormals and zero mapped to 1
   i64 m9;   // signed significand << 9  (|m9| < 2^62)
