@@ -54,10 +54,10 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 167 GLUP/s (0.79 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 169 GLUP/s (0.786 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 148 (115.7);
-// 192^3 with a narrow Gaussian 133 at first, 123 over 200 steps.
+// the launch before this one), with the reference's source term 150 (115.7);
+// 192^3 with a narrow Gaussian 135 at first, 124 over 200 steps.
 // About 140 warp instructions per point (300 for an integer row of that
 // launch); at 320^3 the ALU pipe is 58 % busy, FMA-heavy (18 of its instructions the
 // wide multiply-adds, twice the cost of the others) the same, FP64 53 %, issue 61 %,
@@ -155,37 +155,42 @@ struct TableMaps {
   __device__ __forceinline__ const CUtensorMap *r() const { return &tm[3]; }
 };
 
-// Exponent range and signs of a set of values, from their high words.  Zeros
-// do not count in mn (t - 1 wraps to the top), nor do subnormals, which beside
-// a normal number are below 2^-60 units and read as 0; fx_tile tells a region
-// of zeros from one of subnormals.
+// Sizes and signs of a set of values, from their high words, an instruction or two
+// each (masking the exponents first cost 1 % more in all).  Zeros do not count
+// in mn (it wraps to the top); subnormals count as too small to be held, and
+// beside a normal number are below 2^-60 units and read as 0.  fx_tile tells a
+// region of zeros from one of subnormals.
 struct Range {
-  unsigned mx = 0, mn = ~0u, sg = 0;
-  __device__ __forceinline__ void see(u64 v) {
-    const unsigned hi = (unsigned)(v >> 32), t = hi & kExpMask;
-    mx = max(mx, t);
-    mn = min(mn, t - 1);
-    sg |= hi;
-  }
-  // A value that only has to be below the scale.
+  unsigned neg = 0;  // largest size of a negative value, its sign bit set
+  int pos = 0;       // largest size of another one
+  unsigned mn = ~0u; // smallest nonzero size, twice, less 2
   __device__ __forceinline__ void bound(u64 v) {
     const unsigned hi = (unsigned)(v >> 32);
-    mx = max(mx, hi & kExpMask);
-    sg |= hi;
+    neg = max(neg, hi);
+    pos = max(pos, (int)hi);
+  }
+  __device__ __forceinline__ void see(u64 v) {
+    bound(v);
+    mn = min(mn, (unsigned)(v >> 32) * 2u - 2u);
   }
   __device__ __forceinline__ void see(const Range &o) {
-    mx = max(mx, o.mx);
+    neg = max(neg, o.neg);
+    pos = max(pos, o.pos);
     mn = min(mn, o.mn);
-    sg |= o.sg;
+  }
+  __device__ __forceinline__ bool negative() const { return (int)neg < 0; }
+  __device__ __forceinline__ unsigned size() const {
+    return negative() ? max((unsigned)pos, neg & 0x7fffffffu) : (unsigned)pos;
   }
   // Scale (exponent field) of the region.
   __device__ __forceinline__ unsigned scale() const {
-    const unsigned up = (int)sg < 0 ? 2 * kExp : kExp;
-    return max((mx + up) & ~(2 * kExp - 1), kLowE);
+    const unsigned up = negative() ? 2 * kExp : kExp;
+    return max((size() + up) & ~(2 * kExp - 1), kLowE);
   }
+  __device__ __forceinline__ bool zero() const { return size() < kExp; }
   // Whether the scale holds every value seen exactly.
   __device__ __forceinline__ bool held(unsigned E) const {
-    return E - min(mn, E) <= kSlack + 1 && E <= kHighE && mx != 0;
+    return 2 * E - min(mn, 2 * E) <= 2 * kSlack + 2 && E <= kHighE && !zero();
   }
 };
 
@@ -284,7 +289,7 @@ __device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *r
     vr = __ldcg(rhs);
     r.bound(vr);
   }
-  const unsigned E = r.mx + ((int)r.sg < 0 ? kExp : 0u);
+  const unsigned E = (r.size() & kExpMask) + (r.negative() ? kExp : 0u);
   if (E - kLowE <= kHighE - kLowE) {
     auto load = [&](u64 v) { return with_sign(magnitude(v, E), v); };
     const u64 A = load(c);
@@ -475,7 +480,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     const unsigned En = r.scale();
     const bool held = r.held(En);
     int least = 0;  // high word of the smallest result (its size), in units
-    if (r.mx != 0 && En <= kHighE) {
+    if (!r.zero() && En <= kHighE) {
       if (E != En) {
         if (E != 0 && held) {
           const int d = (int)(En - E) >> 20;
@@ -555,7 +560,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           }
         }
       };
-      if ((int)r.sg >= 0 && E <= kMidE)
+      if (!r.negative() && E <= kMidE)
         patch(Bool<true>{});
       else
         patch(Bool<false>{});
