@@ -54,11 +54,11 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 169 GLUP/s (0.786 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 173 GLUP/s (0.766 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 150 (115.7);
-// 192^3 with a narrow Gaussian 135 at first, 124 over 200 steps.
-// About 140 warp instructions per point (300 for an integer row of that
+// the launch before this one), with the reference's source term 154 (115.7);
+// 192^3 with a narrow Gaussian 136 at first, 126 over 200 steps.
+// About 135 warp instructions per point (300 for an integer row of that
 // launch); at 320^3 the ALU pipe is 58 % busy, FMA-heavy (18 of its instructions the
 // wide multiply-adds, twice the cost of the others) the same, FP64 53 %, issue 61 %,
 // DRAM 24.6 bytes a point.
@@ -190,7 +190,7 @@ struct Range {
   __device__ __forceinline__ bool zero() const { return size() < kExp; }
   // Whether the scale holds every value seen exactly.
   __device__ __forceinline__ bool held(unsigned E) const {
-    return 2 * E - min(mn, 2 * E) <= 2 * kSlack + 2 && E <= kHighE && !zero();
+    return mn >= 2 * (E - kSlack) - 2 && E <= kHighE && !zero();
   }
 };
 
@@ -212,11 +212,14 @@ __device__ __forceinline__ u64 shl(u64 a, unsigned n) {
 
 // |v| in units of 2^(E - 1083): the significand left-aligned, its leading bit
 // or-ed in, shifted right by 3 + E - e (over 63, so to 0, where the exponent
-// field is 0).
+// field is 0).  The bits below the exponent do not matter to that difference once
+// it is rounded up, so only a sign is masked.
+template <bool SIGN>
 __device__ __forceinline__ u64 magnitude(u64 v, unsigned E) {
-  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v, t = hi & kExpMask;
+  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
   const unsigned h = __funnelshift_l(lo, hi, 11) | 0x80000000u;
-  return shr(((u64)h << 32) | (lo << 11), (E + 3 * kExp - t) >> 20);
+  return shr(((u64)h << 32) | (lo << 11),
+             (E + (4 * kExp - 1) - (SIGN ? hi & 0x7fffffffu : hi)) >> 20);
 }
 // The same of a value that is not negative, for E <= kMidE, by the FP64 pipe:
 // the scale goes into the exponent field (0 stays below 1/2 unit) and the
@@ -262,7 +265,7 @@ struct Acc {
   }
   // += v to the nearest unit
   __device__ __forceinline__ void add(u64 v, unsigned E) {
-    const u64 h = magnitude(v, E - kExp);  // in half units
+    const u64 h = magnitude<true>(v, E - kExp);  // in half units
     H += with_sign((h >> 1) + (h & 1), v);
   }
 };
@@ -291,7 +294,7 @@ __device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *r
   }
   const unsigned E = (r.size() & kExpMask) + (r.negative() ? kExp : 0u);
   if (E - kLowE <= kHighE - kLowE) {
-    auto load = [&](u64 v) { return with_sign(magnitude(v, E), v); };
+    auto load = [&](u64 v) { return with_sign(magnitude<true>(v, E), v); };
     const u64 A = load(c);
     Acc a(A);
 #pragma unroll
@@ -416,8 +419,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     E = r.scale();  // at most the first plane's scale, so what that needs exact is exact
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      A1[q] = with_sign(magnitude(b[q], E), b[q]);
-      Dd[q] = with_sign(magnitude(a[q], E), a[q]) - A1[q];
+      A1[q] = with_sign(magnitude<true>(b[q], E), b[q]);
+      Dd[q] = with_sign(magnitude<true>(a[q], E), a[q]) - A1[q];
     }
     if (!r.held(E)) {
       E = 0;
@@ -496,8 +499,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             u64 a = (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E));
             if (E == 0) a = q & 1 ? sm.below[q >> 1][t].y : sm.below[q >> 1][t].x;
             const u64 b = sk.u[o + (q >> 1) * BX + (q & 1)];
-            A1[q] = with_sign(magnitude(b, En), b);
-            Dd[q] = with_sign(magnitude(a, En), a) - A1[q];
+            A1[q] = with_sign(magnitude<true>(b, En), b);
+            Dd[q] = with_sign(magnitude<true>(a, En), a) - A1[q];
           }
         }
         E = En;
@@ -512,7 +515,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
         // compiler forms them one after the other (512^3: 870 to 960 us a step for
         // 788).
         auto load = [&](u64 v) {
-          const u64 m = magnitude(v, E);
+          const u64 m = magnitude<!plain.value>(v, E);
           return plain.value ? m : with_sign(m, v);
         };
         reload();
@@ -548,7 +551,12 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             W1[q] = (unsigned)(kc[x] >> 32) + (unsigned)(ku[x] >> 32);
             a[x].face(A2[q] - A1[q], W0[q], W1[q]);
             Dd[q] = A1[q] - A2[q];
-            if constexpr (RHS) a[x].add(rr[q], E);
+            if constexpr (RHS) {
+              if (plain.value)
+                a[x].H += convert(rr[q], E);
+              else
+                a[x].add(rr[q], E);
+            }
           }
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
@@ -556,7 +564,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             const double v = a[x].rounded();
             const int h = (int)(a[x].H >> 32);
             least = min(least, (plain.value ? h : h ^ (h >> 31)) | skip[q]);
-            out[q] = scaled(v, E);
+            // (0 comes out wrong, but is below kLeast, and formed again.)
+            out[q] = __hiloint2double(__double2hiint(v) + (int)(E - kMidE), __double2loint(v));
           }
         }
       };
