@@ -212,15 +212,15 @@ FX_TRAFFIC_RECORD = ROOT / "profiles" / "fp64_fx_traffic.json"
 
 
 def fx_pipe_record(n, launch_ms, peak_gops):
-    """The default form's FP64-pipe work beside the HBM roofline: two conversions
-    between FP64 and 64-bit integers per point; everything else is on the
+    """The default form's FP64-pipe work beside the HBM roofline: conversions between
+    FP64 and 64-bit integers, seven for four points; everything else is on the
     integer pipes."""
-    ops = (n - 2) ** 3 * 2
+    ops = (n - 2) ** 3 * 7 / 4
     achieved = ops / (launch_ms * 1e-3) / 1e9
     return {"achieved_gops": round(achieved, 1), "peak_gops": round(peak_gops, 1),
             "frac": round(achieved / peak_gops, 4) if peak_gops > 0 else None,
             "ops_per_launch": ops,
-            "note": "2 conversions per point, the rest on the integer pipes; peak = measured FP64 FMA "
+            "note": "7 conversions for 4 points, the rest on the integer pipes; peak = measured FP64 FMA "
                     "rate of this GPU (heat_diag_fp64_rate, eight independent chains per thread)"}
 
 

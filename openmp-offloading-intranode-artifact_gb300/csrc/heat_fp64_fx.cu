@@ -54,17 +54,17 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 173 GLUP/s (0.766 ms a step; 133.5 for
+// Bound: the integer pipes.  At 512^3: 174 GLUP/s (0.763 ms a step; 133.5 for
 // rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 154 (115.7);
+// the launch before this one), with the reference's source term 161 (115.7);
 // 192^3 with a narrow Gaussian 136 at first, 126 over 200 steps.
 // About 135 warp instructions per point (300 for an integer row of that
 // launch); at 320^3 the ALU pipe is 58 % busy, FMA-heavy (18 of its instructions the
 // wide multiply-adds, twice the cost of the others) the same, FP64 53 %, issue 61 %,
 // DRAM 24.6 bytes a point.
-// Measured and not kept (512^3, GLUP/s): the neighbours above and below converted
-// by the FP64 pipe as the patch's own are, 157 for 167 (that pipe is then at 75 %
-// and the others wait for it); no value converted by it 164; five blocks per SM
+// Measured and not kept (512^3, GLUP/s): the neighbours of one
+// row converted by the FP64 pipe as the patch's own are, 169 for 173 (157 for 167 of
+// both); no value converted by it 164 for 167; five blocks per SM
 // at 96 registers 162; 32 x 32 tiles 156; 64 x 8 166; the plane loop unrolled by
 // 2 162.
 //
@@ -532,7 +532,9 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           const u64 ku[2] = {kU.x, kU.y}, vo[2] = {vO.x, vO.y};
           const int q0 = 2 * y;
           A2[q0] = plain.value ? convert(vU.x, E) : load(vU.x);
-          A2[q0 + 1] = plain.value ? convert(vU.y, E) : load(vU.y);
+          // (the fourth on the integer pipes: with the source term 823 us a step at 512^3,
+          // 862 with all four converted, 819 with two; without 763, 766, 771)
+          A2[q0 + 1] = plain.value && y == 0 ? convert(vU.y, E) : load(vU.y);
           Acc a[2] = {Acc(A1[q0]), Acc(A1[q0 + 1])};
 #pragma unroll
           for (int x = 0; x < 2; ++x) a[x].face(Dd[q0 + x], W0[q0 + x], W1[q0 + x]);
