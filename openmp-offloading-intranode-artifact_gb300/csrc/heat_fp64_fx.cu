@@ -49,7 +49,7 @@
 // patch is outside the slack; of 16 x 8-point patches 40 % would be.)
 //
 // Staging: a block is 32 x 16 columns (128 threads, 16 x 8 patches).  Planes of
-// u and K (and the source term) land by TMA in a ring 4 deep (3), boxes 36 x 18
+// u and K (and the source term) land by TMA in a ring 3 deep, boxes 36 x 18
 // from column i0 - 2 (16-byte aligned), each slot completing on its own
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
@@ -91,10 +91,9 @@ constexpr int TX = 32, TY = 16;          // columns of a tile
 constexpr int NTX = TX / 2, NTY = TY / 2;
 constexpr int NT = NTX * NTY;            // threads, one per 2 x 2 patch
 constexpr int BX = TX + 4, BY = TY + 2;  // box: columns i0 - 2 .. i0 + 33, rows j0 - 1 .. j0 + 16
-// Ring depth: planes k, k + 1 and two in flight; one with a source term, whose
-// slots are larger (four blocks of 4 would not fit an SM).
-template <bool RHS>
-constexpr int kRing = RHS ? 3 : 4;
+// Ring depth: planes k, k + 1 and one in flight (a fourth slot: 512^3 763 us a step
+// for 762, 256^3 99.7 for 99.0).
+constexpr int kRing = 3;
 constexpr int kMaxPlanes = 32;  // of a chunk: a bit each in `again`
 constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills
 
@@ -128,12 +127,12 @@ static_assert(sizeof(Slot<false>) % 128 == 0 && sizeof(Slot<true>) % 128 == 0 &&
 
 template <bool RHS>
 struct Smem {
-  Slot<RHS> ring[kRing<RHS>];
+  Slot<RHS> ring[kRing];
   // Each thread's patch at the plane below where its registers do not hold it;
   // after the walk, the list of patches to form again.
   ulonglong2 below[2][NT];
   int count;
-  u64 bar[kRing<RHS>];
+  u64 bar[kRing];
 };
 
 // Where a tile finds its tensor maps: kernel parameters for a single grid,
@@ -367,7 +366,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   const bool active = y0 && (x0 || x1);  // the patch holds a point to write
 
   if (t == 0) {
-    for (int s = 0; s < kRing<RHS>; ++s) tma::mbar_init(&sm.bar[s]);
+    for (int s = 0; s < kRing; ++s) tma::mbar_init(&sm.bar[s]);
     tma::mbar_init_fence();
   }
   chain();
@@ -382,7 +381,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     tma::load3(sl.k, maps.k(), tx * TX - 2, ty * TY, p, b);
     if constexpr (RHS) tma::load3(sl.r, maps.r(), tx * TX, ty * TY + 1, p, b);
   };
-  for (int s = 0; s < kRing<RHS>; ++s) issue(kb - 1 + s, s);
+  for (int s = 0; s < kRing; ++s) issue(kb - 1 + s, s);
 
   // Carried along z, points in the order (i, j), (i + 1, j), (i, j + 1),
   // (i + 1, j + 1): the patch at plane k (A1) and its difference to plane k - 1
@@ -440,12 +439,12 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   unsigned again = 0;  // bit p: the patch at plane kb + p is to be formed point by point
   int k = kb;
   for (; k < ke; ++k, w += S) {
-    const int s2 = s1 == kRing<RHS> - 1 ? 0 : s1 + 1;
+    const int s2 = s1 == kRing - 1 ? 0 : s1 + 1;
     if (s2 == 0) parity ^= 1;
     if (!failed) failed = !tma::mbar_wait(&sm.bar[s2], parity, wait_limit);
     failed = __syncthreads_or(failed);
     if (failed) break;
-    issue(k - 1 + kRing<RHS>, s0);  // every thread is done with plane k - 1
+    issue(k - 1 + kRing, s0);  // every thread is done with plane k - 1
     const Slot<RHS> &sk = sm.ring[s1], &sn = sm.ring[s2];
 
     s0 = s1;
@@ -608,10 +607,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     r0 = r1;
     r1 = r2;
   }
-  // Planes k - 1 and on were requested up to plane k + kRing<RHS> - 2.
+  // Planes k - 1 and on were requested up to plane k + kRing - 2.
   if (failed && t == 0)
-    for (int p = k - 1; p <= min(k + kRing<RHS> - 2, ke); ++p)
-      tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing<RHS>], (p - kb + 1) / kRing<RHS> & 1u);
+    for (int p = k - 1; p <= min(k + kRing - 2, ke); ++p)
+      tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing], (p - kb + 1) / kRing & 1u);
   // Marked and formed after the walk: inside it, inlined or called, it costs the
   // loop its schedule (512^3: 808 to 930 us a step for 788).
   if (__syncthreads_or(again != 0 && !failed))
