@@ -183,10 +183,7 @@ int heat_tune_batch(int precision, unsigned flags, int max_nz, int force);
 /* z-chunk the batch kernel will use for a grid of depth nz.                   */
 int heat_tune_lookup(int precision, unsigned flags, int nz, int *kchunk);
 
-/* The autotuner's choices for a grid of depth nz of this form, or the defaults
- * where its class is not tuned: the batch then cuts TMA-staged tiles by its cost
- * model (at most kchunk planes for HEAT_FP64) and takes two FP32C steps per
- * launch where the form has them.                                            */
+/* Every choice the batch makes for a grid of depth nz of this form.         */
 typedef struct heat_tune_entry {
   int kchunk;          /* planes per tile's z-walk                          */
   int rows;            /* rows per thread: tiles of 32 x (8 * rows) columns  */

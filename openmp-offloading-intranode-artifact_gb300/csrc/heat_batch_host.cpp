@@ -14,18 +14,12 @@
 // depth class (heat_tune.cpp).
 //
 // Grids large enough to fill the GPU alone (HEAT_BATCH_SOLO_POINTS interior
-// points) are stepped with their single-grid kernels instead, on a stream of their
-// own beside the table kernels; the tile table carries the small grids, which one
-// launch per grid would leave the GPU mostly idle for.  The TMA-staged kinds' tiles
-// are those of the single-grid kernels and share the GPU best in one launch (six
-// FP64 grids of 160^3: 148 GLUP/s in the table, 130 solo; two of 320^3 161 and
-// 165), so they stay in it up to 32 M points; the column walks up to 2 M (two
-// bit-exact grids of 128^3 beside small ones: 56 GLUP/s solo, 40 in the table).
-//
-// The TMA-staged kinds' tiles are cut into z-chunks by the cost model of the
-// single-grid kernels over the whole table, and FP32C grids take two steps per
-// launch unless the autotuner chose one.  12 grids of 48 to 192 points per axis,
-// microseconds a step: FP32C alone 51.7 -> 29.0, FP64 alone 76.5 -> 72.1.
+// points, default 2,000,000) are stepped with their single-grid kernels
+// instead (two FP32C steps per launch) on a stream of their own beside the table
+// kernels; the tile table carries the small grids, which one launch per grid
+// would leave the GPU mostly idle for.
+// On configuration 3 (64 grids of 48..384 points per axis) the table alone
+// measured 129 GLUP/s, with solo grids 137.
 //
 // Bookkeeping: every active context advances one step per batch step; the
 // device table records each grid's current buffer at build time and each
@@ -63,9 +57,7 @@ struct heat_batch {
   std::vector<Entry> entries;
   std::vector<int> active;  // entry indices in table order, then solo entries
   std::vector<int> solo;    // the active entries stepped alone
-  // Interior points from which a grid runs alone: of the kinds that walk columns,
-  // and of the TMA-staged ones.
-  long long solo_points[2] = {2000000, 32000000};
+  long long solo_points = 2000000;
   cudaStream_t solo_stream = nullptr;
   cudaEvent_t solo_join = nullptr;
 
@@ -259,69 +251,33 @@ int rebuild(heat_batch *b) {
   auto points = [](const heat_ctx *c) {
     return (long long)(c->g.nx - 2) * (c->g.ny - 2) * (c->g.nz - 2);
   };
-  struct Plan {
-    heat::TuneChoice ch;
-    bool tuned;
-    int form, ntx, nty;
-  };
-  // The grid's form, the autotuner's choices for its depth class, and its tiles.
-  // A class not tuned takes two FP32C steps per launch where its form has them.
-  auto plan = [&](const heat_ctx *c) {
-    Plan p;
-    p.form = heat::batch_form(c);
-    p.ch = heat::tuned_choice(p.form, c->g.nz, &p.tuned);
-    if (b->override_.kchunk > 0) p.ch.kchunk = b->override_.kchunk;
-    if (b->override_.rows > 0) p.ch.rows = b->override_.rows;
-    if (b->override_.minb > 0) p.ch.minb = b->override_.minb;
-    if (b->override_.depth > 0) p.ch.depth = b->override_.depth;
-    p.tuned |= b->override_.depth > 0;
-    if (p.form == heat::kFormF32c && (p.ch.depth == 2 || !p.tuned) && heat::two_step_form(c))
-      p.form = heat::kFormF32c2;
-    if (p.form == heat::kFormFx) {
-      p.ntx = heat::fx_tiles_x(c->g.nx);
-      p.nty = heat::fx_tiles_y(c->g.ny);
-    } else {
-      p.ch.rows = p.form == heat::kFormF32c2 ? 1 : std::max(1, std::min(p.ch.rows, 2));
-      const int tile_h = p.form == heat::kFormF32c2 ? heat::fp32c_tile_rows() : 8 * p.ch.rows;
-      p.ntx = (c->g.nx - 2 + 31) / 32;
-      p.nty = (c->g.ny - 2 + tile_h - 1) / tile_h;
-    }
-    return p;
-  };
-  auto solo = [&](const Plan &p, const heat_ctx *c) {
-    const long long from = b->solo_points[p.form == heat::kFormFx || p.form == heat::kFormF32c2];
-    return from > 0 && points(c) >= from;
-  };
-  // The TMA-staged kinds' tiles: default FP64 without and with a source term,
-  // two-step FP32C.
-  std::vector<heat::Walk> walks[3];
-  auto walk_of = [](const Plan &p, const heat_ctx *c) {
-    return p.form == heat::kFormFx ? (int)grid_has_rhs(c) : p.form == heat::kFormF32c2 ? 2 : -1;
-  };
-  for (const heat_batch::Entry &en : b->entries) {
-    if (en.remaining <= 0) continue;
-    const Plan p = plan(en.ctx);
-    if (const int w = walk_of(p, en.ctx); w >= 0 && !solo(p, en.ctx))
-      walks[w].push_back({(long)p.ntx * p.nty, en.ctx->g.nz - 2});
-  }
-  const int chunk[3] = {heat::fx_table_chunk(walks[0].data(), walks[0].size(), false),
-                        heat::fx_table_chunk(walks[1].data(), walks[1].size(), true),
-                        heat::fp32c_table_chunk(walks[2].data(), walks[2].size())};
+  // Planes of default-FP64 tiles in the table, without and with a source term.
+  long fx_planes[2] = {0, 0};
+  for (const heat_batch::Entry &en : b->entries)
+    if (en.remaining > 0 && !(b->solo_points > 0 && points(en.ctx) >= b->solo_points) &&
+        heat::batch_form(en.ctx) == heat::kFormFx)
+      fx_planes[en.ctx->rhs != nullptr] += (long)heat::fx_tiles_x(en.ctx->g.nx) *
+                                           heat::fx_tiles_y(en.ctx->g.ny) * (en.ctx->g.nz - 2);
   for (size_t e = 0; e < b->entries.size(); ++e) {
     heat_batch::Entry &en = b->entries[e];
     if (en.remaining <= 0) continue;
     heat_ctx *c = en.ctx;
     en.base_steps = c->steps_done;
     en.pairs = false;
-    const Plan p = plan(c);
-    en.solo = solo(p, c);
+    en.solo = b->solo_points > 0 && points(c) >= b->solo_points;
     if (en.solo) {
       b->solo.push_back((int)e);
       continue;
     }
-    const int form = p.form;
-    const int minb =
-        std::max(heat::kMinbLo, std::min(p.ch.minb, heat::kMinbLo + heat::kNumMinb - 1));
+    int form = heat::batch_form(c);
+    // The autotuner's choices for the grid's form and depth class.
+    heat::TuneChoice ch = heat::tuned_choice(form, c->g.nz);
+    if (b->override_.kchunk > 0) ch.kchunk = b->override_.kchunk;
+    if (b->override_.rows > 0) ch.rows = b->override_.rows;
+    if (b->override_.minb > 0) ch.minb = b->override_.minb;
+    if (b->override_.depth > 0) ch.depth = b->override_.depth;
+    const int minb = std::max(heat::kMinbLo, std::min(ch.minb, heat::kMinbLo + heat::kNumMinb - 1));
+    if (form == heat::kFormF32c && ch.depth == 2 && heat::two_step_form(c)) form = heat::kFormF32c2;
     // The TMA-staged table kernels come in one variant.
     const bool one = form == heat::kFormF32c2 || form == heat::kFormFx;
     const int kind = heat::kind_of(form, grid_has_rhs(c), one ? heat::kMinbLo : minb);
@@ -329,7 +285,8 @@ int rebuild(heat_batch *b) {
     grids.push_back(describe(c, form));
     b->active.push_back((int)e);
     const int interior = c->g.nz - 2;
-    int kc = std::max(1, std::min(p.ch.kchunk, interior));
+    int kc = std::max(1, std::min(ch.kchunk, interior));
+    int rows = std::max(1, std::min(ch.rows, 2)), tile_h = 8 * rows;
     if (form == heat::kFormF32c2) {
       en.pairs = true;
       b->pairs.push_back((int)e);
@@ -337,23 +294,25 @@ int rebuild(heat_batch *b) {
       maps.resize(maps.size() + 7);
       std::copy(c->maps, c->maps + 7, maps.end() - 7);
       // the temporal blocking wants long z-walks
-      kc = p.tuned ? std::max(kc, std::min(16, interior)) : std::min(chunk[2], interior);
+      kc = std::max(kc, std::min(16, interior));
+      rows = 1;
+      tile_h = heat::fp32c_tile_rows();
     }
+    int ntx = (c->g.nx - 2 + 31) / 32, nty = (c->g.ny - 2 + tile_h - 1) / tile_h;
     if (form == heat::kFormFx) {
       map_at.push_back({gi, (int)maps.size()});
       maps.resize(maps.size() + 4);
       std::copy(c->maps, c->maps + 4, maps.end() - 4);
-      kc = std::min(kc, chunk[grid_has_rhs(c)]);
-    }
-    if (one) {  // even chunks
-      const int chunks = (interior + kc - 1) / kc;
-      kc = (interior + chunks - 1) / chunks;
+      // A small table fills the GPU with shorter tiles than the tuned ones.
+      kc = std::min(kc, heat::fx_fill_chunk(fx_planes[c->rhs != nullptr], c->rhs));
+      rows = 1;
+      ntx = heat::fx_tiles_x(c->g.nx);
+      nty = heat::fx_tiles_y(c->g.ny);
     }
     for (int k0 = 1; k0 < c->g.nz - 1; k0 += kc) {
       const int k1 = std::min(k0 + kc, c->g.nz - 1);
-      for (int ty = 0; ty < p.nty; ++ty)
-        for (int tx = 0; tx < p.ntx; ++tx)
-          per_form[kind].push_back({gi, tx, ty, k0, k1, p.ch.rows});
+      for (int ty = 0; ty < nty; ++ty)
+        for (int tx = 0; tx < ntx; ++tx) per_form[kind].push_back({gi, tx, ty, k0, k1, rows});
     }
     work[kind] += (double)(c->g.nx - 2) * (c->g.ny - 2) * interior / kFormRate[form];
   }
@@ -362,12 +321,6 @@ int rebuild(heat_batch *b) {
   double total = 0;
   b->nforms = 0;
   for (int f = 0; f < heat::kNumKinds; ++f) {
-    // Long tiles first: short ones fill the end of the launch (40 FP64 grids of 24 to 96
-    // points per axis 102 us a step, 105 in table order).
-    std::stable_sort(per_form[f].begin(), per_form[f].end(),
-                     [](const heat::BatchTile &x, const heat::BatchTile &y) {
-                       return x.k1 - x.k0 > y.k1 - y.k0;
-                     });
     b->tile_begin[f] = (int)tiles.size();
     b->tile_count[f] = (int)per_form[f].size();
     tiles.insert(tiles.end(), per_form[f].begin(), per_form[f].end());
@@ -584,8 +537,7 @@ int heat_batch_create(heat_batch **out, void *stream, unsigned flags) {
             cudaStreamCreateWithFlags(&b->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaStreamCreateWithFlags(&b->solo_stream, cudaStreamNonBlocking) == cudaSuccess &&
        cudaEventCreateWithFlags(&b->solo_join, cudaEventDisableTiming) == cudaSuccess;
-  if (const char *ev = std::getenv("HEAT_BATCH_SOLO_POINTS"))
-    b->solo_points[0] = b->solo_points[1] = std::atoll(ev);
+  if (const char *ev = std::getenv("HEAT_BATCH_SOLO_POINTS")) b->solo_points = std::atoll(ev);
   if (!ok) {
     cudaGetLastError();
     release(b);

@@ -67,11 +67,10 @@ cudaError_t launch_batch_fx(const BatchGrid *grids, const BatchTile *tiles, int 
                             int flip, cudaStream_t st);
 int fx_tiles_x(int nx);
 int fx_tiles_y(int ny);
-// Most planes per tile of a table of n grids.
-int fx_table_chunk(const Walk *w, size_t n, bool rhs);
+// Most planes per tile of a table of tile_planes planes of such tiles in all.
+int fx_fill_chunk(long tile_planes, bool rhs);
 // heat_fp32c_tma.cu: the two-step FP32C table kernel.
 int fp32c_tile_rows();
-int fp32c_table_chunk(const Walk *w, size_t n);
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,
                                    int flip, cudaStream_t st);
 
@@ -84,7 +83,7 @@ int batch_form(const heat_ctx *c);
 struct TuneChoice {
   int kchunk, rows, minb, depth;
 };
-TuneChoice tuned_choice(int form, int nz, bool *tuned = nullptr);
+TuneChoice tuned_choice(int form, int nz);
 // Default blocks-per-SM variant of a form's table kernel.
 inline int default_minb(int form) { return form == kFormFx ? 3 : 4; }
 

@@ -441,13 +441,10 @@ int fp32c_tile_rows() { return OY; }
 
 // A chunk's start costs about 4 planes' time: two planes of step t+1, their loads
 // and the halo planes.
-int fp32c_table_chunk(const Walk *w, size_t n) {
-  static const long resident = ready() ? resident_blocks((const void *)k_fp32c_tb2, NT, kSmem) : 0;
-  return balanced_chunk(w, n, resident, 4, 0.95, 128);
-}
 int fp32c_tb2_chunk(const heat_geom &g) {
-  const Walk w = {(long)((g.nx - 2 + OX - 1) / OX) * ((g.ny - 2 + OY - 1) / OY), g.nz - 2};
-  return fp32c_table_chunk(&w, 1);
+  const long tiles = (long)((g.nx - 2 + OX - 1) / OX) * ((g.ny - 2 + OY - 1) / OY);
+  static const long resident = ready() ? resident_blocks((const void *)k_fp32c_tb2, NT, kSmem) : 0;
+  return balanced_chunk(tiles, g.nz - 2, resident, 4, 0.95, 128);
 }
 
 cudaError_t launch_batch_fp32c_tb2(const BatchGrid *grids, const BatchTile *tiles, int ntiles,

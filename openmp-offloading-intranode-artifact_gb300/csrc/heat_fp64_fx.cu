@@ -710,14 +710,20 @@ cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_li
 int fx_tiles_x(int nx) { return (nx - 1 + TX - 1) / TX; }
 int fx_tiles_y(int ny) { return (ny - 2 + TY - 1) / TY; }
 
+// Short tiles until a table holds 1.7 blocks for every resident one, as a small
+// grid alone wants (64^3: 4.8 us a step at 1 plane, 6.7 at 2, 9.9 at 8); never
+// more than kMaxPlanes.
+int fx_fill_chunk(long tile_planes, bool rhs) {
+  const long n = rhs ? resident<true>() : resident<false>();
+  const long kc = n > 0 ? (3 * tile_planes + 5 * n - 1) / (5 * n) : 16;
+  return kc < 1 ? 1 : kc < kMaxPlanes ? (int)kc : kMaxPlanes;
+}
+
 // A chunk's start, its first loads, costs about a plane's time; 384^3 runs 329 us
 // a step at 20 planes, 355 at 191.
-int fx_table_chunk(const Walk *w, size_t n, bool rhs) {
-  return balanced_chunk(w, n, rhs ? resident<true>() : resident<false>(), 1, 0.53, kMaxPlanes);
-}
 int fx_chunk(const heat_geom &g, bool rhs) {
-  const Walk w = {(long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny), g.nz - 2};
-  return fx_table_chunk(&w, 1, rhs);
+  return balanced_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny), g.nz - 2,
+                        rhs ? resident<true>() : resident<false>(), 1, 0.53, kMaxPlanes);
 }
 
 bool fx_usable(bool rhs) { return rhs ? usable<true>() : usable<false>(); }

@@ -167,28 +167,25 @@ inline int wave_chunk(const heat_geom &g, int tile_x, int tile_y, long resident,
   return (int)((interior + chunks - 1) / chunks);
 }
 
-struct Walk {  // `tiles` tiles over `interior` planes
-  long tiles;
-  int interior;
-};
-// Most planes per block for a launch of the tiles of n grids whose blocks run
-// `resident` at a time: those with the least estimated time.  A round of blocks takes (planes + overhead) plane times; `alone` is a
+// Planes per block for a launch of `tiles` tiles over `interior` planes whose
+// blocks run `resident` at a time: the chunk count with the least estimated
+// time.  A round of blocks takes (planes + overhead) plane times; `alone` is a
 // plane's time with one block on an SM as a fraction of its time on a full one
 // (latency keeps it from falling with the load), between which it rises steeply
 // at first (k_fx: 0.53, 0.88, 0.94, 1 for 1 to 4 blocks).  At most `most` planes:
-// few long rounds end less evenly than this counts on.  Against the chunk that measured best of 19 it costs 2 to 8 % on
+// few long rounds end less evenly than this counts on.  Worked out once per
+// context.  Against the chunk that measured best of 19 it costs 2 to 8 % on
 // grids from 40 x 33 x 28 to 512^3.
-inline int balanced_chunk(const Walk *w, size_t n, long resident, int overhead, double alone,
+inline int balanced_chunk(long tiles, int interior, long resident, int overhead, double alone,
                           int most) {
-  int interior = 1;
-  for (size_t g = 0; g < n; ++g) interior = w[g].interior > interior ? w[g].interior : interior;
   if (resident <= 0) return interior < 32 ? interior : 32;
   const long per_sm = (resident + 151) / 152;
   double best = 0;
   int best_kc = 0;
-  for (int kc = interior < most ? interior : most; kc >= 1; --kc) {
-    long blocks = 0;
-    for (size_t g = 0; g < n; ++g) blocks += w[g].tiles * ((w[g].interior + kc - 1) / kc);
+  for (int most_kc = interior < most ? interior : most; most_kc >= 1; --most_kc) {
+    const int chunks = (interior + most_kc - 1) / most_kc;
+    const int kc = (interior + chunks - 1) / chunks;
+    const long blocks = tiles * chunks;
     const long rest = (blocks % resident + 151) / 152;  // blocks per SM in the last round
     double rounds = (double)(blocks / resident);
     if (rest)
@@ -200,11 +197,6 @@ inline int balanced_chunk(const Walk *w, size_t n, long resident, int overhead, 
     }
   }
   return best_kc;
-}
-inline int balanced_chunk(long tiles, int interior, long resident, int overhead, double alone,
-                          int most) {
-  const Walk w = {tiles, interior};
-  return balanced_chunk(&w, 1, resident, overhead, alone, most);
 }
 
 // heat_fp64_exact.cu (compiled with --fmad=false)

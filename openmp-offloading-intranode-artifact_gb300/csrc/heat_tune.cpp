@@ -171,16 +171,12 @@ double time_candidate(std::vector<heat_ctx *> &cs, heat_batch *b, const heat::Tu
 
 namespace heat {
 
-TuneChoice tuned_choice(int form, int nz, bool *tuned) {
+TuneChoice tuned_choice(int form, int nz) {
   std::lock_guard<std::mutex> lk(g_mu);
   load_locked();
   const int cls = class_of(nz);
   for (const TuneEntry &t : g_table)
-    if (t.form == form && t.nz_max == cls) {
-      if (tuned) *tuned = true;
-      return t.ch;
-    }
-  if (tuned) *tuned = false;
+    if (t.form == form && t.nz_max == cls) return t.ch;
   return default_choice(form);
 }
 
