@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <new>
 #include <vector>
 
@@ -73,11 +74,14 @@ struct heat_batch {
   long long pair_flips = 0;     // buffer swaps of those grids since the table was built
   cudaEvent_t table_ev[2] = {nullptr, nullptr};
   bool table_used[2] = {false, false};
-  // Table uploads run on their own stream (a pageable upload first waits for
-  // everything queued on its stream; this one has nothing queued), and the
-  // batch stream waits on copy_ev before the next launch.
+  // Table uploads run on their own stream and read page-locked memory of the
+  // table copy they fill, which is written again only once copy_ev, recorded
+  // behind them, has passed (an upload from pageable memory may read it after the
+  // call has returned); the batch stream waits on copy_ev before the next launch.
   cudaStream_t copy_stream = nullptr;
-  cudaEvent_t copy_ev = nullptr;
+  cudaEvent_t copy_ev[2] = {nullptr, nullptr};
+  char *stage[2] = {nullptr, nullptr};
+  size_t stage_cap[2] = {0, 0};
   int tb = 0;                          // table copy in use
   heat::BatchGrid *d_grids = nullptr;  // == g_buf[tb]
   heat::BatchTile *d_tiles = nullptr;  // == t_buf[tb]
@@ -158,8 +162,9 @@ void release(heat_batch *b) {
     cudaStreamSynchronize(b->copy_stream);
     cudaStreamDestroy(b->copy_stream);
   }
-  if (b->copy_ev) cudaEventDestroy(b->copy_ev);
   for (int i = 0; i < 2; ++i) {
+    if (b->copy_ev[i]) cudaEventDestroy(b->copy_ev[i]);
+    if (b->stage[i]) cudaFreeHost(b->stage[i]);
     if (b->g_buf[i]) cudaFree(b->g_buf[i]);
     if (b->t_buf[i]) cudaFree(b->t_buf[i]);
     if (b->m_buf[i]) cudaFree(b->m_buf[i]);
@@ -182,6 +187,37 @@ int grow(T **p, size_t *cap, size_t need) {
   *p = q;
   *cap = n;
   return HEAT_OK;
+}
+
+// Page-locked memory of table copy i for `need` bytes of uploads, its earlier ones
+// complete.
+int grow_stage(heat_batch *b, int i, size_t need) {
+  if (cudaEventSynchronize(b->copy_ev[i]) != cudaSuccess) {
+    cudaGetLastError();
+    return HEAT_ECUDA;
+  }
+  if (need <= b->stage_cap[i]) return HEAT_OK;
+  const size_t n = std::max<size_t>({need, b->stage_cap[i] * 2, 256u << 10});
+  void *q = nullptr;
+  if (cudaHostAlloc(&q, n, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    return HEAT_ENOMEM;
+  }
+  if (b->stage[i]) cudaFreeHost(b->stage[i]);
+  b->stage[i] = static_cast<char *>(q);
+  b->stage_cap[i] = n;
+  return HEAT_OK;
+}
+
+// Queue the upload of v to dst through *stage, which moves on behind it.
+template <class T>
+bool upload_table(T *dst, const std::vector<T> &v, char **stage, cudaStream_t st) {
+  if (v.empty()) return true;
+  const size_t bytes = v.size() * sizeof(T);
+  std::memcpy(*stage, v.data(), bytes);
+  const bool ok = cudaMemcpyAsync(dst, *stage, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
+  *stage += bytes;
+  return ok;
 }
 
 bool grid_has_rhs(const heat_ctx *c) {
@@ -358,19 +394,15 @@ int rebuild(heat_batch *b) {
   for (const auto &gm : map_at) grids[gm.first].tmaps = b->m_buf[nb] + gm.second;
   for (int f = 0; f < heat::kNumKinds; ++f)
     if (b->tile_count[f] && !ensure_side(b, f)) return HEAT_ECUDA;
-  if (!maps.empty() && cudaMemcpyAsync(b->m_buf[nb], maps.data(), maps.size() * sizeof(CUtensorMap),
-                                       cudaMemcpyHostToDevice, b->copy_stream) != cudaSuccess) {
-    cudaGetLastError();
-    return HEAT_ECUDA;
-  }
-  // Pageable sources: the copies are staged before the calls return.
-  if (!grids.empty() &&
-      (cudaMemcpyAsync(b->g_buf[nb], grids.data(), grids.size() * sizeof(heat::BatchGrid),
-                       cudaMemcpyHostToDevice, b->copy_stream) != cudaSuccess ||
-       cudaMemcpyAsync(b->t_buf[nb], tiles.data(), tiles.size() * sizeof(heat::BatchTile),
-                       cudaMemcpyHostToDevice, b->copy_stream) != cudaSuccess ||
-       cudaEventRecord(b->copy_ev, b->copy_stream) != cudaSuccess ||
-       cudaStreamWaitEvent(b->stream, b->copy_ev, 0) != cudaSuccess)) {
+  rc = grow_stage(b, nb, maps.size() * sizeof(CUtensorMap) + grids.size() * sizeof(heat::BatchGrid) +
+                             tiles.size() * sizeof(heat::BatchTile));
+  if (rc != HEAT_OK) return rc;
+  char *stage = b->stage[nb];
+  if (!upload_table(b->m_buf[nb], maps, &stage, b->copy_stream) ||
+      !upload_table(b->g_buf[nb], grids, &stage, b->copy_stream) ||
+      !upload_table(b->t_buf[nb], tiles, &stage, b->copy_stream) ||
+      cudaEventRecord(b->copy_ev[nb], b->copy_stream) != cudaSuccess ||
+      cudaStreamWaitEvent(b->stream, b->copy_ev[nb], 0) != cudaSuccess) {
     cudaGetLastError();
     return HEAT_ECUDA;
   }
@@ -533,7 +565,8 @@ int heat_batch_create(heat_batch **out, void *stream, unsigned flags) {
   bool ok = cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&b->table_ev[0], cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&b->table_ev[1], cudaEventDisableTiming) == cudaSuccess &&
-            cudaEventCreateWithFlags(&b->copy_ev, cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&b->copy_ev[0], cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&b->copy_ev[1], cudaEventDisableTiming) == cudaSuccess &&
             cudaStreamCreateWithFlags(&b->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaStreamCreateWithFlags(&b->solo_stream, cudaStreamNonBlocking) == cudaSuccess &&
        cudaEventCreateWithFlags(&b->solo_join, cudaEventDisableTiming) == cudaSuccess;
