@@ -407,11 +407,8 @@ __global__ void __launch_bounds__(NT, 2)
   const BatchGrid &g = grids[tl.grid];
   const int src = g.cur ^ flip, dst = src ^ 1;
   const CUtensorMap *tm = static_cast<const CUtensorMap *>(g.tmaps);
-  // The maps were written by a host copy before the launch; order the tensor
-  // proxy's reads of them after it.
   if (threadIdx.x == 0)  // the thread that issues the loads
-    for (int m = 0; m < 7; ++m)
-      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm + m) : "memory");
+    for (int m = 0; m < 7; ++m) tma::acquire_map(tm + m);
   __syncthreads();
   tb2_tile(TableMaps{tm, src}, (float *)g.f[dst], g.cr[dst], 1 + OX * tl.tx, 1 + OY * tl.ty, g.nx,
            g.ny, g.nz, g.P, g.S, tl.k0, tl.k1, g.err, kWaitLimit);

@@ -648,13 +648,10 @@ __global__ void __launch_bounds__(NT, kMinB)
   const BatchGrid &g = grids[tl.grid];
   const int src = g.cur ^ flip, dst = src ^ 1;
   const CUtensorMap *tm = static_cast<const CUtensorMap *>(g.tmaps);
-  // The maps were written by a host copy before the launch; order the tensor
-  // proxy's reads of them after it.
   // By the thread that issues the loads, for each map: a fence orders its own
   // thread's accesses.
   if (threadIdx.x == 0)
-    for (int m = 0; m < 4; ++m)
-      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm + m) : "memory");
+    for (int m = 0; m < 4; ++m) tma::acquire_map(tm + m);
   __syncthreads();
   if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq,
                    (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1,

@@ -72,6 +72,13 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Orders this thread's use of a tensor map in device memory after the copy that
+// wrote it.  At system scope: the writer is a host copy, not a kernel of this GPU,
+// and the same memory holds other maps from one table to the next.
+__device__ __forceinline__ void acquire_map(const CUtensorMap *map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 // 3-D box load of `map` at element coordinates (x, y, z) into dst; the box's
 // x origin times the element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void load3(void *dst, const CUtensorMap *map, int x, int y, int z,

@@ -4,6 +4,7 @@ from page-locked memory that the batch owns and does not touch meanwhile."""
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 
 import pytest
@@ -26,3 +27,11 @@ def test_table_uploads_read_memory_the_batch_keeps(program):
     env = {**os.environ, "ASAN_OPTIONS": "detect_leaks=0"}
     r = subprocess.run([str(program)], capture_output=True, text=True, env=env)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_tensor_maps_are_acquired_at_system_scope():
+    """The table kernels' tensor maps are written by host copies into memory that held
+    other maps before: an acquire at GPU scope does not order their use after that."""
+    scopes = [(f.name, scope) for f in sorted((PKG / "csrc").iterdir()) if f.suffix in (".cu", ".cuh")
+              for scope in re.findall(r"fence\.proxy\.tensormap::generic\.acquire\.(\w+)", f.read_text())]
+    assert scopes and all(scope == "sys" for _, scope in scopes), scopes
