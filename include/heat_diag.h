@@ -30,7 +30,7 @@ int heat_diag_field_diff(struct heat_ctx *a, struct heat_ctx *b, double *max_abs
                          double *rel_l2);
 
 /* Bounded-wait check.  One block waits, with the same bounded mbarrier wait
- * the TMA kernels use (each attempt a try_wait of up to ~2 us), capped at
+ * the TMA kernels use (each attempt a try_wait of about 4 us), capped at
  * `attempts` tries (1 .. 2^22, the kernels' own limit; HEAT_EINVAL otherwise),
  * on an mbarrier that nothing arrives at.  The wait must give
  * up: *timed_out = 1 and the call returns HEAT_ETIMEOUT, the status a TMA

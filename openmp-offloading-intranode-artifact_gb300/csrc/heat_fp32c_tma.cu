@@ -101,6 +101,8 @@ struct Maps {
 // __grid_constant__ parameters, or seven maps per grid in device memory for
 // the batch table (buffer `src` of v and carry, then wx, wy, wz).
 struct ParamMaps {
+  static constexpr bool kInMemory = false;
+  static constexpr unsigned kLimit = kWaitLimit;
   const Maps &in;
   __device__ __forceinline__ const CUtensorMap *v() const { return &in.v; }
   __device__ __forceinline__ const CUtensorMap *c() const { return &in.c; }
@@ -109,6 +111,8 @@ struct ParamMaps {
   __device__ __forceinline__ const CUtensorMap *wz() const { return &in.wz; }
 };
 struct TableMaps {
+  static constexpr bool kInMemory = true;
+  static constexpr unsigned kLimit = kTableWaitLimit;
   const CUtensorMap *tm;
   int src;
   __device__ __forceinline__ const CUtensorMap *v() const { return &tm[src]; }
@@ -197,7 +201,6 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     tma::mbar_init_fence();
   }
   chain();
-  __syncthreads();
 
   // Every warp waits on the mbarriers itself (warp 0 alone, handing the planes
   // on through the block barrier: 319 GLUP/s for 335 at 384^3); thread 0 issues
@@ -230,7 +233,22 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     pending &= ~(1u << s);
   };
 
-  for (int p = kb - 2; p <= kb + 1; ++p) issue(p);
+  // The flag is read before the first loads where a wrong map could be what set it,
+  // else behind them, where their own time hides it.
+  bool stop = M::kInMemory && tid == 0 && tma::gave_up(err);
+  if (!stop)
+    for (int p = kb - 2; p <= kb + 1; ++p) issue(p);
+  if (!M::kInMemory) stop = tid == 0 && tma::gave_up(err);
+  // Before the block's shared memory goes its own loads in flight must have landed
+  // (each wait bounded).
+  auto drain = [&] {
+    for (int s = 0; s < R; ++s)
+      if (pending & (1u << s)) mbar_wait(&sm.bar[s], (phase >> s) & 1u, M::kLimit);
+  };
+  if (__syncthreads_or(stop)) {
+    if (!M::kInMemory && tid == 0) drain();
+    return;
+  }
 
   // This thread's step-(t+1) points: columns gx, gx + 1 (gx even) of row gy,
   // pair lp and row ly of the (17 x 22) region, and their shared-memory offsets.
@@ -378,11 +396,7 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
   }
   if (failed) {
     if (tid == 0) atomicExch(err, 1);
-    // Let the block's own loads in flight land before its shared memory goes
-    // (each wait bounded).
-    if (tid == 0)
-      for (int s = 0; s < R; ++s)
-        if (pending & (1u << s)) mbar_wait(&sm.bar[s], (phase >> s) & 1u);
+    if (tid == 0) drain();
   }
 }
 
@@ -411,7 +425,7 @@ __global__ void __launch_bounds__(NT, 2)
     for (int m = 0; m < 7; ++m) tma::acquire_map(tm + m);
   __syncthreads();
   tb2_tile(TableMaps{tm, src}, (float *)g.f[dst], g.cr[dst], 1 + OX * tl.tx, 1 + OY * tl.ty, g.nx,
-           g.ny, g.nz, g.P, g.S, tl.k0, tl.k1, g.err, kWaitLimit);
+           g.ny, g.nz, g.P, g.S, tl.k0, tl.k1, g.err, kTableWaitLimit);
 }
 
 bool encode(CUtensorMap *m, const void *base, bool bf16, const heat_geom &g) {

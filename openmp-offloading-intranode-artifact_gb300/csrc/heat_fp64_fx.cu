@@ -141,12 +141,16 @@ struct Maps {
   CUtensorMap u, k, r;
 };
 struct ParamMaps {
+  static constexpr bool kInMemory = false;
+  static constexpr unsigned kLimit = kWaitLimit;
   const Maps &m;
   __device__ __forceinline__ const CUtensorMap *u() const { return &m.u; }
   __device__ __forceinline__ const CUtensorMap *k() const { return &m.k; }
   __device__ __forceinline__ const CUtensorMap *r() const { return &m.r; }
 };
 struct TableMaps {
+  static constexpr bool kInMemory = true;
+  static constexpr unsigned kLimit = kTableWaitLimit;
   const CUtensorMap *tm;
   int src;
   __device__ __forceinline__ const CUtensorMap *u() const { return &tm[src]; }
@@ -352,12 +356,14 @@ __device__ __forceinline__ ulonglong2 ld2(const u64 *p) {
 }
 
 // One step over the (32 x 16)-column tile (tx, ty), planes [kb, ke), of the
-// field u into un; at most kMaxPlanes planes.  Returns true if a wait ran out.
+// field u into un; at most kMaxPlanes planes.  Returns true if a wait ran out, here or
+// in a launch before (*err).
 template <bool RHS, class M>
 __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__restrict__ un,
                                         const u64 *__restrict__ u, const u64 *__restrict__ K,
                                         const u64 *__restrict__ rhs, int tx, int ty, int nx, int ny,
-                                        int P, size_t S, int kb, int ke, unsigned wait_limit) {
+                                        int P, size_t S, int kb, int ke, const int *err,
+                                        unsigned wait_limit) {
   const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
   const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly;  // patch: i, i + 1; j, j + 1
   const int o = (2 * ly + 1) * BX + 2 * lx + 2;              // its first point in a box
@@ -370,7 +376,6 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     tma::mbar_init_fence();
   }
   chain();
-  __syncthreads();
   auto issue = [&](int p, int s) {
     if (t != 0 || p > ke) return;
     Slot<RHS> &sl = sm.ring[s];
@@ -381,7 +386,17 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     tma::load3(sl.k, maps.k(), tx * TX - 2, ty * TY, p, b);
     if constexpr (RHS) tma::load3(sl.r, maps.r(), tx * TX, ty * TY + 1, p, b);
   };
-  for (int s = 0; s < kRing; ++s) issue(kb - 1 + s, s);
+  // The flag is read before the first loads where a wrong map could be what set it,
+  // else behind them (40 x 33 x 28: 3.49 us a step, 3.65 the other way, 3.36 unread).
+  bool stop = M::kInMemory && t == 0 && tma::gave_up(err);
+  if (!stop)
+    for (int s = 0; s < kRing; ++s) issue(kb - 1 + s, s);
+  if (!M::kInMemory) stop = t == 0 && tma::gave_up(err);
+  if (__syncthreads_or(stop)) {
+    if (!M::kInMemory && t == 0)
+      for (int s = 0; s < kRing && kb - 1 + s <= ke; ++s) tma::mbar_wait(&sm.bar[s], 0, M::kLimit);
+    return true;
+  }
 
   // Carried along z, points in the order (i, j), (i + 1, j), (i, j + 1),
   // (i + 1, j + 1): the patch at plane k (A1) and its difference to plane k - 1
@@ -610,7 +625,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   // Planes k - 1 and on were requested up to plane k + kRing - 2.
   if (failed && t == 0)
     for (int p = k - 1; p <= min(k + kRing - 2, ke); ++p)
-      tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing], (p - kb + 1) / kRing & 1u);
+      tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing], (p - kb + 1) / kRing & 1u, M::kLimit);
   // Marked and formed after the walk: inside it, inlined or called, it costs the
   // loop its schedule (512^3: 808 to 930 us a step for 788).
   if (__syncthreads_or(again != 0 && !failed))
@@ -634,7 +649,7 @@ __global__ void __launch_bounds__(NT, kMinB)
   const int ke = min(kb + kchunk, nz - 1);
   if (kb >= ke) return;  // whole block
   if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P,
-                   S, kb, ke, wait_limit) &&
+                   S, kb, ke, err, wait_limit) &&
       threadIdx.x == 0)
     atomicExch(err, 1);
 }
@@ -655,7 +670,7 @@ __global__ void __launch_bounds__(NT, kMinB)
   __syncthreads();
   if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq,
                    (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1,
-                   kWaitLimit) &&
+                   g.err, kTableWaitLimit) &&
       threadIdx.x == 0)
     atomicExch(g.err, 1);
 }

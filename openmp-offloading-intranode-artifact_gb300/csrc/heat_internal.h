@@ -116,9 +116,13 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
 constexpr int kNormBlocks = 152 * 4;   // partial-sum blocks of the norm pass
 
 // Bound of every device-side mbarrier wait in the TMA kernels (try_wait
-// attempts, each suspending up to ~2 us); a wait that runs out sets the
-// context's error flag and the launch returns with its outputs unwritten.
+// attempts of about 4 us); a wait that runs out sets the context's error flag and
+// the launch returns with its outputs unwritten.  Blocks that start with the flag
+// set leave at once, so all that is queued behind a failure ends within a wait.
 constexpr unsigned kWaitLimit = 1u << 22;
+// The same in the table kernels: 65 ms.  Their loads go by tensor maps in device
+// memory, and a wrong one is a load that never completes.
+constexpr unsigned kTableWaitLimit = 1u << 14;
 
 // Planes per block for a launch of (tile_x x tile_y)-column tiles over the
 // grid's interior: enough z-chunks that tiles x chunks reaches `want` blocks

@@ -66,6 +66,14 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
   return false;
 }
 
+// Whether a launch before this one set the flag `err`; read past L1, whose lines
+// outlive a launch.
+__device__ __forceinline__ bool gave_up(const int *err) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(err) : "memory");
+  return v != 0;
+}
+
 // Orders this thread's earlier generic-proxy accesses of shared memory before
 // the async-proxy (TMA) writes that follow.
 __device__ __forceinline__ void fence_proxy_async() {
