@@ -655,8 +655,9 @@ int batch_run(heat_batch *b, long long max_steps, long long *steps_taken, bool s
       cudaGetLastError();
       return HEAT_ECUDA;
     }
-  for (int e : b->active)
-    if (b->entries[e].ctx->steps_done != b->entries[e].base_steps + b->since_build) b->dirty = true;
+  if (!b->dirty)  // (else `active` may name entries that are gone)
+    for (int e : b->active)
+      if (b->entries[e].ctx->steps_done != b->entries[e].base_steps + b->since_build) b->dirty = true;
   for (;;) {
     if (b->dirty) {
       rc = rebuild(b);

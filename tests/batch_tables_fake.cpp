@@ -150,6 +150,11 @@ int main() {
     heat_ctx *c = contexts[q % 8];
     if (q % 3 == 2 && heat_batch_remove(b, c) == HEAT_OK) heat_batch_add(b, c, 4);
     if (q == 5) heat_batch_add(b, context(11), 9);
+    if (q == 7 || q == 9) {  // one leaves with steps left, and goes
+      heat_batch_remove(b, contexts.back());
+      delete contexts.back();
+      contexts.pop_back();
+    }
   }
   heat_batch_run(b, -1, nullptr);
   heat_batch_destroy(b);

@@ -16,7 +16,7 @@ from conftest import PKG, ROOT
 def program(tmp_path_factory):
     import heat_build
     exe = tmp_path_factory.mktemp("batch") / "batch_tables"
-    subprocess.run(["g++", "-g", "-O1", "-std=c++17", "-fsanitize=address", "-I", str(ROOT / "include"),
+    subprocess.run(["g++", "-g", "-O1", "-std=c++17", "-fsanitize=address", "-D_GLIBCXX_ASSERTIONS", "-I", str(ROOT / "include"),
                     "-I", str(PKG / "csrc"), "-I", str(heat_build._cuda_include(heat_build._nvcc())),
                     str(ROOT / "tests" / "batch_tables_fake.cpp"), str(PKG / "csrc" / "heat_batch_host.cpp"),
                     "-o", str(exe)], check=True)
