@@ -74,6 +74,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "heat_batch_internal.h"
@@ -644,8 +645,8 @@ template <bool RHS>
 __global__ void __launch_bounds__(NT, kMinB)
     k_fx(const __grid_constant__ Maps maps, double *__restrict__ un, const u64 *__restrict__ u,
          const u64 *__restrict__ K, const u64 *__restrict__ rhs, int nx, int ny, int nz, int P,
-         size_t S, int kchunk, int *__restrict__ err, unsigned wait_limit) {
-  const int kb = 1 + blockIdx.z * kchunk;
+         size_t S, int k0, int kchunk, int *__restrict__ err, unsigned wait_limit) {
+  const int kb = k0 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
   if (kb >= ke) return;  // whole block
   if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P,
@@ -707,12 +708,16 @@ template <bool RHS>
 cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_limit) {
   const heat_geom &g = c->g;
   const int kc = c->kchunk;
-  dim3 gr(fx_tiles_x(g.nx), fx_tiles_y(g.ny), (g.nz - 2 + kc - 1) / kc);
-  return launch_chained(k_fx<RHS>, gr, NT, smem_bytes<RHS>(), st,
-                        Maps{c->maps[cur], c->maps[2], c->maps[3]}, c->u[cur ^ 1],
-                        (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny, g.nz,
-                        g.pitch, g.plane, kc,
-                        c->err, wait_limit);
+  // A chunk has at most kMaxPlanes planes and a launch kMaxGridZ chunks: past 2 M
+  // planes a step takes several launches.
+  cudaError_t e = cudaSuccess;
+  for (int k0 = 1, left = (g.nz - 2 + kc - 1) / kc; left > 0 && e == cudaSuccess;
+       left -= kMaxGridZ, k0 += kMaxGridZ * kc)
+    e = launch_chained(k_fx<RHS>, dim3(fx_tiles_x(g.nx), fx_tiles_y(g.ny), std::min(left, kMaxGridZ)),
+                       NT, smem_bytes<RHS>(), st, Maps{c->maps[cur], c->maps[2], c->maps[3]},
+                       c->u[cur ^ 1], (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny,
+                       g.nz, g.pitch, g.plane, k0, kc, c->err, wait_limit);
+  return e;
 }
 
 }  // namespace
@@ -734,7 +739,8 @@ int fx_fill_chunk(long tile_planes, bool rhs) {
 // A chunk's start, its first loads, costs about a plane's time; 384^3 runs 329 us
 // a step at 20 planes, 355 at 191.
 int fx_chunk(const heat_geom &g, bool rhs) {
-  return balanced_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny), g.nz - 2,
+  return balanced_chunk((long)fx_tiles_x(g.nx) * fx_tiles_y(g.ny),
+                        std::min(g.nz - 2, kMaxGridZ * kMaxPlanes),
                         rhs ? resident<true>() : resident<false>(), 1, 0.53, kMaxPlanes);
 }
 

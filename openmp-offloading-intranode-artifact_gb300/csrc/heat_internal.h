@@ -177,16 +177,19 @@ inline int wave_chunk(const heat_geom &g, int tile_x, int tile_y, long resident,
 // plane's time with one block on an SM as a fraction of its time on a full one
 // (latency keeps it from falling with the load), between which it rises steeply
 // at first (k_fx: 0.53, 0.88, 0.94, 1 for 1 to 4 blocks).  At most `most` planes:
-// few long rounds end less evenly than this counts on.  Worked out once per
-// context.  Against the chunk that measured best of 19 it costs 2 to 8 % on
+// few long rounds end less evenly than this counts on; more only where a launch
+// could not have that many chunks.  Against the chunk that measured best of 19 it costs 2 to 8 % on
 // grids from 40 x 33 x 28 to 512^3.
+constexpr int kMaxGridZ = 65535;  // most blocks along z of a launch
 inline int balanced_chunk(long tiles, int interior, long resident, int overhead, double alone,
                           int most) {
-  if (resident <= 0) return interior < 32 ? interior : 32;
+  const int least = (interior + kMaxGridZ - 1) / kMaxGridZ;
+  if (most < least) most = least;
+  if (resident <= 0) return interior < most ? interior : most;
   const long per_sm = (resident + 151) / 152;
   double best = 0;
   int best_kc = 0;
-  for (int most_kc = interior < most ? interior : most; most_kc >= 1; --most_kc) {
+  for (int most_kc = interior < most ? interior : most; most_kc >= least; --most_kc) {
     const int chunks = (interior + most_kc - 1) / most_kc;
     const int kc = (interior + chunks - 1) / chunks;
     const long blocks = tiles * chunks;
