@@ -72,6 +72,7 @@
 // next barrier (the flag is OR-reduced), thread 0 waits (bounded) for its loads
 // in flight, *err is set and the host reports HEAT_ETIMEOUT.
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
@@ -101,6 +102,7 @@ constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills
 constexpr unsigned kExp = 1u << 20;      // one binary order in the high word of a double
 constexpr unsigned kExpMask = 0x7ff00000u;
 constexpr unsigned kSlack = 8 * kExp;
+constexpr unsigned kUnheld = 1;  // of a patch's scale: does not hold its plane before exactly
 constexpr int kLeast = 1 << (53 - 32);  // high word of 2^53
 constexpr unsigned kLowE = 128 * kExp, kMidE = 1083 * kExp, kHighE = 2030 * kExp;
 
@@ -225,9 +227,8 @@ __device__ __forceinline__ u64 magnitude(u64 v, unsigned E) {
   return shr(((u64)h << 32) | (lo << 11),
              (E + (4 * kExp - 1) - (SIGN ? hi & 0x7fffffffu : hi)) >> 20);
 }
-// The same of a value that is not negative, for E <= kMidE, by the FP64 pipe:
-// the scale goes into the exponent field (0 stays below 1/2 unit) and the
-// conversion does the rest.
+// A value, with its sign, for E <= kMidE, by the FP64 pipe: the scale goes into the
+// exponent field (0 stays below 1/2 unit) and the conversion does the rest.
 __device__ __forceinline__ u64 convert(u64 v, unsigned E) {
   return (u64)__double2ll_rn(
       __hiloint2double((int)((unsigned)(v >> 32) + (kMidE - E)), (int)(unsigned)v));
@@ -235,6 +236,12 @@ __device__ __forceinline__ u64 convert(u64 v, unsigned E) {
 __device__ __forceinline__ u64 with_sign(u64 a, u64 v) {
   const u64 s = (u64)((i64)v >> 63);
   return (a ^ s) - s;
+}
+
+// A value of point q of a patch, as the patch form rounds it where the scale does not
+// hold it.
+__device__ __forceinline__ u64 carried(u64 v, int q, unsigned E) {
+  return q == 3 || E > kMidE ? with_sign(magnitude<true>(v, E), v) : convert(v, E);
 }
 
 // r units of 2^(E - 1083).
@@ -246,6 +253,15 @@ __device__ __forceinline__ double scaled(double r, unsigned E) {
 template <bool B>
 struct Bool {
   static constexpr bool value = B;
+};
+
+// Kinds of patch code: for values that are not negative, for any sign, and for scales
+// above kMidE.  The first two round every value alike, so a patch of the first kind has
+// the same bits in either.
+constexpr int kPlain = 0, kSigned = 1, kAnyScale = 2;
+template <int K>
+struct Kind {
+  static constexpr int value = K;
 };
 
 struct Acc {
@@ -401,7 +417,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
 
   // Carried along z, points in the order (i, j), (i + 1, j), (i, j + 1),
   // (i + 1, j + 1): the patch at plane k (A1) and its difference to plane k - 1
-  // (Dd) at scale E (0: not held), the weight limbs of the face below and the
+  // (Dd) at scale E (0: none yet), the weight limbs of the face below and the
   // ranges.
   u64 Dd[4], A1[4];
   unsigned W0[4], W1[4];
@@ -438,7 +454,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
       Dd[q] = with_sign(magnitude<true>(a[q], E), a[q]) - A1[q];
     }
     if (!r.held(E)) {
-      E = 0;
+      E = kUnheld;
       sm.below[0][t] = make_ulonglong2(a[0], a[1]);
       sm.below[1][t] = make_ulonglong2(a[2], a[3]);
     }
@@ -499,8 +515,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     const bool held = r.held(En);
     int least = 0;  // high word of the smallest result (its size), in units
     if (!r.zero() && En <= kHighE) {
-      if (E != En) {
-        if (E != 0 && held) {
+      if ((E & ~kUnheld) != En) {
+        if (!(E & kUnheld) && held) {
           const int d = (int)(En - E) >> 20;
           const unsigned dn = (unsigned)max(d, 0), ups = (unsigned)max(-d, 0);
 #pragma unroll
@@ -512,26 +528,27 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             u64 a = (u64)__double_as_longlong(scaled(__ll2double_rn((i64)(A1[q] + Dd[q])), E));
-            if (E == 0) a = q & 1 ? sm.below[q >> 1][t].y : sm.below[q >> 1][t].x;
+            if (E & kUnheld) a = q & 1 ? sm.below[q >> 1][t].y : sm.below[q >> 1][t].x;
             const u64 b = sk.u[o + (q >> 1) * BX + (q & 1)];
-            A1[q] = with_sign(magnitude<true>(b, En), b);
-            Dd[q] = with_sign(magnitude<true>(a, En), a) - A1[q];
+            A1[q] = carried(b, q, En);
+            Dd[q] = carried(a, q, En) - A1[q];
           }
         }
-        E = En;
       }
+      E = En;
       // The values are read from shared memory again here, row by row, rather
       // than kept in registers from the range pass.
       u64 A2[4];
       least = 0x7fffffff;
       double out[4];
-      auto patch = [&](auto plain) {
+      auto patch = [&](auto kind) {
         // One straight line, no branch in it: with one between the points the
         // compiler forms them one after the other (512^3: 870 to 960 us a step for
         // 788).
+        constexpr bool plain = kind.value == kPlain;
         auto load = [&](u64 v) {
-          const u64 m = magnitude<!plain.value>(v, E);
-          return plain.value ? m : with_sign(m, v);
+          const u64 m = magnitude<!plain>(v, E);
+          return plain ? m : with_sign(m, v);
         };
         reload();
 #pragma unroll
@@ -546,10 +563,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           const u64 kc[2] = {kC.x, kC.y}, ki[2] = {kI.x, kI.y}, ko[2] = {kO.x, kO.y};
           const u64 ku[2] = {kU.x, kU.y}, vo[2] = {vO.x, vO.y};
           const int q0 = 2 * y;
-          A2[q0] = plain.value ? convert(vU.x, E) : load(vU.x);
+          A2[q0] = kind.value != kAnyScale ? convert(vU.x, E) : load(vU.x);
           // (the fourth on the integer pipes: with the source term 823 us a step at 512^3,
           // 862 with all four converted, 819 with two; without 763, 766, 771)
-          A2[q0 + 1] = plain.value && y == 0 ? convert(vU.y, E) : load(vU.y);
+          A2[q0 + 1] = kind.value != kAnyScale && y == 0 ? convert(vU.y, E) : load(vU.y);
           Acc a[2] = {Acc(A1[q0]), Acc(A1[q0 + 1])};
 #pragma unroll
           for (int x = 0; x < 2; ++x) a[x].face(Dd[q0 + x], W0[q0 + x], W1[q0 + x]);
@@ -569,7 +586,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             a[x].face(A2[q] - A1[q], W0[q], W1[q]);
             Dd[q] = A1[q] - A2[q];
             if constexpr (RHS) {
-              if (plain.value)
+              if (kind.value != kAnyScale)
                 a[x].H += convert(rr[q], E);
               else
                 a[x].add(rr[q], E);
@@ -580,16 +597,21 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
             const int q = q0 + x;
             const double v = a[x].rounded();
             const int h = (int)(a[x].H >> 32);
-            least = min(least, (plain.value ? h : h ^ (h >> 31)) | skip[q]);
+            least = min(least, (plain ? h : h ^ (h >> 31)) | skip[q]);
             // (0 comes out wrong, but is below kLeast, and formed again.)
             out[q] = __hiloint2double(__double2hiint(v) + (int)(E - kMidE), __double2loint(v));
           }
         }
       };
-      if (!r.negative() && E <= kMidE)
-        patch(Bool<true>{});
+      // One negative value and the lanes that are together take the code for any sign:
+      // apart they cost both (random signs at 256^3, once smooth: 191 us a step without
+      // the points formed again, 147 so).
+      if (E > kMidE)
+        patch(Kind<kAnyScale>{});
+      else if (cooperative_groups::coalesced_threads().any(r.negative()))
+        patch(Kind<kSigned>{});
       else
-        patch(Bool<false>{});
+        patch(Kind<kPlain>{});
 #pragma unroll
       for (int q = 0; q < 4; ++q) A1[q] = A2[q];
 #pragma unroll
@@ -611,10 +633,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
         W0[q] = (unsigned)Kc + (unsigned)Ku;
         W1[q] = (unsigned)(Kc >> 32) + (unsigned)(Ku >> 32);
       }
-      // Zeros all around (of either sign; E = 0: the patch below is in shared memory)
+      // Zeros all around (of either sign; the patch below, not held, is in shared memory)
       // give zeros, without a mark: a body that is cold but for a spot is mostly this
       // (256^3 of zeros: 81 us a step, 540 with every point formed again).
-      if (E == 0 && r.zero()) {
+      if ((E & kUnheld) && r.zero()) {
         u64 any = 0;
         auto with = [&](const ulonglong2 &v) { any |= v.x | v.y; };
 #pragma unroll
@@ -637,9 +659,10 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
           }
         }
       }
+      E = 0;
     }
     if (!held) {
-      E = 0;
+      E |= kUnheld;
       sm.below[0][t] = ld2(&sk.u[o]);
       sm.below[1][t] = ld2(&sk.u[o + BX]);
     }
