@@ -36,11 +36,12 @@
 // FP64 multiply-adds has seven roundings, and rounded weights besides.  A
 // constant region stays exactly constant (every D is 0).
 //
-// Points formed on their own (results too small for their patch's units,
-// exponents near either end, infinities, NaNs) are aligned to the largest
-// exponent of their own seven values.  Which way a point goes, and E, depend only
-// on the field's values in the patch's region, never on tiles or z-chunks, so a
-// grid's results are the same bits in any launch.
+// Points formed on their own (results too small for their patch's units, patches without
+// a scale: exponents near either end, infinities, NaNs) are aligned to the largest
+// exponent of their own seven values.  Which way a point goes, and E, depend only on the
+// field's values in the patch's region, never on tiles or z-chunks, so a grid's results
+// are the same bits in any launch.  They are formed after the walk, from a list of
+// patches or, where those are more than half of some planes, in a second walk.
 //
 // The integers carried along z move to a new scale by shifting, which is exact
 // where both scales hold the patch exactly; elsewhere they are taken from the
@@ -81,7 +82,6 @@
 #include "heat_batch_internal.h"
 #include "heat_internal.h"
 #include "heat_tma.cuh"
-#include "heat_walk.cuh"
 
 namespace heat {
 namespace {
@@ -134,7 +134,8 @@ struct Smem {
   // Each thread's patch at the plane below where its registers do not hold it;
   // after the walk, the list of patches to form again.
   ulonglong2 below[2][NT];
-  int count;
+  int count;        // of marked patches
+  unsigned planes;  // that have some, a bit each
   u64 bar[kRing];
 };
 
@@ -227,6 +228,12 @@ __device__ __forceinline__ u64 magnitude(u64 v, unsigned E) {
   return shr(((u64)h << 32) | (lo << 11),
              (E + (4 * kExp - 1) - (SIGN ? hi & 0x7fffffffu : hi)) >> 20);
 }
+// The same of any value, subnormal ones exactly too.
+__device__ __forceinline__ u64 magnitude_low(u64 v, unsigned E) {
+  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v, e = hi >> 20 & 0x7ff;
+  const unsigned h = (__funnelshift_l(lo, hi, 11) & 0x7fffffffu) | (e ? 0x80000000u : 0u);
+  return shr(((u64)h << 32) | (lo << 11), (E >> 20) + 3 - max(e, 1u));
+}
 // A value, with its sign, for E <= kMidE, by the FP64 pipe: the scale goes into the
 // exponent field (0 stays below 1/2 unit) and the conversion does the rest.
 __device__ __forceinline__ u64 convert(u64 v, unsigned E) {
@@ -290,47 +297,103 @@ struct Acc {
   }
 };
 
-// One point from global memory (u, K and the source term at it): the same
-// arithmetic at the point's own scale, the largest exponent of its seven values
-// (and the source term), every value cut to that scale's units; exponents near
-// either end, infinities and NaNs take walk::int_point.
+// A point's values and weights (f and k: above, below, west, east, south, north) and
+// source term.
+struct Stencil {
+  u64 c, f[6], kc, k[6], vr;
+};
+// A point in FP64 operations.
 template <bool RHS>
-__device__ __forceinline__ double point(const u64 *u, const u64 *K, const u64 *rhs, int P,
-                                        size_t S) {
-  const u64 c = __ldcg(u);
-  const u64 f[6] = {__ldcg(u + S), __ldcg(u - S), __ldcg(u - 1),
-                    __ldcg(u + 1), __ldcg(u - P), __ldcg(u + P)};
-  const u64 kc = __ldcg(K);
-  const u64 k[6] = {__ldcg(K + S), __ldcg(K - S), __ldcg(K - 1),
-                    __ldcg(K + 1), __ldcg(K - P), __ldcg(K + P)};
+__device__ __forceinline__ double fp64_point(const Stencil &s) {
+  const double uc = __longlong_as_double((i64)s.c);
+  double acc = RHS ? uc + __longlong_as_double((i64)s.vr) : uc;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const int w0 = (int)((unsigned)s.kc + (unsigned)s.k[q]);
+    const i64 w1 = (unsigned)(s.kc >> 32) + (unsigned)(s.k[q] >> 32);
+    acc = fma((double)(w1 * (1ll << 31) + w0) * 0x1p-63, __longlong_as_double((i64)s.f[q]) - uc, acc);
+  }
+  return acc;
+}
+template <bool RHS>
+__device__ __forceinline__ Range range(const Stencil &s) {
   Range r;
-  r.bound(c);
+  r.bound(s.c);
 #pragma unroll
-  for (int q = 0; q < 6; ++q) r.bound(f[q]);
-  u64 vr = 0;
-  if constexpr (RHS) {
-    vr = __ldcg(rhs);
-    r.bound(vr);
-  }
-  const unsigned E = (r.size() & kExpMask) + (r.negative() ? kExp : 0u);
-  if (E - kLowE <= kHighE - kLowE) {
-    auto load = [&](u64 v) { return with_sign(magnitude<true>(v, E), v); };
-    const u64 A = load(c);
-    Acc a(A);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) a.face(load(f[q]) - A, kc, k[q]);
-    if constexpr (RHS) a.add(vr, E);
-    return scaled(a.rounded(), E);
-  }
-  if (((c | f[0] | f[1] | f[2] | f[3] | f[4] | f[5] | vr) << 1) == 0) return 0.0;
-  auto w = [](u64 x) {  // K in units of 2^-64, as int_point takes it
-    return (x & 0xffffffff00000000ull) + 2ull * (u64)(i64)(int)(unsigned)x;
+  for (int q = 0; q < 6; ++q) r.bound(s.f[q]);
+  if constexpr (RHS) r.bound(s.vr);
+  return r;
+}
+__device__ __forceinline__ unsigned own_scale(const Range &r) {
+  return (r.size() & kExpMask) + (r.negative() ? kExp : 0u);
+}
+// A point at scale E, a whole exponent.  LOW: for scales below kLowE too, where values
+// and the result may be subnormal.
+template <bool RHS, bool SIGN, bool LOW>
+__device__ __forceinline__ double at_scale(const Stencil &s, unsigned E) {
+  auto load = [&](u64 v) {
+    const u64 m = LOW ? magnitude_low(v, E) : magnitude<SIGN>(v, E);
+    return SIGN ? with_sign(m, v) : m;
   };
-  return walk::int_point<RHS>(walk::decode(c), walk::decode(f[0]), walk::decode(f[1]),
-                              walk::decode(f[3]), walk::decode(f[2]), walk::decode(f[5]),
-                              walk::decode(f[4]), w(kc), w(k[0]), w(k[1]), w(k[3]), w(k[2]),
-                              w(k[5]), w(k[4]), vr,
-                              [=] { return walk::Raw7{c, f[3], f[2], f[5], f[4], f[0], f[1]}; });
+  const u64 A = load(s.c);
+  Acc a(A);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) a.face(load(s.f[q]) - A, s.kc, s.k[q]);
+  if constexpr (RHS) {
+    if (LOW) {
+      const u64 h = magnitude_low(s.vr, E - kExp);
+      a.H += with_sign((h >> 1) + (h & 1), s.vr);
+    } else {
+      a.add(s.vr, E);
+    }
+  }
+  const bool up = LOW && E < kLowE;
+  const double r = scaled(a.rounded(), up ? E + 200 * kExp : E);
+  return up ? r * 0x1p-200 : r;
+}
+
+// One point with values of 2^1007 and more, by way of a power of two; infinities and
+// NaNs in FP64 operations.
+template <bool RHS>
+__device__ __forceinline__ double high_point(Stencil &s) {
+  if (range<RHS>(s).size() >= kExpMask) return fp64_point<RHS>(s);
+  auto times = [](u64 &v) { v = (u64)__double_as_longlong(__longlong_as_double((i64)v) * 0x1p-200); };
+  times(s.c);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) times(s.f[q]);
+  if constexpr (RHS) times(s.vr);
+  return at_scale<RHS, true, false>(s, own_scale(range<RHS>(s))) * 0x1p200;
+}
+
+// N points from their values and weights, in one straight line: the same arithmetic at
+// each point's own scale, the largest exponent of its seven values (and the source
+// term), every value cut to that scale's units.
+template <bool RHS, int N>
+__device__ __forceinline__ void points(Stencil (&s)[N], double (&out)[N]) {
+  unsigned E[N];
+  bool neg = false, low = false, high = false;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const Range r = range<RHS>(s[n]);
+    E[n] = max(own_scale(r), 2 * kExp);
+    neg |= r.negative();
+    low |= E[n] < kLowE;
+    high |= E[n] > kHighE;
+  }
+  auto all = [&](auto sign, auto subnormal) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) out[n] = at_scale<RHS, sign.value, subnormal.value>(s[n], E[n]);
+  };
+  if (low)
+    all(Bool<true>{}, Bool<true>{});
+  else if (neg)
+    all(Bool<true>{}, Bool<false>{});
+  else
+    all(Bool<false>{}, Bool<false>{});
+  if (high)
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if (E[n] > kHighE) out[n] = high_point<RHS>(s[n]);
 }
 
 // The points of the marked patches (bit p of a thread's `again`: plane kb + p),
@@ -360,16 +423,103 @@ __device__ __noinline__ void form_alone(unsigned again, unsigned short *list, in
       const int j = 1 + ty * TY + 2 * (t / NTX) + (me >> 1 & 1);
       if (i < 1 || i >= nx - 1 || j >= ny - 1) continue;
       const size_t g = (size_t)k * S + (size_t)j * P + i;
-      un[g] = point<RHS>(u + g, K + g, RHS ? rhs + g : nullptr, P, S);
+      const u64 *v = u + g, *kv = K + g;
+      Stencil st[1] = {{__ldcg(v),
+                        {__ldcg(v + S), __ldcg(v - S), __ldcg(v - 1), __ldcg(v + 1), __ldcg(v - P),
+                         __ldcg(v + P)},
+                        __ldcg(kv),
+                        {__ldcg(kv + S), __ldcg(kv - S), __ldcg(kv - 1), __ldcg(kv + 1),
+                         __ldcg(kv - P), __ldcg(kv + P)},
+                        RHS ? __ldcg(rhs + g) : 0}};
+      double out[1];
+      points<RHS>(st, out);
+      un[g] = out[0];
     }
   }
+}
+
+__device__ __forceinline__ ulonglong2 ld2(const u64 *p) {
+  return *reinterpret_cast<const ulonglong2 *>(p);
 }
 
 // Keeps the compiler from holding values read before this point in registers.
 __device__ __forceinline__ void reload() { asm volatile("" ::: "memory"); }
 
-__device__ __forceinline__ ulonglong2 ld2(const u64 *p) {
-  return *reinterpret_cast<const ulonglong2 *>(p);
+// The marked patches in a second walk, over the planes from kb + first to kb + last: the
+// same points from the ring, whose n loads of the first walk give the parities.  Returns
+// true if a wait ran out.  Bound: integer instructions, 220 a point.  256^3 where every
+// patch has values 2^40 apart: 274 us a step, 584 from the list; a hot cube in zeros,
+// steps 20 to 220, 249 for 390.  Forming such patches inside the first walk costs that
+// its schedule (512^3: 804 to 850 us a step for 770).
+template <bool RHS, class M>
+__device__ __noinline__ bool form_walk(const M maps, Smem<RHS> &sm, unsigned again, int n,
+                                       double *un, int tx, int ty, int nx, int ny, int P, size_t S,
+                                       int kb, int first, int last, unsigned wait_limit) {
+  const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
+  const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly, o = (2 * ly + 1) * BX + 2 * lx + 2;
+  const bool x0 = i >= 1 && i < nx - 1, x1 = i + 1 < nx - 1;
+  const bool y0 = j < ny - 1, y1 = j + 1 < ny - 1;
+  const int k0 = kb + first, ke = kb + last + 1, planes = ke - k0 + 2;
+  auto issue = [&](int p) {  // plane k0 - 1 + p
+    if (t != 0 || p >= planes) return;
+    Slot<RHS> &sl = sm.ring[p % kRing];
+    u64 *b = &sm.bar[p % kRing];
+    tma::fence_proxy_async();
+    tma::mbar_expect(b, kSlotBytes<RHS>);
+    tma::load3(sl.u, maps.u(), tx * TX - 2, ty * TY, k0 - 1 + p, b);
+    tma::load3(sl.k, maps.k(), tx * TX - 2, ty * TY, k0 - 1 + p, b);
+    if constexpr (RHS) tma::load3(sl.r, maps.r(), tx * TX, ty * TY + 1, k0 - 1 + p, b);
+  };
+  auto wait = [&](int p, unsigned limit) {
+    const int s = p % kRing;
+    return tma::mbar_wait(&sm.bar[s], ((n - s + kRing - 1) / kRing + p / kRing) & 1u, limit);
+  };
+  for (int p = 0; p < kRing; ++p) issue(p);
+  bool failed = !wait(0, wait_limit) || !wait(1, wait_limit);
+  u64 lo[4], kl[4];  // the patch below and its weights
+  auto below = [&](const Slot<RHS> &s) {
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const ulonglong2 v = ld2(&s.u[o + y * BX]), k = ld2(&s.k[o + y * BX]);
+      lo[2 * y] = v.x, lo[2 * y + 1] = v.y, kl[2 * y] = k.x, kl[2 * y + 1] = k.y;
+    }
+  };
+  below(sm.ring[0]);
+  double *w = un + (size_t)k0 * S + (size_t)j * P + i;
+  int p = 1;  // of plane k
+  for (int k = k0; k < ke; ++k, ++p, w += S) {
+    if (!failed) failed = !wait(p + 1, wait_limit);
+    failed = __syncthreads_or(failed);
+    if (failed) break;
+    issue(p - 1 + kRing);
+    const Slot<RHS> &sk = sm.ring[p % kRing], &sn = sm.ring[(p + 1) % kRing];
+    if (again >> (k - kb) & 1u) {
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        if (!(y ? y1 : y0)) continue;
+        Stencil st[2];
+        double out[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int c = o + y * BX + x, q = 2 * y + x;
+          st[x] = {sk.u[c],
+                   {sn.u[c], lo[q], sk.u[c - 1], sk.u[c + 1], sk.u[c - BX], sk.u[c + BX]},
+                   sk.k[c],
+                   {sn.k[c], kl[q], sk.k[c - 1], sk.k[c + 1], sk.k[c - BX], sk.k[c + BX]},
+                   0};
+          if constexpr (RHS) st[x].vr = sk.r[(2 * ly + y) * TX + 2 * lx + x];
+        }
+        points<RHS>(st, out);
+        if (x0) w[y ? P : 0] = out[0];
+        if (x1) w[(y ? P : 0) + 1] = out[1];
+      }
+    }
+    below(sk);
+  }
+  // Planes p - 1 and on were requested up to p + kRing - 2.
+  if (failed && t == 0)
+    for (int q = p - 1; q <= min(p + kRing - 2, planes - 1); ++q) wait(q, M::kLimit);
+  return failed;
 }
 
 // One step over the (32 x 16)-column tile (tx, ty), planes [kb, ke), of the
@@ -676,11 +826,25 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
   if (failed && t == 0)
     for (int p = k - 1; p <= min(k + kRing - 2, ke); ++p)
       tma::mbar_wait(&sm.bar[(p - kb + 1) % kRing], (p - kb + 1) / kRing & 1u, M::kLimit);
-  // Marked and formed after the walk: inside it, inlined or called, it costs the
-  // loop its schedule (512^3: 808 to 930 us a step for 788).
-  if (__syncthreads_or(again != 0 && !failed))
-    form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs,
-                    tx, ty, kb, nx, ny, P, S);
+  // Formed after the walk: inside it, inlined or called, it costs the loop its schedule
+  // (512^3: 808 to 930 us a step for 788).  A plane of the second walk takes about as
+  // long as half its patches from the list (104 x 107 x 63 with a narrow Gaussian 13.8 us
+  // a step; 15.4 with the line at a quarter).
+  if (!__syncthreads_or(again != 0 && !failed)) return failed;
+  if (t == 0) sm.count = 0, sm.planes = 0;
+  __syncthreads();
+  const unsigned some = __reduce_or_sync(~0u, again), many = __reduce_add_sync(~0u, __popc(again));
+  if (t % 32 == 0) {
+    atomicAdd(&sm.count, (int)many);
+    atomicOr(&sm.planes, some);
+  }
+  __syncthreads();
+  const int first = __ffs(sm.planes) - 1, last = 31 - __clz(sm.planes);
+  if (2 * sm.count > NT * (last - first + 1))
+    return form_walk<RHS>(maps, sm, again, ke - kb + 2, un, tx, ty, nx, ny, P, S, kb, first, last,
+                          wait_limit);
+  form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs, tx,
+                  ty, kb, nx, ny, P, S);
   return failed;
 }
 

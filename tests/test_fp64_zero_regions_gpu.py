@@ -79,3 +79,41 @@ def test_zero_regions_run_at_speed(heat, cuda_device):
                 best = min(best, a.elapsed_time(b))
             times.append(best)
     assert times[1] <= 2 * times[0], times
+
+
+def test_points_formed_from_the_list_and_in_the_second_walk_agree(heat, cuda_device):
+    """A block forms its marked patches from a list where they are few and in a second
+    walk where they are many: the same plane of values, once in a grid of few and once in
+    one of many, gives the same bits."""
+    H = heat
+    nx, ny, nz = 34, 18, 40
+    kappa, u0, h, dt = H.inputs_config(0, 41, nx, ny, nz)
+    rng = np.random.default_rng(2)
+    steep = u0 * np.exp2(rng.integers(-60, 1, u0.shape))
+    few = u0.copy()
+    few[16:23] = steep[16:23]
+    results = []
+    for u in (few, steep):
+        u = u.copy()
+        with H.Solver(kappa, u, h, dt) as s:
+            s.step(3)
+            results.append(s.field()[19])  # depends on planes 16 to 22 alone
+    assert np.array_equal(results[0].view(np.uint64), results[1].view(np.uint64))
+
+
+def test_huge_and_tiny_neighbours(heat, oracle, cuda_device):
+    """Points beyond both ends of the patch form's exponents, subnormal ones and ones of
+    2^1007 and more among them: a few units of the last place of the largest of the seven
+    values, or of the smallest number there is."""
+    H = heat
+    nx, ny, nz = 37, 21, 26
+    kappa, u0, h, dt = H.inputs_config(0, 43, nx, ny, nz)
+    rng = np.random.default_rng(8)
+    for low, high in ((-1074, -900), (900, 1020), (-1074, 1020)):
+        u = u0 * np.ldexp(1.0, rng.integers(low, high, u0.shape)) * rng.choice([-1.0, 1.0], u0.shape)
+        with H.Solver(kappa, u, h, dt) as s:
+            s.step(1)
+            got = s.field()
+        ref = oracle.steps(u, kappa, h, dt, 1)
+        assert np.all(np.isfinite(ref))
+        assert np.all(np.abs(got - ref) <= 5 * 2.0 ** -52 * local_max(u, 1) + 8 * 5e-324)
