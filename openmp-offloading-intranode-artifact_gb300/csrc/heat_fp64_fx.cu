@@ -21,7 +21,7 @@
 //     kSlack = 8 binary orders below E, those A are exact, and are carried along
 //     z.  Other values are cut to whole units, an error of one unit times the
 //     weight.  A result below 2^53 units, where a unit is more than 1/2 ulp, is
-//     formed anew on its own.
+//     formed anew on its own (2^51 where the region has both signs).
 //   * Weights come from the per-point K = factor * kappa, kept as two limbs
 //     K = k1 2^-32 + k0 2^-63 with |k0| <= 2^30: a face weight is the two limb
 //     sums, no carry, and its low limb is a signed 32-bit number.
@@ -112,7 +112,8 @@ constexpr unsigned kExp = 1u << 20;      // one binary order in the high word of
 constexpr unsigned kExpMask = 0x7ff00000u;
 constexpr unsigned kSlack = 8 * kExp;
 constexpr unsigned kUnheld = 1;  // of a patch's scale: does not hold its plane before exactly
-constexpr int kLeast = 1 << (53 - 32);  // high word of 2^53
+constexpr int kLeast = 1 << (53 - 32);          // high word of 2^53
+constexpr int kLeastCrossing = 1 << (51 - 32);  // of 2^51
 constexpr unsigned kLowE = 128 * kExp, kMidE = 1083 * kExp, kHighE = 2030 * kExp;
 
 // Element count of `rows` box rows padded to 128 bytes: each array of a slot
@@ -195,6 +196,7 @@ struct Range {
     mn = min(mn, o.mn);
   }
   __device__ __forceinline__ bool negative() const { return (int)neg < 0; }
+  __device__ __forceinline__ bool crossing() const { return (int)neg < 0 && pos >= (int)kExp; }
   __device__ __forceinline__ unsigned size() const {
     return negative() ? max((unsigned)pos, neg & 0x7fffffffu) : (unsigned)pos;
   }
@@ -672,6 +674,12 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     }
     const unsigned En = r.scale();
     const bool held = r.held(En);
+    // Results of fewer units than this are formed on their own.  Where the field changes
+    // sign a small result is mostly the difference of large terms, to which rounded
+    // FP64 operations add more than the fixed point does, and fewer are (random signs at
+    // 256^3: 164 us a step at first and 200 later with 2^53, 135 and 168 so; 512^3
+    // without signs 812, 820 so).
+    const int enough = r.crossing() ? kLeastCrossing : kLeast;
     int least = 0;  // high word of the smallest result (its size), in units
     if (!r.zero() && En <= kHighE) {
       if ((E & ~kUnheld) != En) {
@@ -827,7 +835,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     }
     // No scale, or a result too small for its units (zeros in the patch, small
     // neighbours).
-    if (least < kLeast) again |= 1u << (k - kb);
+    if (least < enough) again |= 1u << (k - kb);
     r0 = r1;
     r1 = r2;
   }
