@@ -226,7 +226,7 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
   const heat_geom &g = c->g;
   const size_t bytes = g.elems * sizeof(double);
   int rc = HEAT_OK;
-  double *kap = nullptr;  // raw kappa on the device (kept only for the naive kernel)
+  double *kap = nullptr;  // raw kappa on the device (kept for the naive kernel and the default form)
   SideStream side;
   bool split = false;
   cudaStream_t ust = c->stream;  // stream of the u0 upload
@@ -297,6 +297,9 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
         cudaFreeAsync(c->kq, c->stream);
         c->kq = nullptr;
         fixed = false;
+      } else {
+        c->kappa = kap;
+        kap = nullptr;
       }
     }
     if (!fixed) {

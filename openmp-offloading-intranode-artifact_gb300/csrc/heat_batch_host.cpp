@@ -253,6 +253,7 @@ heat::BatchGrid describe(const heat_ctx *c, int form) {
       for (int a = 0; a < 3; ++a) g.w[a + 1] = c->cf[a];
     } else {
       g.kq = c->kq;
+      g.w[0] = c->kappa;
     }
   }
   return g;

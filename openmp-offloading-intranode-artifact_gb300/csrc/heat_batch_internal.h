@@ -29,7 +29,7 @@ struct BatchGrid {
   void *f[2];
   uint16_t *cr[2];
   const void *rhs;
-  const void *w[4];  // Hw: c0, cx, cy, cz   Exact: kx, ky, kz   F32c: wx, wy, wz
+  const void *w[4];  // Hw: c0, cx, cy, cz   Exact: kx, ky, kz   F32c: wx, wy, wz   Fx: kappa
   const unsigned long long *kq;  // Fx
   int *err;            // the context's error flag (bounded waits that ran out)
   const void *tmaps;   // CUtensorMaps in device memory: Fx four (u0 u1 K rhs), F32c2 seven

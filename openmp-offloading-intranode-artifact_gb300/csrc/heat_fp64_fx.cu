@@ -376,17 +376,44 @@ __device__ __forceinline__ double high_point(Stencil &s) {
   return at_scale<RHS, true, false>(s, own_scale(range<RHS>(s))) * 0x1p200;
 }
 
-// N points from their values and weights, in one straight line: the same arithmetic at
-// each point's own scale, the largest exponent of its seven values (and the source
-// term), every value cut to that scale's units.
+// The conductivities themselves, for results that live on small weights.
+struct Kappa {
+  const double *k;  // the grid's
+  double factor;
+  int P;
+  size_t S;
+};
+// A point, at offset g, of values that are all of one sign (so that nothing cancels) and
+// weights below 2^-20, of which K has 43 bits and fewer: in FP64 operations of the
+// conductivities.  (Insulators of 1e-9 among conductors, cold at first: largest relative
+// error after 10 steps 6.5e-9 without, 1.5e-9 so; 5.5e-9 for the launch before the fixed
+// point.  A hot cube in zeros at 256^3 255 us a step without, 275 so.)
+template <bool RHS>
+__device__ __forceinline__ double weak_point(const Stencil &s, const Kappa &kap, size_t g) {
+  const double *k = kap.k + g;
+  const size_t S = kap.S;
+  const int P = kap.P;
+  const double kf[6] = {__ldcg(k + S), __ldcg(k - S), __ldcg(k - 1),
+                        __ldcg(k + 1), __ldcg(k - P), __ldcg(k + P)};
+  const double kc = __ldcg(k), uc = __longlong_as_double((i64)s.c);
+  double sum = 0.0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) sum = fma(kc + kf[q], __longlong_as_double((i64)s.f[q]) - uc, sum);
+  return fma(kap.factor, sum, RHS ? uc + __longlong_as_double((i64)s.vr) : uc);
+}
+// N points, at offsets g, from their values and weights, in one straight line: the same
+// arithmetic at each point's own scale, the largest exponent of its seven values (and the
+// source term), every value cut to that scale's units.
 template <bool RHS, int N>
-__device__ __forceinline__ void points(Stencil (&s)[N], double (&out)[N]) {
+__device__ __forceinline__ void points(Stencil (&s)[N], const Kappa &kap, const size_t (&g)[N],
+                                       double (&out)[N]) {
   unsigned E[N];
-  bool neg = false, low = false, high = false;
+  bool neg = false, low = false, high = false, one_sign[N];
 #pragma unroll
   for (int n = 0; n < N; ++n) {
     const Range r = range<RHS>(s[n]);
     E[n] = max(own_scale(r), 2 * kExp);
+    one_sign[n] = !r.crossing() && E[n] <= kHighE;
     neg |= r.negative();
     low |= E[n] < kLowE;
     high |= E[n] > kHighE;
@@ -405,6 +432,15 @@ __device__ __forceinline__ void points(Stencil (&s)[N], double (&out)[N]) {
 #pragma unroll
     for (int n = 0; n < N; ++n)
       if (E[n] > kHighE) out[n] = high_point<RHS>(s[n]);
+  // A result of fewer than 2^46 units by such weights alone.
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+    if (((unsigned)__double2hiint(out[n]) & 0x7fffffffu) + 14 * kExp < E[n] && one_sign[n]) {
+      unsigned top = 0;  // the largest weight's high limb, units of 2^-32
+#pragma unroll
+      for (int q = 0; q < 6; ++q) top = max(top, (unsigned)(s[n].k[q] >> 32));
+      if (top + (unsigned)(s[n].kc >> 32) < 1u << 12) out[n] = weak_point<RHS>(s[n], kap, g[n]);
+    }
 }
 
 // The points of the marked patches (bit p of a thread's `again`: plane kb + p),
@@ -415,7 +451,8 @@ __device__ __forceinline__ void points(Stencil (&s)[N], double (&out)[N]) {
 template <bool RHS>
 __device__ __noinline__ void form_alone(unsigned again, unsigned short *list, int *count,
                                         double *un, const u64 *u, const u64 *K, const u64 *rhs,
-                                        int tx, int ty, int kb, int nx, int ny, int P, size_t S) {
+                                        Kappa kap, int tx, int ty, int kb, int nx, int ny, int P,
+                                        size_t S) {
   const int me = threadIdx.x;
   for (int first = 0; first < kMaxPlanes; first += 16) {
     __syncthreads();
@@ -433,18 +470,18 @@ __device__ __noinline__ void form_alone(unsigned again, unsigned short *list, in
       const int i = tx * TX + 2 * (t % NTX) + (me & 1);
       const int j = 1 + ty * TY + 2 * (t / NTX) + (me >> 1 & 1);
       if (i < 1 || i >= nx - 1 || j >= ny - 1) continue;
-      const size_t g = (size_t)k * S + (size_t)j * P + i;
-      const u64 *v = u + g, *kv = K + g;
+      const size_t g[1] = {(size_t)k * S + (size_t)j * P + i};
+      const u64 *v = u + g[0], *kv = K + g[0];
       Stencil st[1] = {{__ldcg(v),
                         {__ldcg(v + S), __ldcg(v - S), __ldcg(v - 1), __ldcg(v + 1), __ldcg(v - P),
                          __ldcg(v + P)},
                         __ldcg(kv),
                         {__ldcg(kv + S), __ldcg(kv - S), __ldcg(kv - 1), __ldcg(kv + 1),
                          __ldcg(kv - P), __ldcg(kv + P)},
-                        RHS ? __ldcg(rhs + g) : 0}};
+                        RHS ? __ldcg(rhs + g[0]) : 0}};
       double out[1];
-      points<RHS>(st, out);
-      un[g] = out[0];
+      points<RHS>(st, kap, g, out);
+      un[g[0]] = out[0];
     }
   }
 }
@@ -464,8 +501,8 @@ __device__ __forceinline__ void reload() { asm volatile("" ::: "memory"); }
 // its schedule (512^3: 804 to 850 us a step for 770).
 template <bool RHS, class M>
 __device__ __noinline__ bool form_walk(const M maps, Smem<RHS> &sm, unsigned again, int n,
-                                       double *un, int tx, int ty, int nx, int ny, int P, size_t S,
-                                       int kb, int first, int last, unsigned wait_limit) {
+                                       double *un, Kappa kap, int tx, int ty, int nx, int ny, int P,
+                                       size_t S, int kb, int first, int last, unsigned wait_limit) {
   const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
   const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly, o = (2 * ly + 1) * BX + 2 * lx + 2;
   const bool x0 = i >= 1 && i < nx - 1, x1 = i + 1 < nx - 1;
@@ -520,7 +557,8 @@ __device__ __noinline__ bool form_walk(const M maps, Smem<RHS> &sm, unsigned aga
                    0};
           if constexpr (RHS) st[x].vr = sk.r[(2 * ly + y) * TX + 2 * lx + x];
         }
-        points<RHS>(st, out);
+        const size_t g = w - un + (y ? P : 0);
+        points<RHS>(st, kap, {g, g + 1}, out);
         if (x0) w[y ? P : 0] = out[0];
         if (x1) w[(y ? P : 0) + 1] = out[1];
       }
@@ -539,8 +577,9 @@ __device__ __noinline__ bool form_walk(const M maps, Smem<RHS> &sm, unsigned aga
 template <bool RHS, class M>
 __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__restrict__ un,
                                         const u64 *__restrict__ u, const u64 *__restrict__ K,
-                                        const u64 *__restrict__ rhs, int tx, int ty, int nx, int ny,
-                                        int P, size_t S, int kb, int ke, const int *err,
+                                        const u64 *__restrict__ rhs, const double *kappa,
+                                        double factor, int tx, int ty, int nx, int ny, int P,
+                                        size_t S, int kb, int ke, const int *err,
                                         unsigned wait_limit) {
   const int t = threadIdx.x, lx = t % NTX, ly = t / NTX;
   const int i = tx * TX + 2 * lx, j = 1 + ty * TY + 2 * ly;  // patch: i, i + 1; j, j + 1
@@ -856,12 +895,13 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     atomicOr(&sm.planes, some);
   }
   __syncthreads();
+  const Kappa kap{kappa, factor, P, S};
   const int first = __ffs(sm.planes) - 1, last = 31 - __clz(sm.planes);
   if (2 * sm.count > NT * (last - first + 1))
-    return form_walk<RHS>(maps, sm, again, ke - kb + 2, un, tx, ty, nx, ny, P, S, kb, first, last,
+    return form_walk<RHS>(maps, sm, again, ke - kb + 2, un, kap, tx, ty, nx, ny, P, S, kb, first, last,
                           wait_limit);
-  form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs, tx,
-                  ty, kb, nx, ny, P, S);
+  form_alone<RHS>(again, reinterpret_cast<unsigned short *>(sm.below), &sm.count, un, u, K, rhs, kap,
+                  tx, ty, kb, nx, ny, P, S);
   return failed;
 }
 
@@ -874,12 +914,12 @@ __device__ __forceinline__ Smem<RHS> &smem() {
 template <bool RHS>
 __global__ void __launch_bounds__(NT, kMinB)
     k_fx(const __grid_constant__ Maps maps, double *__restrict__ un, const u64 *__restrict__ u,
-         const u64 *__restrict__ K, const u64 *__restrict__ rhs, int nx, int ny, int nz, int P,
-         size_t S, int k0, int kchunk, int *__restrict__ err, unsigned wait_limit) {
+         const u64 *__restrict__ K, const u64 *__restrict__ rhs, const double *__restrict__ kappa,
+         double factor, int nx, int ny, int nz, int P, size_t S, int k0, int kchunk, int *__restrict__ err, unsigned wait_limit) {
   const int kb = k0 + blockIdx.z * kchunk;
   const int ke = min(kb + kchunk, nz - 1);
   if (kb >= ke) return;  // whole block
-  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, blockIdx.x, blockIdx.y, nx, ny, P,
+  if (fx_tile<RHS>(ParamMaps{maps}, smem<RHS>(), un, u, K, rhs, kappa, factor, blockIdx.x, blockIdx.y, nx, ny, P,
                    S, kb, ke, err, wait_limit) &&
       threadIdx.x == 0)
     atomicExch(err, 1);
@@ -900,7 +940,7 @@ __global__ void __launch_bounds__(NT, kMinB)
     for (int m = 0; m < 4; ++m) tma::acquire_map(tm + m);
   __syncthreads();
   if (fx_tile<RHS>(TableMaps{tm, src}, smem<RHS>(), (double *)g.f[dst], (const u64 *)g.f[src], g.kq,
-                   (const u64 *)g.rhs, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1,
+                   (const u64 *)g.rhs, (const double *)g.w[0], g.factor, tl.tx, tl.ty, g.nx, g.ny, g.P, g.S, tl.k0, tl.k1,
                    g.err, kTableWaitLimit) &&
       threadIdx.x == 0)
     atomicExch(g.err, 1);
@@ -945,8 +985,8 @@ cudaError_t launch(const heat_ctx *c, int cur, cudaStream_t st, unsigned wait_li
        left -= kMaxGridZ, k0 += kMaxGridZ * kc)
     e = launch_chained(k_fx<RHS>, dim3(fx_tiles_x(g.nx), fx_tiles_y(g.ny), std::min(left, kMaxGridZ)),
                        NT, smem_bytes<RHS>(), st, Maps{c->maps[cur], c->maps[2], c->maps[3]},
-                       c->u[cur ^ 1], (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, g.nx, g.ny,
-                       g.nz, g.pitch, g.plane, k0, kc, c->err, wait_limit);
+                       c->u[cur ^ 1], (const u64 *)c->u[cur], c->kq, (const u64 *)c->rhs, c->kappa,
+                       c->factor, g.nx, g.ny, g.nz, g.pitch, g.plane, k0, kc, c->err, wait_limit);
   return e;
 }
 

@@ -34,7 +34,7 @@ struct heat_ctx {
   double *rhs;              // NULL when the problem has no source term
 
   // Per-form coefficient planes (only the ones the chosen kernel uses).
-  double *kappa;            // raw conductivity (naive kernel)
+  double *kappa;            // raw conductivity (naive kernel; default form, small weights)
   double *ks[3];            // face kappa sums kx, ky, kz (bit-exact kernel)
   double *c0;               // centre weight 1 - sum of face weights (fast, FP64 pipe)
   double *cf[3];            // face weights factor*(kappa_a+kappa_b) (fast, FP64 pipe)
