@@ -42,20 +42,25 @@ __global__ void k_kq_setup(u64 *__restrict__ K, int *__restrict__ bad,
     }
 }
 
-// bad[0] is set where a centre weight 1 - sum_f w_f is below 2^-24: with every
-// centre weight above that no sum of the fixed-point form leaves 64 bits.
+// bad[0] is set where a centre weight 1 - sum_f w_f is below 2^-40, or the high limbs of
+// the six weights sum to more than 1 (low limbs below zero; only for centre weights below
+// 7 x 2^-32).  With neither, no sum of the fixed-point form leaves 64 bits: a result is a
+// mean of values, and the sum of d0 w1 stays below 2^32 (2^32 - 1) + 2^31.
 __global__ void k_kq_check(const u64 *__restrict__ K, int *__restrict__ bad, int nx, int ny, int nz,
                            int P, size_t S) {
-  const unsigned *k1 = reinterpret_cast<const unsigned *>(K) + 1;  // high limbs, units of 2^-32
   bool ok = true;
   const long rows = (long)(ny - 2) * (nz - 2);
   for (long r = blockIdx.x; r < rows; r += gridDim.x) {
     const size_t row = (size_t)(1 + r / (ny - 2)) * S + (size_t)(1 + r % (ny - 2)) * P;
     for (int i = 1 + threadIdx.x; i < nx - 1; i += blockDim.x) {
-      const size_t c = row + i;
-      const u64 s = 6ull * k1[2 * c] + k1[2 * (c + 1)] + k1[2 * (c - 1)] + k1[2 * (c + P)] +
-                    k1[2 * (c - P)] + k1[2 * (c + S)] + k1[2 * (c - S)];
-      ok &= s <= (1ull << 32) - (1ull << 8);
+      const u64 *k = K + row + i;
+      u64 s1 = 6 * (*k >> 32);             // units of 2^-32
+      i64 s0 = 6ll * (int)(unsigned)*k;    // of 2^-63
+      for (const u64 v : {k[1], k[-1], k[P], k[-(ptrdiff_t)P], k[S], k[-(ptrdiff_t)S]}) {
+        s1 += v >> 32;
+        s0 += (int)(unsigned)v;
+      }
+      ok &= s1 <= 1ull << 32 && (s1 << 31) + (u64)s0 <= (1ull << 63) - (1ull << 23);
     }
   }
   if (!ok) atomicOr(bad, 1);
