@@ -21,7 +21,9 @@
 // Cache file: $HEAT_TUNE_CACHE, else heat_tune.json next to libheat.so (read
 // again whenever that path changes).  One entry per line:
 //   {"form": F, "nz_max": N, "kchunk": K, "rows": R, "minb": M, "depth": D, "glups": G},
-// (entries written before rows / minb / depth existed read with the defaults).
+// (entries written before rows / minb / depth existed read with the defaults).  The first
+// line says which kernels were timed ("kernels": kKernels); a file of others is not read,
+// one that does not say is.
 
 #include <dlfcn.h>
 
@@ -50,6 +52,8 @@ struct TuneEntry {
 
 const int kClasses[] = {64, 128, 256, 384, 512, 1024, 2048, 1 << 30};
 constexpr int kDefaultKchunk = 32;
+// Raised whenever a table kernel changes what its choices mean or how they rank.
+constexpr int kKernels = 2;
 
 std::mutex g_mu;
 std::vector<TuneEntry> g_table;
@@ -82,6 +86,10 @@ void load_locked() {
   if (!f) return;
   char line[512];
   while (std::fgets(line, sizeof line, f)) {
+    int kernels = 0;
+    if (const char *q = std::strstr(line, "\"kernels\":");
+        q && std::sscanf(q, "\"kernels\": %d", &kernels) == 1 && kernels != kKernels)
+      break;
     const char *p = std::strstr(line, "{\"form\":");
     if (!p) continue;
     TuneEntry t{};
@@ -111,7 +119,7 @@ void load_locked() {
 int save_locked() {
   FILE *f = std::fopen(cache_path().c_str(), "w");
   if (!f) return HEAT_EINVAL;
-  std::fprintf(f, "{\"device\": \"%s\", \"entries\": [\n", g_device);
+  std::fprintf(f, "{\"device\": \"%s\", \"kernels\": %d, \"entries\": [\n", g_device, kKernels);
   for (size_t i = 0; i < g_table.size(); ++i) {
     const TuneEntry &t = g_table[i];
     std::fprintf(f,
@@ -247,8 +255,10 @@ extern "C" int heat_tune_batch(int precision, unsigned flags, int max_nz, int fo
           best_ch = ch;
         }
       };
+      // The fixed-point table kernel has one variant and tiles of at most 32 planes.
+      const bool fx = form == heat::kFormFx;
       for (int kc : {8, 16, 32, 64, 128, 256, 512, nz - 2}) {
-        if (kc > nz - 2) continue;
+        if (kc > nz - 2 || (fx && kc > 32)) continue;
         heat::TuneChoice ch = best_ch;
         ch.kchunk = kc;
         consider(ch);
@@ -256,12 +266,12 @@ extern "C" int heat_tune_batch(int precision, unsigned flags, int max_nz, int fo
       for (int rows : {1, 2}) {
         heat::TuneChoice ch = best_ch;
         ch.rows = rows;
-        if (rows != best_ch.rows) consider(ch);
+        if (rows != best_ch.rows && !fx) consider(ch);
       }
       for (int m = heat::kMinbLo; m < heat::kMinbLo + heat::kNumMinb; ++m) {
         heat::TuneChoice ch = best_ch;
         ch.minb = m;
-        if (m != best_ch.minb) consider(ch);
+        if (m != best_ch.minb && !fx) consider(ch);
       }
       if (form == heat::kFormF32c) {
         heat::TuneChoice ch = best_ch;
