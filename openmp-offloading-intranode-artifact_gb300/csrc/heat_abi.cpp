@@ -278,8 +278,10 @@ int init_fp64(heat_ctx *c, const heat_desc *d) {
     }
   } else {
     // Default form: per-point fixed-point weights.  Problems they cannot
-    // represent, and HEAT_HWFP64, use the FP64-pipe kernel and its FP64 weights.
-    bool fixed = !(c->flags & HEAT_HWFP64) && heat::fx_usable(d->rhs != nullptr);
+    // represent, thin sheets and HEAT_HWFP64 use the FP64-pipe kernel and its FP64
+    // weights.
+    bool fixed = !(c->flags & HEAT_HWFP64) && heat::fx_usable(d->rhs != nullptr) &&
+                 !heat::thin_sheet(g, heat::kThinRowsFp64);
     if (fixed) {
       TRY(dalloc(&c->kq, g.elems, c->stream));
       fixed = heat::encode_fx_maps(c->maps, c->u, c->kq, c->rhs, g);
@@ -398,7 +400,8 @@ int cuda_fail(cudaError_t e, const char *what) {
 }
 
 bool two_step_form(const heat_ctx *c) {
-  return c->precision == HEAT_FP32C && !c->frhs && !(c->flags & HEAT_NO_TEMPORAL) && c->have_maps;
+  return c->precision == HEAT_FP32C && !c->frhs && !(c->flags & HEAT_NO_TEMPORAL) && c->have_maps &&
+         !thin_sheet(c->g, kThinRowsFp32c);
 }
 
 int check_err(heat_ctx *c) {

@@ -206,6 +206,18 @@ inline int balanced_chunk(long tiles, int interior, long resident, int overhead,
   return best_kc;
 }
 
+// Sheets of a few rows, which the TMA-staged kernels' tiles (16 and 20 rows high) would
+// leave mostly empty, step with the column walks instead, where the sheet is large
+// enough that a step is not all launch.  us a step, walk and tiles: default form (two
+// rows at most) 4096 x 4 x 2048 231 and 438, 512 x 4 x 512 15.0 and 17.4, but 256 x 4 x
+// 256 8.3 and 7.5, and three rows of 1024 x 1024 64 and 59; FP32C (eight rows at most)
+// 1024 x 10 x 1024 50 and 54, 512 x 3 x 512 10.3 and 14.6, but 256 x 10 x 256 7.7 and
+// 6.2, and ten rows of 1024 x 1024 72 and 54.
+inline bool thin_sheet(const heat_geom &g, int rows) {
+  return g.ny - 2 <= rows && (long long)(g.nx - 2) * (g.nz - 2) >= 200000;
+}
+constexpr int kThinRowsFp64 = 2, kThinRowsFp32c = 8;
+
 // heat_fp64_exact.cu (compiled with --fmad=false)
 cudaError_t launch_exact_raw(double *u_new, const double *u_old, const double *rhs,
                              const double *kappa, const heat_geom &g, double factor,

@@ -74,3 +74,17 @@ def test_default_form(heat, oracle, cuda_device, planes):
         got = s.field()
     # a rounding and about one unit of the last place a step, the oracle's seven
     assert np.abs(got - ref).max() <= STEPS * 5 * 2.0 ** -52 * np.abs(u0).max()
+
+
+@pytest.mark.gpu
+def test_default_form_in_tiles(heat, oracle, cuda_device):
+    """Three rows: the tiled kernel, in two launches a step."""
+    H = heat
+    kappa, u0, h, dt = H.inputs_config(0, 7, 3, 5, 2_100_000)
+    ref = oracle.steps(u0, kappa, h, dt, STEPS)
+    with H.Solver(kappa, u0, h, dt) as s:
+        s.step(STEPS)
+        got = s.field()
+        assert H.lib().heat_diag_fp64_timeout(s._ctx) == H.HEAT_OK  # it steps with that kernel
+        assert H.lib().heat_sync(s._ctx) == H.HEAT_ETIMEOUT
+    assert np.abs(got - ref).max() <= STEPS * 5 * 2.0 ** -52 * np.abs(u0).max()
