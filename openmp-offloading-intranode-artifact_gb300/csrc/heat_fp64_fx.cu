@@ -111,6 +111,11 @@ constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills
 constexpr unsigned kExp = 1u << 20;      // one binary order in the high word of a double
 constexpr unsigned kExpMask = 0x7ff00000u;
 constexpr unsigned kSlack = 8 * kExp;
+// A patch with a nonzero value this far below E (binary orders, in place) is left to be
+// formed point by point: nearly all of its results would be too small.  (256^3, us a
+// step: a hot cube in zeros, steps 20 to 220, 275 without, 245 at 13 orders, 252 at 16,
+// 267 at 24; random signs 169, 171, 169, 168.)
+constexpr unsigned kSteep = 14 * kExp;
 constexpr unsigned kUnheld = 1;  // of a patch's scale: does not hold its plane before exactly
 constexpr int kLeast = 1 << (53 - 32);          // high word of 2^53
 constexpr int kLeastCrossing = 1 << (51 - 32);  // of 2^51
@@ -206,6 +211,7 @@ struct Range {
     return max((size() + up) & ~(2 * kExp - 1), kLowE);
   }
   __device__ __forceinline__ bool zero() const { return size() < kExp; }
+  __device__ __forceinline__ bool steep(unsigned E) const { return mn < 2 * (E - kSteep) - 2; }
   // Whether the scale holds every value seen exactly.
   __device__ __forceinline__ bool held(unsigned E) const {
     return mn >= 2 * (E - kSlack) - 2 && E <= kHighE && !zero();
@@ -720,7 +726,7 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
     // without signs 812, 820 so).
     const int enough = r.crossing() ? kLeastCrossing : kLeast;
     int least = 0;  // high word of the smallest result (its size), in units
-    if (!r.zero() && En <= kHighE) {
+    if (!r.zero() && En <= kHighE && !r.steep(En)) {
       if ((E & ~kUnheld) != En) {
         if (!(E & kUnheld) && held) {
           const int d = (int)(En - E) >> 20;
@@ -872,8 +878,8 @@ __device__ __forceinline__ bool fx_tile(const M &maps, Smem<RHS> &sm, double *__
       sm.below[0][t] = ld2(&sk.u[o]);
       sm.below[1][t] = ld2(&sk.u[o + BX]);
     }
-    // No scale, or a result too small for its units (zeros in the patch, small
-    // neighbours).
+    // No scale, values too far apart, or a result too small for its units (zeros in the
+    // patch, small neighbours).
     if (least < enough) again |= 1u << (k - kb);
     r0 = r1;
     r1 = r2;
