@@ -233,22 +233,21 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
     pending &= ~(1u << s);
   };
 
-  // The flag is read before the first loads where a wrong map could be what set it,
-  // else behind them, where their own time hides it.
-  bool stop = M::kInMemory && tid == 0 && tma::gave_up(err);
-  if (!stop)
-    for (int p = kb - 2; p <= kb + 1; ++p) issue(p);
-  if (!M::kInMemory) stop = tid == 0 && tma::gave_up(err);
+  // The flag is read before the first loads where a wrong map could be what set it, else
+  // beside them by another warp, and looked at with the first planes.
+  bool stop = tid == (M::kInMemory ? 0 : NT - 1) && tma::gave_up(err);
+  if (M::kInMemory) {
+    if (__syncthreads_or(stop)) return;
+    stop = false;
+  }
+  for (int p = kb - 2; p <= kb + 1; ++p) issue(p);
+  if (!M::kInMemory) __syncthreads();
   // Before the block's shared memory goes its own loads in flight must have landed
   // (each wait bounded).
   auto drain = [&] {
     for (int s = 0; s < R; ++s)
       if (pending & (1u << s)) mbar_wait(&sm.bar[s], (phase >> s) & 1u, M::kLimit);
   };
-  if (__syncthreads_or(stop)) {
-    if (!M::kInMemory && tid == 0) drain();
-    return;
-  }
 
   // This thread's step-(t+1) points: columns gx, gx + 1 (gx even) of row gy,
   // pair lp and row ly of the (17 x 22) region, and their shared-memory offsets.
@@ -300,7 +299,7 @@ __device__ __forceinline__ void tb2_tile(const M &maps, float *__restrict__ vn,
   wait_plane(kb - 1);
   wait_plane(kb);
   wait_plane(kb + 1);
-  failed = __syncthreads_or(failed);
+  failed = __syncthreads_or(failed || stop);
   // Level-1 window: v(p-1), v(p), wz(p-1) for the next plane p to compute.
   f2 vm = 0, v0 = 0, wzm = 0;
   // Level-2 window at the top of iteration k: own step-(t+1) values at planes
