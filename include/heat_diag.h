@@ -47,15 +47,17 @@ int heat_diag_wait_timeout(unsigned attempts, int *timed_out);
  * unchanged.  The next call that synchronises the context -- heat_sync,
  * heat_norm, heat_get_field, or heat_batch_run of a batch holding it --
  * returns HEAT_ETIMEOUT, once.  HEAT_ESTATE for a context that does not step
- * with the two-step kernel (HEAT_FP64, a source term, HEAT_NO_TEMPORAL).    */
+ * with the two-step kernel (HEAT_FP64, a source term, HEAT_NO_TEMPORAL, wide
+ * grids of few interior rows or columns).                                    */
 int heat_diag_fp32c_timeout(struct heat_ctx *c);
 
 /* The same for the default FP64 form's TMA-staged launch (the kernel
  * heat_step uses for HEAT_FP64 contexts, with or without a source term): one
- * launch with its wait limit at 0 attempts gives up at its first wait, flags the context and returns without writing a point; the next
- * synchronising call reports HEAT_ETIMEOUT once.  HEAT_ESTATE for a context
- * that does not step with that launch (HEAT_BITEXACT, HEAT_NAIVE,
- * HEAT_HWFP64, HEAT_FP32C).                                                  */
+ * launch with its wait limit at 0 attempts gives up at its first wait, flags
+ * the context and returns without writing a point; the next synchronising call
+ * reports HEAT_ETIMEOUT once.  HEAT_ESTATE for a context that does not step
+ * with that launch (HEAT_BITEXACT, HEAT_NAIVE, HEAT_HWFP64, HEAT_FP32C, weights
+ * outside the fixed point's range, wide grids of one or two interior rows).   */
 int heat_diag_fp64_timeout(struct heat_ctx *c);
 
 #ifdef __cplusplus

@@ -4,9 +4,9 @@
 //
 // Launch shape: by default one block per tile, scheduled by the hardware; with
 // HEAT_BATCH_PERSISTENT a fixed set of resident blocks strides the table
-// instead.  On configuration 3 (64 uneven grids, half FP64, half FP32C) the
-// hardware-scheduled shape measured 92 GLUP/s against 86 for the persistent
-// one, whose blocks serialise each tile's start-up loads.  Kinds (form x
+// instead, which serialises each tile's start-up loads (64 uneven grids of 48 to 384
+// points per axis, half FP64, half FP32C, with the first column walks: 86 GLUP/s
+// for 92).  Kinds (form x
 // source term x blocks-per-SM variant) present together run on their own
 // streams (created on first use), forked from and joined to the batch stream,
 // unless HEAT_BATCH_SERIAL_FORMS.  Each grid's z-chunk, rows per thread,
@@ -17,9 +17,8 @@
 // points, default 2,000,000) are stepped with their single-grid kernels
 // instead (two FP32C steps per launch) on a stream of their own beside the table
 // kernels; the tile table carries the small grids, which one launch per grid
-// would leave the GPU mostly idle for.
-// On configuration 3 (64 grids of 48..384 points per axis) the table alone
-// measured 129 GLUP/s, with solo grids 137.
+// would leave the GPU mostly idle for.  (The same 64 grids with the first column
+// walks: 129 GLUP/s in the table alone, 137 so.)
 //
 // Bookkeeping: every active context advances one step per batch step; the
 // device table records each grid's current buffer at build time and each

@@ -27,8 +27,8 @@
 // bit-identical to two single steps.  Points on the grid boundary keep their
 // values at both levels.
 //
-// Bound: latency between the barriers (24 warps an SM, issue 45 % busy, DRAM
-// 70 %).  512^3: 376 GLUP/s, where one thread per point in 20 warps ran 331.
+// Bound: issue and latency between the barriers (24 warps an SM, issue 52 % busy at
+// 400^3, shared-memory reads the first stall).  512^3: 375 GLUP/s, where one thread per point in 20 warps ran 331.
 // Measured and not kept at 512^3: 16 rows (10 warps of pairs, which load the
 // schedulers 3 : 3 : 2 : 2) 327, three blocks of them per SM at 64 registers 355;
 // 13 rows in 8 warps, three blocks per SM, 357; 28 rows in 16 warps 319; two

@@ -64,19 +64,22 @@
 // mbarrier; one block barrier per plane frees the oldest slot, whose next plane
 // thread 0 then requests.
 //
-// Bound: the integer pipes.  At 512^3: 174 GLUP/s (0.763 ms a step; 133.5 for
-// rows split between 7 FP64 operations and a per-point alignment in integers,
-// the launch before this one), with the reference's source term 161 (115.7);
-// 192^3 with a narrow Gaussian 136 at first, 126 over 200 steps.
-// About 135 warp instructions per point (300 for an integer row of that
-// launch); at 320^3 the ALU pipe is 58 % busy, FMA-heavy (18 of its instructions the
-// wide multiply-adds, twice the cost of the others) the same, FP64 53 %, issue 61 %,
-// DRAM 24.6 bytes a point.
-// Measured and not kept (512^3, GLUP/s): the neighbours of one
-// row converted by the FP64 pipe as the patch's own are, 169 for 173 (157 for 167 of
-// both); no value converted by it 164 for 167; five blocks per SM
-// at 96 registers 162; 32 x 32 tiles 156; 64 x 8 166; the plane loop unrolled by
-// 2 162.
+// Bound: the integer pipes and the latency between them.  At 512^3: 163 GLUP/s
+// (0.814 ms a step; 133.5 for rows split between 7 FP64 operations and a per-point
+// alignment in integers, the launch before the fixed point), with the reference's
+// source term 153 (115.7); 192^3 with a narrow Gaussian 128.  155 instructions a point,
+// with all the launch's share (300 for an integer row of that launch); at 320^3 the ALU
+// pipe is 63 % busy, FMA 28 % (18 wide multiply-adds a point, each two of the others),
+// FP64 45 %, issue 61 %, DRAM 24.7 bytes a point.
+// Fields that the plain loop does not hold are slower (256^3, us a step, against the
+// row-split launch's 137 to 198 for the same field): smooth 105, one sign throughout
+// 120 to 125, zeros 80, random signs 139 at first and 170 once smooth (137), a
+// front of 40 binary orders in zeros 117 at first and up to 250 while it spreads (190).
+// Measured and not kept, each against the loop of its time (512^3, GLUP/s): the
+// neighbours of one row converted by the FP64 pipe as the patch's own are, 169 for 173
+// (157 for 167 of both); no value converted by it 164 for 167; five blocks per SM at 96
+// registers 162 for 167; 32 x 32 tiles 156, 64 x 8 166, the plane loop unrolled by 2 162
+// for the same 167.
 //
 // Every mbarrier wait is bounded: a wait that runs out stops the block at the
 // next barrier (the flag is OR-reduced), thread 0 waits (bounded) for its loads
@@ -102,8 +105,8 @@ constexpr int TX = 32, TY = 16;          // columns of a tile
 constexpr int NTX = TX / 2, NTY = TY / 2;
 constexpr int NT = NTX * NTY;            // threads, one per 2 x 2 patch
 constexpr int BX = TX + 4, BY = TY + 2;  // box: columns i0 - 2 .. i0 + 33, rows j0 - 1 .. j0 + 16
-// Ring depth: planes k, k + 1 and one in flight (a fourth slot: 512^3 763 us a step
-// for 762, 256^3 99.7 for 99.0).
+// Ring depth: planes k, k + 1 and one in flight (with a fourth slot 512^3 took
+// 0.1 % longer, 256^3 0.7 %).
 constexpr int kRing = 3;
 constexpr int kMaxPlanes = 32;  // of a chunk: a bit each in `again`
 constexpr int kMinB = 4;   // blocks per SM: 128 registers a thread, no spills

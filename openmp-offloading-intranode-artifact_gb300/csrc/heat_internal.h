@@ -149,9 +149,9 @@ long resident_blocks(const void *kernel, int threads, size_t smem);
 // `waves` waves of resident blocks, so the last wave, which the GPU may run
 // partly empty, is a small share of it; at least `min_planes` planes per chunk
 // (each chunk re-reads its halo planes and refills its pipeline) unless that
-// would leave fewer than two waves.  At 512^3 the default FP64 launch's 1,024
-// tiles in 3 chunks made 5.05 waves of 608 blocks: 126.4 GLUP/s; 15 chunks
-// (25 waves): 133.4.  Falls back to plane_chunk when `resident` is unknown.
+// would leave fewer than two waves.  Used by the column walks: at 512^3 the FP64-pipe
+// one runs 85.0 GLUP/s so (79.2 with plane_chunk), the FP32C one 210.6 (188.0).  Falls
+// back to plane_chunk when `resident` is unknown.
 inline int wave_chunk(const heat_geom &g, int tile_x, int tile_y, long resident,
                       long waves = 24, int min_planes = 16, int fill_planes = 8) {
   if (resident <= 0) return plane_chunk(g, tile_x, tile_y);
